@@ -17,6 +17,7 @@ FVM_OK, FVM_E_ARG, FVM_E_CUDA, FVM_E_UNSUPPORTED, FVM_E_CAPACITY = 0, -1, -2, -3
 FVM_NOALLOC_SCRATCH_BYTES = 16 * 1024 * 1024
 FVM_MAX_STAGES = 12
 FVM_RED_DOUBLES = 64
+FVM_BACK_SET = (296 * 16 + 2 * 296) * 64
 FVM_PHASE_BC, FVM_PHASE_CELLS, FVM_PHASE_FACES, FVM_PHASE_DIV = 1, 2, 4, 8
 
 _P = ct.c_void_p
@@ -97,6 +98,15 @@ _SIGS = [
                                  _P, _P, ct.c_int64, _P, _P, ct.c_int64, _P, ct.c_int32, _P, _P]),
     ("fvm_mp_gather_f32", ct.c_int, [_P, _P, ct.c_int32, ct.c_int32, _P, _P]),
     ("fvm_mp_layer", ct.c_int, [_P, _P, ct.c_int32, ct.c_int32, _P, _P, _P, _P, _P, ct.c_int32, _P, _P, _P]),
+    ("fvm_mp_layer_train", ct.c_int, [_P, _P, ct.c_int32, ct.c_int32, _P, _P, _P, _P, _P, _P, _P, ct.c_int32, _P, _P,
+                                      _P]),
+    ("fvm_in_layer", ct.c_int, [_P, ct.c_int32, _P, _P, _P, _P, _P, _P]),
+    ("fvm_back_top", ct.c_int, [_P, _P, _P, _P, ct.c_int32, ct.c_int32, _P, _P, _P, _P, _P]),
+    ("fvm_back_decoder", ct.c_int, [_P, _P, ct.c_int32, ct.c_int32, _P, _P]),
+    ("fvm_back_layer", ct.c_int, [_P, _P, _P, _P, ct.c_int32, ct.c_int32, _P, _P, _P, _P]),
+    ("fvm_back_gather", ct.c_int, [_P, _P, ct.c_int32, ct.c_int32, _P, _P, _P, _P, _P, _P, _P, _P]),
+    ("fvm_back_bias", ct.c_int, [_P, _P, ct.c_int32, _P, _P]),
+    ("fvm_back_finish", ct.c_int, [ct.c_int32, _P, _P, _P, _P]),
     ("fvm_mp_scatter_back", ct.c_int, [_P, _P, ct.c_int32, ct.c_int32, ct.c_int32, _P, _P, _P]),
     ("fvm_silu_back", ct.c_int, [_P, _P, ct.c_int32, ct.c_int32, _P, _P, ct.c_int64, _P, _P]),
     ("fvm_transpose_bf16", ct.c_int, [_P, ct.c_int32, ct.c_int32, ct.c_int64, _P, ct.c_int64, _P]),

@@ -17,10 +17,10 @@ Network (width W = 64, L = 4 message-passing layers, SiLU):
     h0 = SiLU(X Win^T + b_in)                                        (h: fp32 residual stream)
     h_{l+1} = h_l + SiLU([bf16(h_l), bf16(mean_{j in nbr} h_l,j)] W_l^T + b_l)  (l = 0..3)
     out = h_L Wout^T + b_out                                        (normalised U_{t+k} - U_t - base)
-All matrix products run on ``fvm_gemm_bf16`` (tcgen05, BF16 operands, FP32 accumulation in tensor
-memory, bias / SiLU / residual fused into the epilogue); the backward pass (SiLU derivative,
-transposed products, split-K weight gradients, the transpose of the neighbour mean) and Adam are
-the library's own kernels as well.  Weights are kept in FP32 (master) with BF16 copies for the GEMMs.
+All matrix products run on tcgen05 (BF16 operands, FP32 accumulation in tensor memory): one fused
+kernel per layer forward (``fvm_mp_layer``) and two backward (``fvm_back_layer`` /
+``fvm_back_gather``: both products of a layer from one copy of its operands, then the transpose of the
+neighbour mean and the next layer's SiLU derivative).  Weights are kept in FP32 (master) with BF16 copies for the GEMMs.
 
 Training data are trajectories the batched FVM solver generates (``BatchedFVM``): every step of a
 spin-up-then-record run is stored on the device and random (U_t, U_{t+k}) windows are drawn.
@@ -159,25 +159,25 @@ class CorrectorNet:
         d, L = self.dev, self.L
         b = {"N": N, "Np": Np,
              "X": torch.zeros((Np, XW), dtype=torch.bfloat16, device=d),
-             "XT": torch.zeros((XW, Np), dtype=torch.bfloat16, device=d),
              "Z": [torch.zeros((N, W), device=d) for _ in range(L + 1)],
              "hf": [torch.zeros((N, W), device=d) for _ in range(L + 1)],
              "A": [torch.zeros((Np, 2 * W), dtype=torch.bfloat16, device=d) for _ in range(L)],
-             "AT": torch.zeros((2 * W, Np), dtype=torch.bfloat16, device=d),
              "dZ": torch.zeros((Np, W), dtype=torch.bfloat16, device=d),
-             "dZT": torch.zeros((W, Np), dtype=torch.bfloat16, device=d),
              "dA": torch.zeros((N, 2 * W), device=d),
              "dh": torch.zeros((N, W), device=d), "dh2": torch.zeros((N, W), device=d),
              "out": torch.zeros((N, self.O), device=d), "dout": torch.zeros((N, self.O), device=d),
+             # column-sum workspace: one set per bias gradient (input layer first), O + 1 for the decoder
+             "sums": torch.zeros((L + 1 + self.O + 1, _lib.FVM_BACK_SET), device=d),
              "loss": torch.zeros(1, dtype=torch.float64, device=d)}
+        g = self.grads
+        dst = [(g["b_in"], W)] + [(g[f"b{l}"], W) for l in range(L)] + [(g["W_out"][o], W) for o in range(self.O)] + \
+            [(g["b_out"], self.O)]
+        n = len(dst)
+        b["finish"] = [(min(32, n - q), (ct.c_void_p * 32)(*[b["sums"][i].data_ptr() for i in range(q, min(q + 32, n))]),
+                        (ct.c_void_p * 32)(*[t.data_ptr() for t, _ in dst[q:q + 32]]),
+                        (ct.c_int32 * 32)(*[c for _, c in dst[q:q + 32]])) for q in range(0, n, 32)]
         self._bufs = b
         return b
-
-    def _gemm(self, A, lda, B, ldb, M, N, K, Df=None, Db=None, ldd=0, bias=None, resid=None, ldr=0, pre=None,
-              act=0, k_splits=1):
-        _lib.check(self.lib.fvm_gemm_bf16(A.data_ptr(), lda, B.data_ptr(), ldb, M, N, K, k_splits, _lib.ptr(bias),
-                                          _lib.ptr(resid), ldr, _lib.ptr(Df), _lib.ptr(Db), ldd, _lib.ptr(pre),
-                                          act, self.err.data_ptr(), _lib.stream_ptr()), "fvm_gemm_bf16")
 
     # -- forward ---------------------------------------------------------------------------------
     def features(self, state, mean, inv_std, geo):
@@ -191,36 +191,27 @@ class CorrectorNet:
     def forward(self, nbr: torch.Tensor, store_pre: bool = True) -> torch.Tensor:
         """Network output for the features already in the X buffer (``features``).
 
-        Training (``store_pre=True``): the input GEMM, then per layer the gather of
-        [bf16(h_i), bf16(mean_j h_j)] from the fp32 residual stream (kept for the backward pass)
-        and a GEMM whose epilogue adds bias, SiLU and the residual, storing the pre-activations;
-        the decoder reads the last fp32 activations.  Inference (``store_pre=False``): the input
-        GEMM, then one persistent fused kernel per layer (``fvm_mp_layer``: the gather built in
-        shared memory, tcgen05 MMA, epilogue), the last one with the decoder in its epilogue.  Both
-        forms do the same arithmetic in the same order and give bitwise the same output."""
+        The input layer (``fvm_in_layer``), then one fused kernel per layer: the operand
+        [bf16(h_i), bf16(mean_j h_j)] built in shared memory, tcgen05 MMA, bias + SiLU + residual, the
+        last one with the decoder.  Training (``store_pre=True``, ``fvm_mp_layer_train``) also stores
+        the pre-activations and the operands for the backward pass; inference does not.  Both forms
+        give bitwise the same output."""
         b = self._bufs
         N, L = b["N"], self.L
         p, s = self.params, _lib.stream_ptr()
-        Z = b["Z"] if store_pre else [None] * (L + 1)
-        self._gemm(b["X"], XW, self.bf["W_in"], XW, N, W, XW, Df=b["hf"][0], ldd=W, bias=p["b_in"], pre=Z[0], act=1)
+        err = self.err.data_ptr()
+        Z = [z.data_ptr() for z in b["Z"]] if store_pre else [None] * (L + 1)
+        _lib.check(self.lib.fvm_in_layer(b["X"].data_ptr(), N, self.bf["W_in"].data_ptr(), p["b_in"].data_ptr(),
+                                         b["hf"][0].data_ptr(), Z[0], err, s), "fvm_in_layer")
         for l in range(L):
-            if not store_pre:
-                last = l == L - 1
-                _lib.check(self.lib.fvm_mp_layer(b["hf"][l].data_ptr(), nbr.data_ptr(), N, nbr.shape[1],
-                                                 self.bf[f"W{l}"].data_ptr(), p[f"b{l}"].data_ptr(),
-                                                 None if last else b["hf"][l + 1].data_ptr(),
-                                                 p["W_out"].data_ptr() if last else None,
-                                                 p["b_out"].data_ptr() if last else None, self.O,
-                                                 b["out"].data_ptr() if last else None, self.err.data_ptr(), s),
-                           "fvm_mp_layer")
-                continue
-            _lib.check(self.lib.fvm_mp_gather_f32(b["hf"][l].data_ptr(), nbr.data_ptr(), N, nbr.shape[1],
-                                                  b["A"][l].data_ptr(), s), "fvm_mp_gather_f32")
-            self._gemm(b["A"][l], 2 * W, self.bf[f"W{l}"], 2 * W, N, W, 2 * W, Df=b["hf"][l + 1], ldd=W,
-                       bias=p[f"b{l}"], resid=b["hf"][l], ldr=W, pre=Z[l + 1], act=1)
-        if store_pre:
-            _lib.check(self.lib.fvm_decoder_f32(b["hf"][L].data_ptr(), p["W_out"].data_ptr(), p["b_out"].data_ptr(),
-                                                N, self.O, b["out"].data_ptr(), s), "fvm_decoder_f32")
+            last = l == L - 1
+            keep = store_pre or not last
+            _lib.check(self.lib.fvm_mp_layer_train(
+                b["hf"][l].data_ptr(), nbr.data_ptr(), N, nbr.shape[1], self.bf[f"W{l}"].data_ptr(),
+                p[f"b{l}"].data_ptr(), b["hf"][l + 1].data_ptr() if keep else None, Z[l + 1],
+                b["A"][l].data_ptr() if store_pre else None, p["W_out"].data_ptr() if last else None,
+                p["b_out"].data_ptr() if last else None, self.O, b["out"].data_ptr() if last else None, err, s),
+                "fvm_mp_layer")
         return b["out"]
 
     # -- backward + optimiser --------------------------------------------------------------------
@@ -229,35 +220,32 @@ class CorrectorNet:
 
         Returns the loss as a device tensor (no host synchronisation)."""
         b = self._bufs
-        N, Np, L, s = b["N"], b["Np"], self.L, _lib.stream_ptr()
+        N, L, s = b["N"], self.L, _lib.stream_ptr()
         p, g = self.params, self.grads
         self.forward(nbr)
         b["loss"].zero_()
         _lib.check(self.lib.fvm_mse(b["out"].data_ptr(), target.data_ptr(), N * self.O, b["loss"].data_ptr(),
                                     b["dout"].data_ptr(), s), "fvm_mse")
-        _lib.check(self.lib.fvm_decoder_back_f32(b["hf"][L].data_ptr(), p["W_out"].data_ptr(), b["dout"].data_ptr(),
-                                                 N, self.O, b["dh"].data_ptr(), g["W_out"].data_ptr(),
-                                                 g["b_out"].data_ptr(), s), "fvm_decoder_back_f32")
+        # per layer: dA and dW on the tensor cores, then dh, the next dZ and the column sums (two
+        # passes each: the second rides on the next kernel that reads the same terms)
+        chk, lib, nk, err = _lib.check, self.lib, nbr.shape[1], self.err.data_ptr()
+        ptr = lambda t: t.data_ptr()
+        bias, dec = b["sums"], ptr(b["sums"][L + 1])
         dh, dh2 = b["dh"], b["dh2"]
-        splits = max(1, min(512, (Np // 64) // 8))
+        chk(lib.fvm_back_top(ptr(b["hf"][L]), ptr(p["W_out"]), ptr(b["dout"]), ptr(b["Z"][L]), N, self.O, ptr(dh),
+                             ptr(b["dZ"]), dec, ptr(bias[L]), s), "fvm_back_top")
+        chk(lib.fvm_back_decoder(ptr(b["hf"][L]), ptr(b["dout"]), N, self.O, dec, s), "fvm_back_decoder")
         for l in reversed(range(L)):
-            _lib.check(self.lib.fvm_silu_back(dh.data_ptr(), b["Z"][l + 1].data_ptr(), N, W, b["dZ"].data_ptr(),
-                                              b["dZT"].data_ptr(), Np, g[f"b{l}"].data_ptr(), s), "fvm_silu_back")
-            _lib.check(self.lib.fvm_transpose_bf16(b["A"][l].data_ptr(), N, 2 * W, 2 * W, b["AT"].data_ptr(), Np, s),
-                       "fvm_transpose_bf16")
-            # dW_l += dZ^T A_l   (M = 64 output channels, N = 128 inputs, K = cells, split-K)
-            self._gemm(b["dZT"], Np, b["AT"], Np, W, 2 * W, Np, Df=g[f"W{l}"], ldd=2 * W, k_splits=splits)
-            # dA = dZ W_l
-            self._gemm(b["dZ"], W, self.bfT[f"W{l}"], W, N, 2 * W, W, Df=b["dA"], ldd=2 * W)
-            # dh_l = dh_{l+1} (residual) + dA[:, :W] + transpose of the neighbour mean of dA[:, W:]
-            _lib.check(self.lib.fvm_mp_scatter_back(b["dA"].data_ptr(), nbr.data_ptr(), N, W, nbr.shape[1],
-                                                    dh.data_ptr(), dh2.data_ptr(), s), "fvm_mp_scatter_back")
+            chk(lib.fvm_back_layer(ptr(b["dZ"]), ptr(b["A"][l]), ptr(self.bfT[f"W{l}"]), ptr(nbr), nk, N, ptr(b["dA"]),
+                                   ptr(g[f"W{l}"]), err, s), "fvm_back_layer")
+            chk(lib.fvm_back_gather(ptr(b["dA"]), ptr(nbr), N, nk, ptr(dh), ptr(b["Z"][l + 1]), ptr(bias[l + 1]),
+                                    ptr(b["Z"][l]), ptr(dh2), ptr(b["dZ"]), ptr(bias[l]), s), "fvm_back_gather")
             dh, dh2 = dh2, dh
-        _lib.check(self.lib.fvm_silu_back(dh.data_ptr(), b["Z"][0].data_ptr(), N, W, b["dZ"].data_ptr(),
-                                          b["dZT"].data_ptr(), Np, g["b_in"].data_ptr(), s), "fvm_silu_back")
-        _lib.check(self.lib.fvm_transpose_bf16(b["X"].data_ptr(), N, XW, XW, b["XT"].data_ptr(), Np, s),
-                   "fvm_transpose_bf16")
-        self._gemm(b["dZT"], Np, b["XT"], Np, W, XW, Np, Df=g["W_in"], ldd=XW, k_splits=splits)
+        chk(lib.fvm_back_layer(ptr(b["dZ"]), ptr(b["X"]), None, None, 0, N, None, ptr(g["W_in"]), err, s),
+            "fvm_back_layer")
+        chk(lib.fvm_back_bias(ptr(dh), ptr(b["Z"][0]), N, ptr(bias[0]), s), "fvm_back_bias")
+        for n, sets, dst, cols in b["finish"]:
+            chk(lib.fvm_back_finish(n, sets, dst, cols, s), "fvm_back_finish")
         self.bucket.average()
         self.adam()
         return b["loss"]
@@ -301,7 +289,7 @@ class CorrectorNet:
 
     def check_errors(self):
         if int(self.err.item()) != 0:
-            raise RuntimeError("tensor-core completion wait timed out in fvm_gemm_bf16")
+            raise RuntimeError("tensor-core completion wait timed out in a corrector kernel")
 
 
 # ---------------------------------------------------------------------------------------------

@@ -646,43 +646,46 @@ extern "C" int fvm_corrector_combine(const float* state, const float* base, cons
 
 
 // ------------------------------------------------------------------------------------------
-// Persistent message-passing layer on an fp32 residual stream (fvm_mp_layer).
+// Message-passing layer on an fp32 residual stream (fvm_mp_layer, fvm_mp_layer_train) and the
+// network's input layer (fvm_in_layer).
 //
 //   h'_i = h_i + SiLU([bf16(h_i), bf16(mean_{j in nbr(i)} h_j)] . W^T + b)       (W: bf16 [64][128])
-//   and, for the last layer, out_i = W_out h'_i + b_out instead of storing h'.
+//   and, for the last layer, out_i = W_out h'_i + b_out (h' itself only if asked for);
+//   input layer: h_i = SiLU(X_i . W^T + b)                                       (X, W: bf16, K = 64)
 //
-// One CTA per SM slot runs a grid-stride loop over 128-row tiles with three roles:
-//   * warps 0-7 (loaders): stage tile k's A operand (128 x 128 bf16, canonical no-swizzle K-major
-//     core-matrix layout, two K slices: own row, neighbour mean) into shared-memory stage k % 2;
-//     the neighbour mean is an fp32 sum over the valid neighbours in table order times 1 / count
-//     (the gathers are latency-bound: eight warps, each thread with two rows' loads in flight);
-//   * thread 0 (a loader) issues the tile's eight tcgen05.mma (M 128, N 64, K 16) into tensor-memory
-//     accumulator k % 2 and commits to two mbarriers: "stage free" and "accumulator full";
-//   * warps 8-11 (epilogue): read accumulator k % 2 (warp 8 + w owns TMEM lanes 32w..32w+31 = tile
-//     rows), free it for tile k + 2 (an mbarrier), add bias, SiLU, the fp32 residual and store h'
-//     (or the decoder's outputs) with 256-bit accesses.
-// So the gathers of tile k + 1, the MMAs of tile k and the epilogue of tile k - 1 overlap.  The
-// weights stay in shared memory for the whole launch.  Every mbarrier wait is bounded; a wait that
-// gives up sets *err and ends the role's loop, and the final MMA wait is bounded too, so the kernel
-// always returns and frees its tensor memory.
+// Per row a layer reads h (256 B), gathers up to KN neighbour rows and writes h' (256 B); the
+// neighbours of the Morton-ordered cells are mostly in the same tile, so the gathers hit L1 (72 %)
+// and the floor is the 512 bytes of DRAM traffic.  What bounds it is latency: a tile is a chain of
+// neighbour list -> gathers -> MMA -> epilogue.  One CTA of 128 rows therefore runs that chain without
+// any role split, small enough (64 registers, 54 KB of shared memory, 64 TMEM columns) that four CTAs
+// share an SM and fill each other's waits; one CTA per SM with gather and epilogue warps side by side
+// left 12 warps per SM and took 111 us per layer at 278 k rows of 64.  The
+// epilogue goes through shared memory (the operand's own buffer, free once the MMAs are done), so
+// the residual, the pre-activation and h' move as whole 128-byte lines instead of one line per lane.
+// The mbarrier wait is bounded; a wait that gives up sets *err and ends the CTA.
 // ------------------------------------------------------------------------------------------
 namespace fvm {
 namespace corr {
 
-constexpr int kLayerLoaders = 256;                       // warps 0-7: gathers (+ the MMA issuer)
-constexpr int kLayerThreads = kLayerLoaders + 128;       // warps 8-11: epilogue
+constexpr int kLayerThreads = 256;
+constexpr int kLayerCtas = 4;                            // CTAs per SM
 constexpr int kLayerW = 64;                              // channels
-constexpr int kLayerStageBytes = 2 * TM * TK * 2;        // two K slices of 128 x 64 bf16
-constexpr int kLayerWBytes = kLayerW * 2 * kLayerW * 2;  // W: 64 x 128 bf16
-constexpr int kLayerSmem = kLayerWBytes + 2 * kLayerStageBytes + 1024;
+constexpr int kUnitBytes = TM * 16;                      // one 8-channel unit of a tile's rows
+constexpr int kLayerABytes = 16 * kUnitBytes;            // operand tile, 128 channels (input layer: half)
+constexpr int kLayerWUnit = kLayerW * 16;                // one 8-channel unit of the weights' rows
+constexpr int kLayerWBytes = 16 * kLayerWUnit;           // W: 64 x 128 bf16
+constexpr int kLayerSmem = kLayerWBytes + kLayerABytes;
 
 struct LayerArgs {
     const float* h;              // [M][64] fp32 residual stream (input)
     const int32_t* nbr;          // [M][KN]
+    const __nv_bfloat16* X;      // input layer: [M][64] features (h and nbr unused)
     int M, KN;
-    const __nv_bfloat16* Wt;     // [64][128]
+    const __nv_bfloat16* Wt;     // [64][128] (input layer: [64][64])
     const float* bias;           // [64]
     float* h_out;                // [M][64] or null (decoder only)
+    float* Z;                    // [M][64] pre-activations or null (training)
+    __nv_bfloat16* A;            // [M][128] operand rows or null (training)
     const float* Wo;             // [O][64] decoder weights or null
     const float* bo;             // [O]
     int O;
@@ -700,20 +703,12 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
 }
-__device__ __forceinline__ void loader_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
-// Named barrier of the 256 loader threads that also returns whether any of them passed v != 0,
-// so every loader takes the same branch afterwards.
-__device__ __forceinline__ int loader_sync_or(int v) {
-    int r;
+__device__ __forceinline__ void tc_mma(uint32_t d, uint64_t ad, uint64_t bd, uint32_t idesc, bool accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.b32 p, %1, 0;\n\t"
-        "bar.red.or.pred q, 1, 256, p;\n\t"
-        "selp.b32 %0, 1, 0, q;\n\t}\n"
-        : "=r"(r)
-        : "r"(v)
-        : "memory");
-    return r;
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(d),
+        "l"(ad), "l"(bd), "r"(idesc), "r"(accumulate ? 1u : 0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
 }
 
 // 32 accumulator columns [c0, c0 + 32) of this warp's TMEM lanes.
@@ -729,295 +724,269 @@ __device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&r)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// Stage rows [m0, m0 + 128) of tile into the two K slices at sA (own row, neighbour mean), bf16.
-// Loader thread lt (0..255) handles the 8-channel unit u = (lt >> 3) & 7 of rows
-// (lt & 7) + 8 * (lt >> 6) + 32 q, q = 0..3: a warp covers 8 rows x 4 units per q, so its 16-byte
-// shared-memory stores hit all 32 banks once per 8 lanes and its global reads are 128-byte row
-// segments.  With at most KM <= 4 neighbours the loads of two rows (own + KM neighbours each) are
-// all issued before any is used -- a missing neighbour reads the row itself and contributes +0,
-// which leaves the sum unchanged (the sum starts at +0 and is never -0) -- so a thread keeps ten
-// 32-byte loads in flight instead of one; wider neighbour lists take the row-by-row loop.
-__device__ __forceinline__ void stage_store(uint8_t* sA, int r, int u, const float (&own)[8], const float (&acc)[8],
-                                            float inv) {
-    const int slice_bytes = (TM / 8) * 256;
-    __align__(16) __nv_bfloat16 a[8], b[8];
+// Operand layout of a tile: 16-byte unit u (8 channels) of row r at u * kUnitBytes + 16 r.  Eight
+// consecutive rows of a unit are one core matrix, so the tile reads as a K-major operand with the
+// channels as K (core matrices of a K step LBO = kUnitBytes apart, 8-row groups SBO = 128 apart).
+__device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
+    __align__(16) __nv_bfloat16 a[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-        a[e] = __float2bfloat16(own[e]);
-        b[e] = __float2bfloat16(acc[e] * inv);
-    }
-    const int off = (u >> 1) * slice_bytes + (r >> 3) * 256 + (u & 1) * 128 + (r & 7) * 16;
-    *reinterpret_cast<uint4*>(sA + off) = *reinterpret_cast<const uint4*>(a);
-    *reinterpret_cast<uint4*>(sA + TM * TK * 2 + off) = *reinterpret_cast<const uint4*>(b);
+    for (int e = 0; e < 8; ++e) a[e] = __float2bfloat16(v[e]);
+    return *reinterpret_cast<const uint4*>(a);
 }
+// Offset of 16-byte chunk c (0..15) of row r in the fp32 epilogue tile (256 bytes per row): the
+// chunk index is xored with the row, so both a warp's 32 rows at one chunk and 8 rows x 4 chunks hit
+// every bank once.
+__device__ __forceinline__ int epi_off(int r, int c) { return r * 256 + ((c ^ (r & 7)) << 4); }
 
-template <int KM>
-__device__ __forceinline__ void stage_layer_tile_batched(uint8_t* sA, const LayerArgs& g, int m0, const int* s_nb,
-                                                         const float* s_inv, int lt) {
-    const int u = (lt >> 3) & 7;
-#pragma unroll 1
-    for (int q0 = 0; q0 < 4; q0 += 2) {
-        float own[2][8], nb[2][KM][8];
-        bool use[2][KM];
-        int rs[2];
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-            const int r = (lt & 7) + 8 * (lt >> 6) + 32 * (q0 + b);
-            rs[b] = r;
-            const int64_t row = (int64_t)m0 + r;
-            const bool valid = row < g.M;
-            const int64_t self = valid ? row : 0;
-            ld8(g.h + self * kLayerW + 8 * u, own[b]);
-#pragma unroll
-            for (int k = 0; k < KM; ++k) {
-                const int j = k < g.KN ? s_nb[r * 8 + k] : -1;
-                use[b][k] = valid && j >= 0;
-                ld8(g.h + (use[b][k] ? (int64_t)j : self) * kLayerW + 8 * u, nb[b][k]);
-            }
-        }
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-            const bool valid = (int64_t)m0 + rs[b] < g.M;
-            float o[8], acc[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                o[e] = valid ? own[b][e] : 0.f;
-                acc[e] = 0.f;
-            }
-#pragma unroll
-            for (int k = 0; k < KM; ++k)
-#pragma unroll
-                for (int e = 0; e < 8; ++e) acc[e] += use[b][k] ? nb[b][k][e] : 0.f;
-            stage_store(sA, rs[b], u, o, acc, s_inv[rs[b]]);
-        }
-    }
-}
-
-__device__ __forceinline__ void stage_layer_tile(uint8_t* sA, const LayerArgs& g, int m0, const int* s_nb,
-                                                 const float* s_inv, int lt) {
-    if (g.KN <= 4) {
-        stage_layer_tile_batched<4>(sA, g, m0, s_nb, s_inv, lt);
-        return;
-    }
-    const int u = (lt >> 3) & 7;
-#pragma unroll 1
-    for (int q = 0; q < 4; ++q) {
-        const int r = (lt & 7) + 8 * (lt >> 6) + 32 * q;
-        const int64_t row = (int64_t)m0 + r;
-        const bool valid = row < g.M;
-        float own[8], acc[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) own[e] = acc[e] = 0.f;
-        if (valid) {
-            ld8(g.h + row * kLayerW + 8 * u, own);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                if (k >= g.KN) break;
-                const int j = s_nb[r * 8 + k];
-                if (j < 0) continue;
-                float v[8];
-                ld8(g.h + (int64_t)j * kLayerW + 8 * u, v);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) acc[e] += v[e];
-            }
-        }
-        stage_store(sA, r, u, own, acc, s_inv[r]);
-    }
-}
-
-__global__ void __launch_bounds__(kLayerThreads, 1) k_mp_layer(LayerArgs g) {
-    extern __shared__ __align__(1024) uint8_t dsmem[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)dsmem + 1023) & ~(uintptr_t)1023);
-    uint8_t* sW = smem;                                   // B operand, both K slices
-    uint8_t* sStage = smem + kLayerWBytes;                // two stages of A
-    __shared__ __align__(8) uint64_t bar_free[2], bar_full[2], bar_empty[2];
+template <bool INPUT>
+__global__ void __launch_bounds__(kLayerThreads, kLayerCtas) k_mp_layer(LayerArgs g) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint8_t* sW = smem;                                   // B operand
+    uint8_t* sA = smem + kLayerWBytes;                    // A operand, then the epilogue tile
+    constexpr int UNITS = INPUT ? 8 : 16;
+    __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t s_taddr;
-    __shared__ int s_nb[TM * 8];
-    __shared__ float s_inv[TM];
+    __shared__ __align__(16) int s_nb[INPUT ? 4 : TM * 8];
+    __shared__ float s_inv[INPUT ? 1 : TM];
     __shared__ float s_bias[kLayerW];
-    __shared__ float s_wo[8 * kLayerW];
-    __shared__ int s_fail;
-    __shared__ int s_last;                                // last local tile whose MMAs were issued
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ __align__(16) float s_wo[INPUT ? 4 : 8 * kLayerW];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ntiles = (g.M + TM - 1) / TM;
-    const int nlocal = blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_taddr)),
-                     "r"(128u));
+                     "r"(64u));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    if (threadIdx.x == 0) {
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(&bar_free[b], 1);
-            mbar_init(&bar_full[b], 1);
-            mbar_init(&bar_empty[b], 4);
-        }
+    if (tid == 0) {
+        mbar_init(&bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;");
-        s_fail = 0;
-        s_last = -1;
     }
-    // weights into the B-operand layout (both K slices), bias and decoder weights
-    for (int t = threadIdx.x; t < 2 * kLayerW * 8; t += blockDim.x) {
-        const int c = t / (kLayerW * 8), rem = t % (kLayerW * 8);
-        const int r = rem >> 3, u = rem & 7;
-        const uint4 v = *reinterpret_cast<const uint4*>(g.Wt + (int64_t)r * 2 * kLayerW + c * TK + 8 * u);
-        const int off = c * (kLayerW * TK * 2) + (u >> 1) * ((kLayerW / 8) * 256) + (r >> 3) * 256 + (u & 1) * 128 +
-                        (r & 7) * 16;
-        *reinterpret_cast<uint4*>(sW + off) = v;
+    dependency_wait();
+    for (int t = tid; t < kLayerW * UNITS; t += kLayerThreads) {
+        const int r = t / UNITS, u = t % UNITS;
+        *reinterpret_cast<uint4*>(sW + u * kLayerWUnit + r * 16) =
+            *reinterpret_cast<const uint4*>(g.Wt + (int64_t)r * 8 * UNITS + 8 * u);
     }
-    for (int t = threadIdx.x; t < kLayerW; t += blockDim.x) s_bias[t] = g.bias[t];
-    if (g.out)
-        for (int t = threadIdx.x; t < g.O * kLayerW; t += blockDim.x) s_wo[t] = g.Wo[t];
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (tid < kLayerW) s_bias[tid] = g.bias[tid];
+    if (!INPUT && g.out)
+        for (int t = tid; t < g.O * kLayerW; t += kLayerThreads) s_wo[t] = g.Wo[t];
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t taddr = s_taddr;
     const uint32_t idesc = make_idesc(kLayerW);
 
-    if (warp < kLayerLoaders / 32) {
-        // ---- loaders (and, thread 0, the MMA issuer) ----
-        // Every decision to stop is taken together (loader_sync_or), so no loader is left waiting
-        // at a named barrier: a loader's own bounded wait that gave up, or thread 0's, counts.
-        const int lt = threadIdx.x;
-        int fail = 0;
-        // neighbour lists are fetched one tile ahead (the gathers of a tile then wait for one
-        // memory round trip, not two)
-        int nxt[8];
-        auto fetch_nbr = [&](int tile) {
-            const int64_t row = (int64_t)tile * TM + lt;
+    // A thread's share of a tile: the 8-channel unit u of rows r0 + 32 q, q = 0..3.  A warp covers
+    // 8 rows x 4 units per q: whole 128-byte lines of global memory, conflict-free 16-byte stores.
+    const int u = (tid >> 3) & 7, r0 = (tid & 7) + 8 * (tid >> 6);
+    // Neighbour lists (thread t: row t) are fetched one tile ahead.
+    int nxt[8];
+    auto fetch_nbr = [&](int tile) {
+        const int64_t row = (int64_t)tile * TM + tid;
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
-                nxt[q] = (lt < TM && row < g.M && q < g.KN) ? __ldg(g.nbr + row * g.KN + q) : -1;
-        };
-        if (nlocal > 0) fetch_nbr((int)blockIdx.x);
-        for (int k = 0; k < nlocal; ++k) {
-            const int tile = (int)blockIdx.x + k * (int)gridDim.x;
-            const int m0 = tile * TM, s = k & 1;
-            uint8_t* sA = sStage + s * kLayerStageBytes;
-            if (k >= 2 && !fail)   // the MMAs of tile k - 2 read this stage
-                fail = !mbar_wait(&bar_free[s], (uint32_t)(((k >> 1) - 1) & 1));
-            // this tile's neighbour lists (every loader finished reading the last ones before the
-            // previous loader_sync)
-            if (lt < TM) {
+        for (int q = 0; q < 8; ++q)
+            nxt[q] = (tid < TM && row < g.M && q < g.KN) ? __ldg(g.nbr + row * g.KN + q) : -1;
+    };
+    if (!INPUT && (int)blockIdx.x < ntiles) fetch_nbr(blockIdx.x);
+    bool ok = true;
+    int k = 0;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++k) {
+        const int m0 = tile * TM;
+        if constexpr (!INPUT) {
+            if (tid < TM) {
                 int cnt = 0;
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
-                    s_nb[lt * 8 + q] = nxt[q];
+                    s_nb[tid * 8 + q] = nxt[q];
                     cnt += nxt[q] >= 0;
                 }
-                s_inv[lt] = cnt > 0 ? 1.f / (float)cnt : 0.f;
+                s_inv[tid] = cnt > 0 ? 1.f / (float)cnt : 0.f;
             }
-            if (k + 1 < nlocal) fetch_nbr(tile + (int)gridDim.x);
-            fail = loader_sync_or(fail);
-            if (fail) break;
-            stage_layer_tile(sA, g, m0, s_nb, s_inv, lt);
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            loader_sync();
-            if (lt == 0) {
-                const int a = k & 1;
-                if (k >= 2) fail = !mbar_wait(&bar_empty[a], (uint32_t)(((k >> 1) - 1) & 1));
-                if (!fail) {
-                    asm volatile("tcgen05.fence::after_thread_sync;");
-                    const uint32_t d = taddr + (uint32_t)(a * kLayerW);
+            if (tile + (int)gridDim.x < ntiles) fetch_nbr(tile + gridDim.x);
+            __syncthreads();
+        }
+        // A operand.  The neighbour mean is the fp32 sum over the valid neighbours in table order
+        // (starting at +0) times 1 / count.  With at most four neighbours all loads of a row's unit
+        // are issued before any is used: a missing neighbour reads the row itself and adds +0,
+        // which leaves the sum unchanged.  Rows past M are zeros.
+#pragma unroll 1
+        for (int q = 0; q < 4; ++q) {
+            const int r = r0 + 32 * q;
+            const int64_t row = (int64_t)m0 + r;
+            const bool valid = row < g.M;
+            const int64_t self = valid ? row : 0;
+            if constexpr (INPUT) {
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                if (valid) v = *reinterpret_cast<const uint4*>(g.X + self * kLayerW + 8 * u);
+                *reinterpret_cast<uint4*>(sA + u * kUnitBytes + r * 16) = v;
+            } else {
+                float own[8], acc[8];
+                ld8(g.h + self * kLayerW + 8 * u, own);
+                if (g.KN <= 4) {
+                    float nb[4][8];
+                    const int4 jj = *reinterpret_cast<const int4*>(s_nb + r * 8);
+                    const int j[4] = {jj.x, jj.y, jj.z, jj.w};
 #pragma unroll
-                    for (int c = 0; c < 2; ++c) {
-                        const uint32_t sa = smem_u32(sA + c * TM * TK * 2);
-                        const uint32_t sb = smem_u32(sW + c * kLayerW * TK * 2);
+                    for (int e = 0; e < 4; ++e)
+                        if (e < 3 || g.KN == 4) ld8(g.h + (j[e] >= 0 ? (int64_t)j[e] : self) * kLayerW + 8 * u, nb[e]);
 #pragma unroll
-                        for (int q = 0; q < TK / 16; ++q) {
-                            const uint64_t ad = make_desc(sa + q * (TM / 8) * 256, 128, 256);
-                            const uint64_t bd = make_desc(sb + q * (kLayerW / 8) * 256, 128, 256);
-                            const uint32_t acc = (c > 0 || q > 0) ? 1u : 0u;
-                            asm volatile(
-                                "{\n\t.reg .pred p;\n\t"
-                                "setp.ne.b32 p, %4, 0;\n\t"
-                                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(
-                                    d),
-                                "l"(ad), "l"(bd), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
-                        }
+                    for (int c = 0; c < 8; ++c) acc[c] = 0.f;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (e < 3 || g.KN == 4)
+#pragma unroll
+                            for (int c = 0; c < 8; ++c) acc[c] += j[e] >= 0 ? nb[e][c] : 0.f;
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) acc[c] = 0.f;
+                    for (int e = 0; e < g.KN; ++e) {
+                        const int j = s_nb[r * 8 + e];
+                        if (j < 0) continue;
+                        float v[8];
+                        ld8(g.h + (int64_t)j * kLayerW + 8 * u, v);
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) acc[c] += v[c];
                     }
-                    tc_commit(&bar_free[s]);
-                    tc_commit(&bar_full[a]);
-                    s_last = k;
+                }
+                const float inv = s_inv[r];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    own[c] = valid ? own[c] : 0.f;
+                    acc[c] = valid ? acc[c] * inv : 0.f;
+                }
+                const uint4 a = pack8(own), b = pack8(acc);
+                *reinterpret_cast<uint4*>(sA + u * kUnitBytes + r * 16) = a;
+                *reinterpret_cast<uint4*>(sA + (8 + u) * kUnitBytes + r * 16) = b;
+                if (g.A && valid) {
+                    *reinterpret_cast<uint4*>(g.A + row * 2 * kLayerW + 8 * u) = a;
+                    *reinterpret_cast<uint4*>(g.A + row * 2 * kLayerW + kLayerW + 8 * u) = b;
                 }
             }
         }
-        if (fail) atomicExch(&s_fail, 1);
-    } else {
-        // ---- epilogue ----
-        const int we = warp - kLayerLoaders / 32;         // TMEM lane quarter = warp % 4
-        for (int k = 0; k < nlocal; ++k) {
-            const int tile = (int)blockIdx.x + k * (int)gridDim.x;
-            const int a = k & 1;
-            {   // the residual row is read after the accumulator: ask for it into L1 now
-                const int64_t prow = (int64_t)tile * TM + 32 * we + lane;
-                if (prow < g.M) {
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(g.h + prow * kLayerW));
-                    asm volatile("prefetch.global.L1 [%0];" ::"l"(g.h + prow * kLayerW + 32));
-                }
-            }
-            bool ok = mbar_wait(&bar_full[a], (uint32_t)((k >> 1) & 1));
-            if (!__all_sync(0xffffffffu, ok)) {
-                if (lane == 0) atomicExch(&s_fail, 1);
-                break;
-            }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncthreads();
+        if (tid == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;");
-            const int64_t row = (int64_t)tile * TM + 32 * we + lane;
-            const uint32_t base = taddr + ((uint32_t)(32 * we) << 16) + (uint32_t)(a * kLayerW);
-            uint32_t r0[32], r1[32];
-            tmem_ld32(base, r0);
-            tmem_ld32(base + 32, r1);
-            asm volatile("tcgen05.fence::before_thread_sync;");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bar_empty[a]);   // accumulator a may take tile k + 2
+#pragma unroll
+            for (int q = 0; q < UNITS / 2; ++q)
+                tc_mma(taddr, make_desc(smem_u32(sA) + 2 * q * kUnitBytes, kUnitBytes, 128),
+                       make_desc(smem_u32(sW) + 2 * q * kLayerWUnit, kLayerWUnit, 128), idesc, q > 0);
+            tc_commit(&bar);
+        }
+        if (!__syncthreads_and(mbar_wait(&bar, (uint32_t)(k & 1)))) {
+            ok = false;
+            break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        {   // accumulator + bias -> epilogue tile; warp w reads TMEM lanes 32 (w % 4), columns 32 (w / 4)
+            const int r = 32 * (warp & 3) + lane, half = warp >> 2;
+            uint32_t z[32];
+            tmem_ld32(taddr + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(32 * half), z);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                float4 v;
+                v.x = __uint_as_float(z[4 * c]) + s_bias[32 * half + 4 * c];
+                v.y = __uint_as_float(z[4 * c + 1]) + s_bias[32 * half + 4 * c + 1];
+                v.z = __uint_as_float(z[4 * c + 2]) + s_bias[32 * half + 4 * c + 2];
+                v.w = __uint_as_float(z[4 * c + 3]) + s_bias[32 * half + 4 * c + 3];
+                *reinterpret_cast<float4*>(sA + epi_off(r, 8 * half + c)) = v;
+            }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncthreads();
+        // activation and residual, row units as in the gather
+#pragma unroll 2
+        for (int q = 0; q < 4; ++q) {
+            const int r = r0 + 32 * q;
+            const int64_t row = (int64_t)m0 + r;
             if (row < g.M) {
-                float dec[8];
+                float x[8], v[8];
+                if constexpr (!INPUT) ld8(g.h + row * kLayerW + 8 * u, x);
+                float4* lo = reinterpret_cast<float4*>(sA + epi_off(r, 2 * u));
+                float4* hi = reinterpret_cast<float4*>(sA + epi_off(r, 2 * u + 1));
+                const float4 a = *lo, b = *hi;
+                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+                if (g.Z) st8(g.Z + row * kLayerW + 8 * u, v);
 #pragma unroll
-                for (int o = 0; o < 8; ++o) dec[o] = (g.out && o < g.O) ? __ldg(g.bo + o) : 0.f;
+                for (int c = 0; c < 8; ++c) {
+                    v[c] = silu(v[c]);
+                    if constexpr (!INPUT) v[c] = __fadd_rn(v[c], x[c]);
+                }
+                if (g.h_out) st8(g.h_out + row * kLayerW + 8 * u, v);
+                if (!INPUT && g.out) {
+                    *lo = make_float4(v[0], v[1], v[2], v[3]);
+                    *hi = make_float4(v[4], v[5], v[6], v[7]);
+                }
+            }
+        }
+        if (!INPUT && g.out) {   // decoder: thread t takes row t % 128, outputs t / 128, t / 128 + 2, ...
+            __syncthreads();
+            const int r = tid & (TM - 1);
+            if (m0 + r < g.M) {
+                float dec[4];
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const uint32_t* r = half ? r1 : r0;
-                    const int c0 = 32 * half;
-                    float v[32], x[32];
+                for (int e = 0; e < 4; ++e) {
+                    const int o = 2 * e + (tid >> 7);
+                    dec[e] = o < g.O ? __ldg(g.bo + o) : 0.f;
+                }
+#pragma unroll 4
+                for (int c = 0; c < 16; ++c) {
+                    const float4 v = *reinterpret_cast<const float4*>(sA + epi_off(r, c));
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) ld8(g.h + row * kLayerW + c0 + 8 * q, x + 8 * q);
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) v[j] = __fadd_rn(silu(__uint_as_float(r[j]) + s_bias[c0 + j]), x[j]);
-                    if (g.h_out)
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) st8(g.h_out + row * kLayerW + c0 + 8 * q, v + 8 * q);
-                    if (g.out) {
-#pragma unroll
-                        for (int o = 0; o < 8; ++o) {
-                            if (o < g.O) {
-#pragma unroll
-                                for (int j = 0; j < 32; ++j)
-                                    dec[o] = fmaf(v[j], s_wo[o * kLayerW + c0 + j], dec[o]);
-                            }
+                    for (int e = 0; e < 4; ++e) {
+                        const int o = 2 * e + (tid >> 7);
+                        if (o < g.O) {
+                            const float4 w = *reinterpret_cast<const float4*>(s_wo + o * kLayerW + 4 * c);
+                            dec[e] = fmaf(v.x, w.x, dec[e]);
+                            dec[e] = fmaf(v.y, w.y, dec[e]);
+                            dec[e] = fmaf(v.z, w.z, dec[e]);
+                            dec[e] = fmaf(v.w, w.w, dec[e]);
                         }
                     }
                 }
-                if (g.out)
 #pragma unroll
-                    for (int o = 0; o < 8; ++o)
-                        if (o < g.O) g.out[row * g.O + o] = dec[o];
+                for (int e = 0; e < 4; ++e) {
+                    const int o = 2 * e + (tid >> 7);
+                    if (o < g.O) g.out[(int64_t)(m0 + r) * g.O + o] = dec[e];
+                }
             }
         }
+        __syncthreads();                                  // the tile's buffers may be overwritten
     }
-    // All MMAs of this CTA have completed once the last accumulator was read.  If a role gave up,
-    // wait (bounded) for the commit of the last tile whose MMAs were issued (one thread issued them
-    // in order, so they complete in order) before the tensor memory is released.
-    __syncthreads();
-    if (s_fail && threadIdx.x == 0) {
-        const int k = s_last;
-        if (k >= 0) mbar_wait(&bar_full[k & 1], (uint32_t)((k >> 1) & 1));
+    if (!ok && tid == 0) {
         if (g.err) atomicExch(g.err, 1);
+        mbar_wait(&bar, (uint32_t)(k & 1));              // a second bounded chance before TMEM is released
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(128u));
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(64u));
+}
+
+// Grid: one wave of resident CTAs (kLayerCtas per SM), or one per tile.
+template <bool INPUT>
+static int launch_layer(const LayerArgs& g, cudaStream_t s) {
+    static int sms[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) {
+        launch_status();
+        return FVM_E_CUDA;
+    }
+    if (!sms[dev]) {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+            cudaFuncSetAttribute(k_mp_layer<INPUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLayerSmem) !=
+                cudaSuccess) {
+            launch_status();
+            return FVM_E_CUDA;
+        }
+        sms[dev] = n;
+    }
+    const int ntiles = (g.M + TM - 1) / TM;
+    FVM_LAUNCH(KID_CORRECTOR, s, launch(k_mp_layer<INPUT>, dim3((unsigned)std::min(ntiles, kLayerCtas * sms[dev])),
+                                        dim3(kLayerThreads), kLayerSmem, s, g));
+    return launch_status();
 }
 
 // Training-path gather with the fused layer's arithmetic: out[i] = [bf16(h_i), bf16(mean_j h_j)]
@@ -1099,34 +1068,53 @@ __global__ void k_decoder_back_f32(const float* __restrict__ h, const float* __r
 }  // namespace corr
 }  // namespace fvm
 
-extern "C" int fvm_mp_layer(const float* h, const int32_t* nbr, int32_t M, int32_t KN, const void* Wt,
-                            const float* bias, float* h_out, const float* Wo, const float* bo, int32_t O, float* out,
-                            int32_t* err, void* stream) {
+extern "C" int fvm_mp_layer_train(const float* h, const int32_t* nbr, int32_t M, int32_t KN, const void* Wt,
+                                  const float* bias, float* h_out, float* Z, void* A, const float* Wo,
+                                  const float* bo, int32_t O, float* out, int32_t* err, void* stream) {
     if (!h || !nbr || !Wt || !bias || M <= 0 || KN <= 0 || KN > 8 || !err) return FVM_E_ARG;
     if (!h_out && !out) return FVM_E_ARG;
     if (out && (!Wo || !bo || O < 1 || O > 8)) return FVM_E_ARG;
     auto a32 = [](const void* p) { return ((uintptr_t)p & 31u) == 0; };
-    if (!a32(h) || !a32(h_out) || (uintptr_t)Wt % 16) return FVM_E_ARG;
+    if (!a32(h) || !a32(h_out) || !a32(Z) || (uintptr_t)Wt % 16 || (uintptr_t)A % 16) return FVM_E_ARG;
     if (h_out == h) return FVM_E_ARG;                    // the neighbours of later tiles read h
-    static int sms = 0;
-    static bool attr = false;
-    if (!attr) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaFuncSetAttribute(corr::k_mp_layer, cudaFuncAttributeMaxDynamicSharedMemorySize, corr::kLayerSmem) !=
-                cudaSuccess) {
-            launch_status();
-            return FVM_E_CUDA;
-        }
-        attr = true;
-    }
-    const int ntiles = (M + corr::TM - 1) / corr::TM;
-    const unsigned grid = (unsigned)std::min(ntiles, sms);
-    corr::LayerArgs g{h, nbr, M, KN, static_cast<const __nv_bfloat16*>(Wt), bias, h_out, Wo, bo, O, out, err};
-    cudaStream_t s = (cudaStream_t)stream;
-    FVM_LAUNCH(KID_CORRECTOR, s, corr::k_mp_layer<<<grid, corr::kLayerThreads, corr::kLayerSmem, s>>>(g));
-    return launch_status();
+    corr::LayerArgs g{};
+    g.h = h;
+    g.nbr = nbr;
+    g.M = M;
+    g.KN = KN;
+    g.Wt = static_cast<const __nv_bfloat16*>(Wt);
+    g.bias = bias;
+    g.h_out = h_out;
+    g.Z = Z;
+    g.A = static_cast<__nv_bfloat16*>(A);
+    g.Wo = Wo;
+    g.bo = bo;
+    g.O = O;
+    g.out = out;
+    g.err = err;
+    return corr::launch_layer<false>(g, (cudaStream_t)stream);
+}
+
+extern "C" int fvm_mp_layer(const float* h, const int32_t* nbr, int32_t M, int32_t KN, const void* Wt,
+                            const float* bias, float* h_out, const float* Wo, const float* bo, int32_t O, float* out,
+                            int32_t* err, void* stream) {
+    return fvm_mp_layer_train(h, nbr, M, KN, Wt, bias, h_out, nullptr, nullptr, Wo, bo, O, out, err, stream);
+}
+
+extern "C" int fvm_in_layer(const void* X, int32_t M, const void* Wt, const float* bias, float* h_out, float* Z,
+                            int32_t* err, void* stream) {
+    if (!X || !Wt || !bias || !h_out || M <= 0 || !err) return FVM_E_ARG;
+    auto a32 = [](const void* p) { return ((uintptr_t)p & 31u) == 0; };
+    if (!a32(h_out) || !a32(Z) || (uintptr_t)X % 16 || (uintptr_t)Wt % 16) return FVM_E_ARG;
+    corr::LayerArgs g{};
+    g.X = static_cast<const __nv_bfloat16*>(X);
+    g.M = M;
+    g.Wt = static_cast<const __nv_bfloat16*>(Wt);
+    g.bias = bias;
+    g.h_out = h_out;
+    g.Z = Z;
+    g.err = err;
+    return corr::launch_layer<true>(g, (cudaStream_t)stream);
 }
 
 extern "C" int fvm_mp_gather_f32(const float* h, const int32_t* nbr, int32_t N, int32_t KN, void* out, void* stream) {
@@ -1152,6 +1140,579 @@ extern "C" int fvm_decoder_back_f32(const float* h, const float* Wo, const float
     cudaStream_t s = (cudaStream_t)stream;
     FVM_LAUNCH(KID_CORRECTOR, s, corr::k_decoder_back_f32<<<corr::nblk((int64_t)N * corr::kLayerW, 256), 256, 0, s>>>(
                                      h, Wo, dOut, N, O, dh, dWo, dbo));
+    return launch_status();
+}
+
+// ------------------------------------------------------------------------------------------
+// Backward pass of the network (fvm_back_top, fvm_back_layer, fvm_back_gather, fvm_back_bias,
+// fvm_back_decoder, fvm_back_finish).
+//
+// Per layer two kernels walk the cells:
+//   * k_back_layer: dA = dZ W (the first 64 columns as they are, the others divided by the row's
+//     neighbour count) and dW += dZ^T A, both on tcgen05 from one staged copy of the tile;
+//   * k_back_gather: dh_l = dh_{l+1} + dA[:, :64] + sum over neighbours of dA[:, 64:], then
+//     dZ = dh_l SiLU'(Z_l) for the layer below.
+// All of them are bound by memory: 0.9 kB and 1.7 kB per cell and layer.  They replace a SiLU kernel
+// with one atomic per element (1178 us per layer at 278 k cells), two transposes, two GEMMs with
+// their operands read again and a scatter that counted every neighbour's neighbours.
+//
+// Column sums (the gradients of the biases and of the decoder) keep the value of one running fp32 sum
+// over the cells in order: with terms of one sign that sum's rounding is systematic (1.6e-4 of the
+// decoder's gradient at 278 k cells), so summing pieces from zero would move the results.  Rounding
+// a + t to fp32 depends on a only through its binade, so each warp walks a contiguous range of rows
+// with an accumulator that starts at the sum of everything before it, taken from a first pass over the
+// same terms, and what it added is exact: the first pass runs in the kernel that produces the terms,
+// the second in the next kernel that reads them, the ranges' increments are added up once at the
+// end (k_back_finish).  The result does not depend on scheduling.
+// ------------------------------------------------------------------------------------------
+namespace fvm {
+namespace corr {
+
+constexpr int kSumBlocks = 2 * 148, kSumWarps = 16, kSumThreads = 32 * kSumWarps;
+constexpr int kSumSegs = kSumBlocks * kSumWarps;         // row ranges, one per warp
+// One set of 64 column sums: the ranges' sums, the blocks' sums, the blocks' increments.
+constexpr int kSumSet = (kSumSegs + 2 * kSumBlocks) * kLayerW;
+static_assert(kSumSet == FVM_BACK_SET, "workspace size");
+__host__ __device__ __forceinline__ constexpr int set_block(int b) { return (kSumSegs + b) * kLayerW; }
+__host__ __device__ __forceinline__ constexpr int set_delta(int b) { return (kSumSegs + kSumBlocks + b) * kLayerW; }
+
+struct Rows {
+    int64_t lo, hi;
+};
+__device__ __forceinline__ Rows warp_rows(int N) {
+    const int64_t per = ((int64_t)N + kSumSegs - 1) / kSumSegs;
+    const int64_t lo = ((int64_t)blockIdx.x * kSumWarps + (threadIdx.x >> 5)) * per;
+    return Rows{min(lo, (int64_t)N), min(lo + per, (int64_t)N)};
+}
+__device__ __forceinline__ float2 ldf2(const float* p, int64_t i) { return __ldg(reinterpret_cast<const float2*>(p) + i); }
+
+// First pass: this warp's sums of channels 2 lane, 2 lane + 1 -> the set; block-wide call.
+__device__ __forceinline__ void put_sums(float* set, float2 v, float (*smem)[kLayerW]) {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    reinterpret_cast<float2*>(set + ((int64_t)blockIdx.x * kSumWarps + w) * kLayerW)[lane] = v;
+    __syncthreads();
+    reinterpret_cast<float2*>(smem[w])[lane] = v;
+    __syncthreads();
+    if (threadIdx.x < kLayerW) {
+        float t = 0.f;
+#pragma unroll
+        for (int q = 0; q < kSumWarps; ++q) t += smem[q][threadIdx.x];
+        set[set_block(blockIdx.x) + threadIdx.x] = t;
+    }
+}
+// Second pass: the sum of everything before this warp's range; block-wide call.
+__device__ __forceinline__ float2 get_prefix(const float* set, float (*smem)[kLayerW]) {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float2 t = make_float2(0.f, 0.f);
+#pragma unroll 4
+    for (int b = w; b < (int)blockIdx.x; b += kSumWarps) {
+        const float2 v = __ldcg(reinterpret_cast<const float2*>(set + set_block(b)) + lane);
+        t.x += v.x;
+        t.y += v.y;
+    }
+    __syncthreads();
+    reinterpret_cast<float2*>(smem[w])[lane] = t;
+    __syncthreads();
+    t = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < kSumWarps; ++q) {
+        const float2 v = reinterpret_cast<const float2*>(smem[q])[lane];
+        t.x += v.x;
+        t.y += v.y;
+    }
+    for (int q = 0; q < w; ++q) {
+        const float2 v = __ldcg(reinterpret_cast<const float2*>(set + ((int64_t)blockIdx.x * kSumWarps + q) * kLayerW) + lane);
+        t.x += v.x;
+        t.y += v.y;
+    }
+    return t;
+}
+// Second pass: what this warp's accumulator gained (exact) -> the block's increment; block-wide call.
+__device__ __forceinline__ void put_delta(float* set, float2 acc, float2 start, float (*smem)[kLayerW]) {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __syncthreads();
+    reinterpret_cast<float2*>(smem[w])[lane] = make_float2(acc.x - start.x, acc.y - start.y);
+    __syncthreads();
+    if (threadIdx.x < kLayerW) {
+        double t = 0.0;
+#pragma unroll
+        for (int q = 0; q < kSumWarps; ++q) t += (double)smem[q][threadIdx.x];
+        set[set_delta(blockIdx.x) + threadIdx.x] = (float)t;
+    }
+}
+
+// dh * SiLU'(z)
+__device__ __forceinline__ float silu_grad(float dh, float z) {
+    const float s = 1.f / (1.f + __expf(-z));
+    return dh * s * (1.f + z * (1.f - s));
+}
+__device__ __forceinline__ float2 silu_grad2(float2 dh, float2 z) {
+    return make_float2(silu_grad(dh.x, z.x), silu_grad(dh.y, z.y));
+}
+__device__ __forceinline__ void st_bf2(__nv_bfloat16* p, int64_t i, float2 v) {
+    reinterpret_cast<__nv_bfloat162*>(p)[i] = __floats2bfloat162_rn(v.x, v.y);
+}
+
+// Decoder backward and the last layer's dZ: dh = dOut Wo, dZ = dh SiLU'(Z); first pass of the sums of
+// dOut^T h, dOut (sets [O] and [1] at `dec`) and dZ (`bias`).
+template <int O>
+__global__ void __launch_bounds__(kSumThreads) k_back_top(const float* __restrict__ h, const float* __restrict__ Wo,
+                                                          const float* __restrict__ dOut, const float* __restrict__ Z,
+                                                          int N, float* __restrict__ dh, __nv_bfloat16* __restrict__ dZ,
+                                                          float* __restrict__ dec, float* __restrict__ bias) {
+    __shared__ __align__(16) float smem[kSumWarps][kLayerW];
+    const int lane = threadIdx.x & 31;
+    float2 w[O], aw[O], ao = make_float2(0.f, 0.f), ab = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int o = 0; o < O; ++o) {
+        w[o] = make_float2(__ldg(Wo + o * kLayerW + 2 * lane), __ldg(Wo + o * kLayerW + 2 * lane + 1));
+        aw[o] = make_float2(0.f, 0.f);
+    }
+    const Rows r = warp_rows(N);
+#pragma unroll 4
+    for (int64_t i = r.lo; i < r.hi; ++i) {
+        const float2 x = ldf2(h, i * 32 + lane), z = ldf2(Z, i * 32 + lane);
+        float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int o = 0; o < O; ++o) {
+            const float d = __ldg(dOut + i * O + o);
+            v.x = fmaf(d, w[o].x, v.x);
+            v.y = fmaf(d, w[o].y, v.y);
+            aw[o].x += d * x.x;
+            aw[o].y += d * x.y;
+            if (2 * lane == o) ao.x += d;
+            if (2 * lane + 1 == o) ao.y += d;
+        }
+        reinterpret_cast<float2*>(dh)[i * 32 + lane] = v;
+        const float2 g = silu_grad2(v, z);
+        st_bf2(dZ, i * 32 + lane, g);
+        ab.x += g.x;
+        ab.y += g.y;
+    }
+#pragma unroll
+    for (int o = 0; o < O; ++o) put_sums(dec + (int64_t)o * kSumSet, aw[o], smem);
+    put_sums(dec + (int64_t)O * kSumSet, ao, smem);
+    put_sums(bias, ab, smem);
+}
+
+// Second pass of the decoder's sums.
+template <int O>
+__global__ void __launch_bounds__(kSumThreads) k_back_decoder(const float* __restrict__ h,
+                                                              const float* __restrict__ dOut, int N,
+                                                              float* __restrict__ dec) {
+    __shared__ __align__(16) float smem[kSumWarps][kLayerW];
+    const int lane = threadIdx.x & 31;
+    float2 s0[O + 1], a[O + 1];
+#pragma unroll
+    for (int o = 0; o <= O; ++o) a[o] = s0[o] = get_prefix(dec + (int64_t)o * kSumSet, smem);
+    const Rows r = warp_rows(N);
+#pragma unroll 4
+    for (int64_t i = r.lo; i < r.hi; ++i) {
+        const float2 x = ldf2(h, i * 32 + lane);
+#pragma unroll
+        for (int o = 0; o < O; ++o) {
+            const float d = __ldg(dOut + i * O + o);
+            a[o].x = __fadd_rn(a[o].x, __fmul_rn(d, x.x));
+            a[o].y = __fadd_rn(a[o].y, __fmul_rn(d, x.y));
+            if (2 * lane == o) a[O].x = __fadd_rn(a[O].x, d);
+            if (2 * lane + 1 == o) a[O].y = __fadd_rn(a[O].y, d);
+        }
+    }
+#pragma unroll
+    for (int o = 0; o <= O; ++o) put_delta(dec + (int64_t)o * kSumSet, a[o], s0[o], smem);
+}
+
+// Second pass of a bias gradient on its own (the input layer's).
+__global__ void __launch_bounds__(kSumThreads) k_back_bias(const float* __restrict__ dh, const float* __restrict__ Z,
+                                                           int N, float* __restrict__ bias) {
+    __shared__ __align__(16) float smem[kSumWarps][kLayerW];
+    const int lane = threadIdx.x & 31;
+    const float2 s0 = get_prefix(bias, smem);
+    float2 a = s0;
+    const Rows r = warp_rows(N);
+#pragma unroll 4
+    for (int64_t i = r.lo; i < r.hi; ++i) {
+        const float2 g = silu_grad2(ldf2(dh, i * 32 + lane), ldf2(Z, i * 32 + lane));
+        a.x = __fadd_rn(a.x, g.x);
+        a.y = __fadd_rn(a.y, g.y);
+    }
+    put_delta(bias, a, s0, smem);
+}
+
+// dh = dh_in + dA[:, :64] + sum_{j in nbr} dA[j][64:], in that order; dZ = dh SiLU'(Z) with the first
+// pass of its column sums (bias), and the second pass of the layer above's (dh_in, Z_in, bias_in).
+// A warp per row, two channels per lane: every access is a whole 256-byte half row.  DEEP: the
+// neighbour count as a compile-time bound, so the gathers of several rows are in flight.
+template <int KM>
+__global__ void __launch_bounds__(kSumThreads, 2) k_back_gather(
+    const float* __restrict__ dA, const int32_t* __restrict__ nbr, int N, int KN, const float* __restrict__ dh_in,
+    const float* __restrict__ Z_in, float* __restrict__ bias_in, const float* __restrict__ Z, float* __restrict__ dh,
+    __nv_bfloat16* __restrict__ dZ, float* __restrict__ bias) {
+    __shared__ __align__(16) float smem[kSumWarps][kLayerW];
+    const int lane = threadIdx.x & 31;
+    const float2 s0 = get_prefix(bias_in, smem);
+    float2 a = s0, ab = make_float2(0.f, 0.f);
+    const Rows r = warp_rows(N);
+#pragma unroll 2
+    for (int64_t i = r.lo; i < r.hi; ++i) {
+        int j[KM];
+#pragma unroll
+        for (int q = 0; q < KM; ++q) j[q] = q < KN ? __ldg(nbr + i * KN + q) : -1;
+        const float2 own = ldf2(dA, i * 64 + lane), up = ldf2(dh_in, i * 32 + lane);
+        const float2 zi = ldf2(Z_in, i * 32 + lane), z = ldf2(Z, i * 32 + lane);
+        float2 nb[KM];
+#pragma unroll
+        for (int q = 0; q < KM; ++q) nb[q] = j[q] >= 0 ? ldf2(dA, (int64_t)j[q] * 64 + 32 + lane) : make_float2(0.f, 0.f);
+        const float2 gi = silu_grad2(up, zi);
+        a.x = __fadd_rn(a.x, gi.x);
+        a.y = __fadd_rn(a.y, gi.y);
+        float2 v = make_float2(own.x + up.x, own.y + up.y);
+#pragma unroll
+        for (int q = 0; q < KM; ++q)
+            if (j[q] >= 0) {
+                v.x += nb[q].x;
+                v.y += nb[q].y;
+            }
+        reinterpret_cast<float2*>(dh)[i * 32 + lane] = v;
+        const float2 g = silu_grad2(v, z);
+        st_bf2(dZ, i * 32 + lane, g);
+        ab.x += g.x;
+        ab.y += g.y;
+    }
+    put_delta(bias_in, a, s0, smem);
+    put_sums(bias, ab, smem);
+}
+
+struct FinishArgs {
+    const float* set[32];
+    float* dst[32];
+    int n[32];
+};
+// dst[c] += the sum of a set's block increments (one block per set).
+__global__ void __launch_bounds__(256) k_back_finish(FinishArgs f) {
+    __shared__ double part[4][kLayerW];
+    const int c = threadIdx.x & 63, q = threadIdx.x >> 6;
+    const float* set = f.set[blockIdx.x];
+    double t = 0.0;
+#pragma unroll 8
+    for (int b = q; b < kSumBlocks; b += 4) t += (double)set[set_delta(b) + c];
+    part[q][c] = t;
+    __syncthreads();
+    if (q == 0 && c < f.n[blockIdx.x])
+        f.dst[blockIdx.x][c] += (float)((part[0][c] + part[1][c]) + (part[2][c] + part[3][c]));
+}
+
+// One layer's products over the cells, a persistent kernel (one CTA per SM, 128-row tiles):
+//   warps 8-11 copy the tile's dZ (128 x 64) and A (128 x 128) into a three-stage ring (cp.async) in
+//   the unit layout of the forward layer; one thread issues the MMAs
+//     dA  [128 x 128] = dZ . W       (K-major dZ and W^T; two accumulators)
+//     dW^T [128 x 64] += A^T . dZ    (the same copies read MN-major, the tile's rows as K; one
+//                                     accumulator in tensor memory for the CTA's whole run);
+//   warps 0-7 read dA (warp w: TMEM lanes 32 (w % 4), columns 64 (w / 4)), divide the neighbour half
+//   by the row's neighbour count and store it.  At the end the CTA adds its dW^T to dW.
+// Without dA (the input layer) A is the [N][64] feature rows and only dW is formed.
+constexpr int kBackLoaders = 128, kBackThreads = 256 + kBackLoaders, kBackStages = 3;
+constexpr int kBackStage = 8 * kUnitBytes + kLayerABytes;                        // dZ and A of one tile
+constexpr int kBackSmem = kBackStages * kBackStage + 8 * kUnitBytes;             // + W^T (128 x 64)
+
+__device__ __forceinline__ int loaders_or(int v) {       // named barrier of the loaders, with an OR
+    int r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %1, 0;\n\t"
+        "bar.red.or.pred q, 1, 128, p;\n\t"
+        "selp.b32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(r)
+        : "r"(v)
+        : "memory");
+    return r;
+}
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+
+template <bool LAYER>
+__global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __nv_bfloat16* __restrict__ dZ,
+                                                                const __nv_bfloat16* __restrict__ A,
+                                                                const __nv_bfloat16* __restrict__ WT,
+                                                                const int32_t* __restrict__ nbr, int KN, int N,
+                                                                float* __restrict__ dA, float* __restrict__ dW,
+                                                                int* __restrict__ err) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    uint8_t* sW = smem + kBackStages * kBackStage;
+    __shared__ __align__(8) uint64_t bar_free[kBackStages], bar_full[2], bar_empty[2];
+    __shared__ uint32_t s_taddr;
+    __shared__ int s_fail, s_last;
+    constexpr int AU = LAYER ? 16 : 8;                    // 8-channel units of an A row
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ntiles = (N + TM - 1) / TM;
+    const int nlocal = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_taddr)),
+                     "r"(512u));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        for (int b = 0; b < kBackStages; ++b) mbar_init(&bar_free[b], 1);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&bar_full[b], 1);
+            mbar_init(&bar_empty[b], 8);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;");
+        s_fail = 0;
+        s_last = -1;
+    }
+    if (LAYER) {
+        for (int t = tid; t < TM * 8; t += kBackThreads)
+            *reinterpret_cast<uint4*>(sW + (t & 7) * kUnitBytes + (t >> 3) * 16) =
+                *reinterpret_cast<const uint4*>(WT + (int64_t)(t >> 3) * kLayerW + 8 * (t & 7));
+    } else {   // rows 64..127 of the input layer's dW^T read zeros
+        for (int st = 0; st < kBackStages; ++st)
+            for (int t = tid; t < 8 * kUnitBytes / 16; t += kBackThreads)
+                reinterpret_cast<uint4*>(smem + st * kBackStage + 16 * kUnitBytes)[t] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const uint32_t taddr = s_taddr, tw = taddr + 256;     // dA: columns 0..255, dW^T: 256..319
+    const uint32_t id_a = make_idesc(TM);
+    const uint32_t id_w = make_idesc(kLayerW) | (1u << 15) | (1u << 16);   // both operands MN-major
+
+    if (warp >= 8) {
+        const int lt = tid - 256;
+        auto load = [&](int k) {
+            if (k < nlocal) {
+                const int64_t m0 = (int64_t)((int)blockIdx.x + k * (int)gridDim.x) * TM;
+                const uint32_t sz = smem_u32(smem + (k % kBackStages) * kBackStage), sa = sz + 8 * kUnitBytes;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const int t = lt + q * kBackLoaders, r = (t & 7) + 8 * (t >> 6), u = (t >> 3) & 7;
+                    const bool on = m0 + r < N;
+                    cp16(sz + u * kUnitBytes + r * 16, dZ + (on ? m0 + r : 0) * kLayerW + 8 * u, on);
+                }
+#pragma unroll
+                for (int q = 0; q < AU; ++q) {
+                    const int t = lt + q * kBackLoaders, r = (t & 7) + 8 * (t / (8 * AU)), u = (t >> 3) % AU;
+                    const bool on = m0 + r < N;
+                    cp16(sa + u * kUnitBytes + r * 16, A + (on ? m0 + r : 0) * (8 * AU) + 8 * u, on);
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        load(0);
+        load(1);
+        int fail = 0;
+        for (int k = 0; k < nlocal; ++k) {
+            if (k >= 1 && !fail)                          // the MMAs of tile k - 1 read the stage of tile k + 2
+                fail = !mbar_wait(&bar_free[(k - 1) % kBackStages], (uint32_t)(((k - 1) / kBackStages) & 1));
+            if (!fail) load(k + 2);
+            else asm volatile("cp.async.commit_group;" ::: "memory");
+            asm volatile("cp.async.wait_group 2;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            fail = loaders_or(fail);
+            if (fail) break;
+            if (lt == 0) {
+                const int a = k & 1, st = k % kBackStages;
+                if (LAYER && k >= 2) fail = !mbar_wait(&bar_empty[a], (uint32_t)(((k >> 1) - 1) & 1));
+                if (!fail) {
+                    asm volatile("tcgen05.fence::after_thread_sync;");
+                    const uint32_t sz = smem_u32(smem + st * kBackStage), sa = sz + 8 * kUnitBytes;
+                    if (LAYER)
+#pragma unroll
+                        for (int q = 0; q < kLayerW / 16; ++q)
+                            tc_mma(taddr + a * TM, make_desc(sz + 2 * q * kUnitBytes, kUnitBytes, 128),
+                                   make_desc(smem_u32(sW) + 2 * q * kUnitBytes, kUnitBytes, 128), id_a, q > 0);
+#pragma unroll
+                    for (int q = 0; q < TM / 16; ++q)
+                        tc_mma(tw, make_desc(sa + q * 256, 128, kUnitBytes), make_desc(sz + q * 256, 128, kUnitBytes),
+                               id_w, k > 0 || q > 0);
+                    tc_commit(&bar_free[st]);
+                    tc_commit(&bar_full[a]);
+                    s_last = k;
+                }
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (fail) atomicExch(&s_fail, 1);
+    } else if (LAYER) {
+        const int half = warp >> 2;
+        for (int k = 0; k < nlocal; ++k) {
+            const int a = k & 1;
+            const int64_t row = (int64_t)((int)blockIdx.x + k * (int)gridDim.x) * TM + 32 * (warp & 3) + lane;
+            int deg = 0;
+            if (half && row < N)
+                for (int q = 0; q < KN; ++q) deg += __ldg(nbr + row * KN + q) >= 0;
+            const bool ok = mbar_wait(&bar_full[a], (uint32_t)((k >> 1) & 1));
+            if (!__all_sync(0xffffffffu, ok)) {
+                if (lane == 0) atomicExch(&s_fail, 1);
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            uint32_t v[2][32];
+            const uint32_t base = taddr + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(a * TM + 64 * half);
+            tmem_ld32(base, v[0]);
+            tmem_ld32(base + 32, v[1]);
+            asm volatile("tcgen05.fence::before_thread_sync;");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar_empty[a]);
+            if (row < N) {
+                const float d = (float)max(deg, 1);
+                float* dst = dA + row * TM + 64 * half;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    float x[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        x[e] = __uint_as_float(v[q >> 2][8 * (q & 3) + e]);
+                        if (half) x[e] = x[e] / d;
+                    }
+                    st8(dst + 8 * q, x);
+                }
+            }
+        }
+    }
+    __syncthreads();
+    // wait for the last tile's commit (the MMAs of one thread complete in order)
+    bool done = true;
+    if (s_last >= 0) done = mbar_wait(&bar_full[s_last & 1], (uint32_t)((s_last >> 1) & 1));
+    if (!__syncthreads_and(done) || s_fail) {
+        if (tid == 0) atomicExch(err, 1);
+    } else if (warp < 4 && s_last >= 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        uint32_t v[32];
+        const int in = 32 * warp + lane;                  // input channel
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            tmem_ld32(tw + ((uint32_t)(32 * warp) << 16) + 32 * half, v);
+            if (in < 8 * AU)
+#pragma unroll
+                for (int n = 0; n < 32; ++n) atomicAdd(dW + (int64_t)(32 * half + n) * (8 * AU) + in, __uint_as_float(v[n]));
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(512u));
+}
+
+template <bool LAYER>
+static int launch_back_layer(const void* dZ, const void* A, const void* WT, const int32_t* nbr, int KN, int N,
+                             float* dA, float* dW, int* err, cudaStream_t s) {
+    static int sms[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) {
+        launch_status();
+        return FVM_E_CUDA;
+    }
+    if (!sms[dev]) {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+            cudaFuncSetAttribute(k_back_layer<LAYER>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBackSmem) !=
+                cudaSuccess) {
+            launch_status();
+            return FVM_E_CUDA;
+        }
+        sms[dev] = n;
+    }
+    const unsigned grid = (unsigned)std::min((N + TM - 1) / TM, sms[dev]);
+    FVM_LAUNCH(KID_CORRECTOR, s, k_back_layer<LAYER><<<grid, kBackThreads, kBackSmem, s>>>(
+                                     static_cast<const __nv_bfloat16*>(dZ), static_cast<const __nv_bfloat16*>(A),
+                                     static_cast<const __nv_bfloat16*>(WT), nbr, KN, N, dA, dW, err));
+    return launch_status();
+}
+
+static inline bool aligned(const void* p, int b) { return ((uintptr_t)p & (b - 1)) == 0; }
+
+}  // namespace corr
+}  // namespace fvm
+
+#define FVM_BY_OUTPUTS(O, CALL)  \
+    switch (O) {                 \
+        case 1: CALL(1); break;  \
+        case 2: CALL(2); break;  \
+        case 3: CALL(3); break;  \
+        case 4: CALL(4); break;  \
+        case 5: CALL(5); break;  \
+        case 6: CALL(6); break;  \
+        case 7: CALL(7); break;  \
+        default: CALL(8); break; \
+    }
+
+extern "C" int fvm_back_top(const float* h, const float* Wo, const float* dOut, const float* Z, int32_t N, int32_t O,
+                            float* dh, void* dZ, float* dec, float* bias, void* stream) {
+    if (!h || !Wo || !dOut || !Z || !dh || !dZ || !dec || !bias || N <= 0 || O < 1 || O > 8) return FVM_E_ARG;
+    if (!corr::aligned(h, 8) || !corr::aligned(Z, 8) || !corr::aligned(dh, 8) || !corr::aligned(dZ, 4) ||
+        !corr::aligned(dec, 8) || !corr::aligned(bias, 8))
+        return FVM_E_ARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    __nv_bfloat16* z = static_cast<__nv_bfloat16*>(dZ);
+#define FVM_CALL(OO) FVM_LAUNCH(KID_CORRECTOR, s, corr::k_back_top<OO><<<corr::kSumBlocks, corr::kSumThreads, 0, s>>>( \
+                                    h, Wo, dOut, Z, N, dh, z, dec, bias))
+    FVM_BY_OUTPUTS(O, FVM_CALL)
+#undef FVM_CALL
+    return launch_status();
+}
+
+extern "C" int fvm_back_decoder(const float* h, const float* dOut, int32_t N, int32_t O, float* dec, void* stream) {
+    if (!h || !dOut || !dec || N <= 0 || O < 1 || O > 8 || !corr::aligned(h, 8) || !corr::aligned(dec, 8))
+        return FVM_E_ARG;
+    cudaStream_t s = (cudaStream_t)stream;
+#define FVM_CALL(OO) FVM_LAUNCH(KID_CORRECTOR, s, corr::k_back_decoder<OO><<<corr::kSumBlocks, corr::kSumThreads, 0, s>>>( \
+                                    h, dOut, N, dec))
+    FVM_BY_OUTPUTS(O, FVM_CALL)
+#undef FVM_CALL
+    return launch_status();
+}
+
+extern "C" int fvm_back_layer(const void* dZ, const void* A, const void* WT, const int32_t* nbr, int32_t KN, int32_t N,
+                              float* dA, float* dW, int32_t* err, void* stream) {
+    if (!dZ || !A || !dW || !err || N <= 0 || !corr::aligned(dZ, 16) || !corr::aligned(A, 16)) return FVM_E_ARG;
+    if (dA && (!WT || !nbr || KN <= 0 || KN > 8 || !corr::aligned(dA, 32) || !corr::aligned(WT, 16))) return FVM_E_ARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    return dA ? corr::launch_back_layer<true>(dZ, A, WT, nbr, KN, N, dA, dW, err, s)
+              : corr::launch_back_layer<false>(dZ, A, nullptr, nullptr, 0, N, nullptr, dW, err, s);
+}
+
+extern "C" int fvm_back_gather(const float* dA, const int32_t* nbr, int32_t N, int32_t KN, const float* dh_in,
+                               const float* Z_in, float* bias_in, const float* Z, float* dh, void* dZ, float* bias,
+                               void* stream) {
+    if (!dA || !nbr || !dh_in || !Z_in || !bias_in || !Z || !dh || !dZ || !bias || N <= 0 || KN <= 0 || KN > 8 ||
+        dh == dh_in)
+        return FVM_E_ARG;
+    if (!corr::aligned(dA, 8) || !corr::aligned(dh_in, 8) || !corr::aligned(Z_in, 8) || !corr::aligned(Z, 8) ||
+        !corr::aligned(dh, 8) || !corr::aligned(dZ, 4) || !corr::aligned(bias_in, 8) || !corr::aligned(bias, 8))
+        return FVM_E_ARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    __nv_bfloat16* z = static_cast<__nv_bfloat16*>(dZ);
+#define FVM_CALL(KM) FVM_LAUNCH(KID_CORRECTOR, s, corr::k_back_gather<KM><<<corr::kSumBlocks, corr::kSumThreads, 0, s>>>( \
+                                    dA, nbr, N, KN, dh_in, Z_in, bias_in, Z, dh, z, bias))
+    if (KN <= 3) FVM_CALL(3);
+    else if (KN == 4) FVM_CALL(4);
+    else FVM_CALL(8);
+#undef FVM_CALL
+    return launch_status();
+}
+
+extern "C" int fvm_back_bias(const float* dh, const float* Z, int32_t N, float* bias, void* stream) {
+    if (!dh || !Z || !bias || N <= 0 || !corr::aligned(dh, 8) || !corr::aligned(Z, 8) || !corr::aligned(bias, 8))
+        return FVM_E_ARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    FVM_LAUNCH(KID_CORRECTOR, s, corr::k_back_bias<<<corr::kSumBlocks, corr::kSumThreads, 0, s>>>(dh, Z, N, bias));
+    return launch_status();
+}
+
+extern "C" int fvm_back_finish(int32_t n_sets, const float* const* sets, float* const* dst, const int32_t* n,
+                               void* stream) {
+    if (n_sets < 1 || n_sets > 32 || !sets || !dst || !n) return FVM_E_ARG;
+    corr::FinishArgs f{};
+    for (int q = 0; q < n_sets; ++q) {
+        if (!sets[q] || !dst[q] || n[q] < 1 || n[q] > corr::kLayerW) return FVM_E_ARG;
+        f.set[q] = sets[q];
+        f.dst[q] = dst[q];
+        f.n[q] = n[q];
+    }
+    cudaStream_t s = (cudaStream_t)stream;
+    FVM_LAUNCH(KID_CORRECTOR, s, corr::k_back_finish<<<n_sets, 256, 0, s>>>(f));
     return launch_status();
 }
 

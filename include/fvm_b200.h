@@ -368,6 +368,39 @@ int fvm_gemm_bf16(const void *A, int64_t lda, const void *B, int64_t ldb, int32_
  * mbarrier wait that gives up sets *err (results invalid). */
 int fvm_mp_layer(const float *h, const int32_t *nbr, int32_t M, int32_t KN, const void *Wt, const float *bias,
                  float *h_out, const float *Wo, const float *bo, int32_t O, float *out, int32_t *err, void *stream);
+/* fvm_mp_layer that also keeps what the backward pass reads: the pre-activations Z [M][64] and the
+ * bf16 operand rows A [M][128] (either may be NULL; Z 32-byte, A 16-byte aligned). */
+int fvm_mp_layer_train(const float *h, const int32_t *nbr, int32_t M, int32_t KN, const void *Wt, const float *bias,
+                       float *h_out, float *Z, void *A, const float *Wo, const float *bo, int32_t O, float *out,
+                       int32_t *err, void *stream);
+/* Input layer h_out_i = SiLU(X_i . Wt^T + bias) with X bf16 [M][64], Wt bf16 [64][64] (16-byte aligned);
+ * Z (or NULL) receives the pre-activations.  Bitwise equal to fvm_gemm_bf16 with bias and SiLU. */
+int fvm_in_layer(const void *X, int32_t M, const void *Wt, const float *bias, float *h_out, float *Z, int32_t *err,
+                 void *stream);
+/* Backward pass of the network (64 channels; fp32 rows 8-byte, bf16 rows 16-byte aligned, dA 32-byte).
+ * Sums over the cells use workspace sets of FVM_BACK_SET floats (8-byte aligned, no clearing needed):
+ * one for each bias gradient and O + 1 consecutive ones (`dec`) for the decoder.  A set is filled by a
+ * first and a second pass over the same terms, and fvm_back_finish adds set q's n[q] column sums to
+ * dst[q] (host arrays, at most 32 sets).  A column sum has the value of one fp32 accumulator that
+ * takes the cells in order, whatever the launch shape.
+ *   fvm_back_top:     dh = dOut Wo; dZ (bf16) = dh SiLU'(Z); first pass of dec and bias
+ *   fvm_back_decoder: second pass of dec (dWo[o] = set o, dbo = the last set's first O columns)
+ *   fvm_back_layer:   dW [64][128] += dZ^T A and dA [N][128] = dZ W with columns 64.. divided by the row's
+ *                     neighbour count (WT = bf16 W^T [128][64]); dA = NULL: input layer, A = X [N][64],
+ *                     dW [64][64]
+ *   fvm_back_gather:  dh = dh_in + dA[:, :64] + sum_{j in nbr(i)} dA[j][64:]; dZ = dh SiLU'(Z) with the first
+ *                     pass of bias; second pass of bias_in (dh_in, Z_in).  dh must not alias dh_in.
+ *   fvm_back_bias:    second pass of bias alone (dh, Z) */
+#define FVM_BACK_SET ((296 * 16 + 2 * 296) * 64)
+int fvm_back_top(const float *h, const float *Wo, const float *dOut, const float *Z, int32_t N, int32_t O, float *dh,
+                 void *dZ, float *dec, float *bias, void *stream);
+int fvm_back_decoder(const float *h, const float *dOut, int32_t N, int32_t O, float *dec, void *stream);
+int fvm_back_layer(const void *dZ, const void *A, const void *WT, const int32_t *nbr, int32_t KN, int32_t N, float *dA,
+                   float *dW, int32_t *err, void *stream);
+int fvm_back_gather(const float *dA, const int32_t *nbr, int32_t N, int32_t KN, const float *dh_in, const float *Z_in,
+                    float *bias_in, const float *Z, float *dh, void *dZ, float *bias, void *stream);
+int fvm_back_bias(const float *dh, const float *Z, int32_t N, float *bias, void *stream);
+int fvm_back_finish(int32_t n_sets, const float *const *sets, float *const *dst, const int32_t *n, void *stream);
 /* out[i] = [bf16(h_i), bf16(mean_{j in nbr(i)} h_j)]  (bf16 [N][128]) from the fp32 stream. */
 int fvm_mp_gather_f32(const float *h, const int32_t *nbr, int32_t N, int32_t KN, void *out, void *stream);
 /* dh_out[i] = dh_in[i] + dA[i][:W] + sum_{j in nbr(i)} dA[j][W:] / deg(j)  (fp32; dh_in may be NULL). */
