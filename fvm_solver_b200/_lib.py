@@ -31,7 +31,8 @@ class Mesh(ct.Structure):
         ("n_cases", ct.c_int32)] + [
         (n, _P) for n in ("cell_case", "face_case", "bc_case", "ch_off", "case_mu", "case_mu_b", "case_kappa")] + [
         ("n_owned", ct.c_int32), ("char_scale_given", ct.c_int32), ("case_active", _P),
-        ("cell_lo", ct.c_int32), ("facet_lo", ct.c_int32)]
+        ("cell_lo", ct.c_int32), ("facet_lo", ct.c_int32)] + [
+        (n, _P) for n in ("cell_tiles", "face_tiles", "div_tiles")]
 
 MESH_PTR_FIELDS = [f for f, t in Mesh._fields_ if t is _P]
 

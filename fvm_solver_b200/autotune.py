@@ -142,10 +142,10 @@ def autotune(eq, reps: int = 5, candidates=CANDIDATES, prefetch=PREFETCH, use_ca
 
 
 def reset():
-    """Back to the defaults (256 threads, no prefetch, per-thread record loads, separate facet and
-    divergence kernels) for every tunable kernel."""
+    """Back to the defaults (256 threads, the cell kernel 128, no prefetch, per-thread record loads,
+    separate facet and divergence kernels) for every tunable kernel."""
     for k in KERNELS.values():
-        _install(k, (256, 0))
+        _install(k, (128 if k == "cell" else 256, 0))
     set_variant("div_stage", 0)
 
 

@@ -34,6 +34,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "fvm_common.cuh"
 
@@ -72,6 +73,7 @@ struct L {
     // weights [DIM][KG], displacements [K][DIM], eps
     static constexpr int GC = 0, GV = 4, DISP = GV + DIM * KG, EPS = DISP + K * DIM;
     static constexpr int SELF_SHIFT = 28;                 // own slot: bits 28..30 of the first column
+    static constexpr int CQ = FVM_CELL_QUADS(DIM), FQ = FVM_FACE_QUADS(DIM), DT = FVM_DIV_TILE(DIM);
     // face record offsets
     static constexpr int FA = 0, FB = 1, INVD = 2, SIZE = 3, NRM = 4, XO = 4 + DIM, RA = 4 + 2 * DIM,
                          RB = 4 + 3 * DIM;
@@ -80,7 +82,21 @@ struct L {
         return comp == DIM ? DIM * (DIM + 1) + d : d * (DIM + 1) + (comp < DIM ? comp : DIM);
     }
     static_assert(EPS + 1 <= CR && RB + DIM <= FR && 2 * K <= DR, "record layout");
+    static_assert(CR == 4 * CQ && RB + DIM <= 4 * FQ, "tiled record layout");
 };
+
+// Tiled tables (cell_tiles, face_tiles): 32 items per tile, 16-byte quad q of item i at
+// ((i / 32) * Q + q) * 128 + 4 (i % 32) floats, so a warp reads a quad of 32 consecutive items as 512
+// contiguous bytes.  The L1 serves that in 4 cycles; the same record as a 128-byte row per lane costs
+// one cycle per lane and 256-bit access, 125 against 32 cycles per 32 cell records.
+template <int Q>
+__device__ __forceinline__ const float* quad_ptr(const float* tiles, int i) {
+    return tiles + (int64_t)(i >> 5) * (Q * 128) + 4 * (i & 31);
+}
+__device__ __forceinline__ void ld4_nc(const float* p, float* v) {
+    const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+}
 
 // N consecutive floats -> registers.  Rows whose width is a multiple of 8 floats start on 32-byte
 // boundaries and move with 256-bit accesses (one L1 wavefront per lane-row instead of two); the
@@ -223,16 +239,17 @@ __device__ __forceinline__ void record_tail(const fvm_mesh_t& m, int f, float (&
     for (int q = 0; q < T; ++q) rec[8 + q] = t[q];
 }
 
-// The KG stencil columns of cell i in slot order, from its compact record: the KG - 1 stored
-// neighbour columns with the cell's own index inserted at its slot `own` (selects only, no
+// The KG stencil columns of cell i in slot order, from its compact record (row or tile): the KG - 1
+// stored neighbour columns with the cell's own index inserted at its slot `own` (selects only, no
 // indexing of register arrays by a runtime value).  Items not loaded get the column 0 everywhere.
-template <int DIM>
+template <int DIM, bool TILED>
 __device__ __forceinline__ void next_cols(const fvm_mesh_t& m, int i, int NA, int* cols, int& own,
                                           bool skip_frozen) {
     using Ly = L<DIM>;
     const bool on = i < NA && (!skip_frozen || case_on(m, m.cell_case, i));
     static_assert(Ly::KG - 1 <= 4 && Ly::GC == 0, "columns in the record's first 16 bytes");
-    const int4 q = on ? __ldg(reinterpret_cast<const int4*>(m.cell_rec + (int64_t)i * Ly::CR)) : make_int4(0, 0, 0, 0);
+    const float* r = TILED ? quad_ptr<Ly::CQ>(m.cell_tiles, i) : m.cell_rec + (int64_t)i * Ly::CR;
+    const int4 q = on ? __ldg(reinterpret_cast<const int4*>(r)) : make_int4(0, 0, 0, 0);
     const int nq[4] = {q.x, q.y, q.z, q.w};
     int nb[Ly::KG - 1];
 #pragma unroll
@@ -440,8 +457,9 @@ __global__ void __launch_bounds__(kBlock) k_bc(fvm_mesh_t m, Phys p, const float
 // ------------------------------------------------------------------------------------------
 // Persistent grid-stride loop (one wave of resident blocks): each thread loads the next cell's
 // gradient-stencil columns one iteration ahead, so the neighbour gathers of a cell are issued at
-// the top of its iteration together with its record, one memory round trip instead of two.
-template <int DIM, bool COH>
+// the top of its iteration together with its record, one memory round trip instead of two.  TILED: the
+// record comes from the tiled table, else from the row table.
+template <int DIM, bool COH, bool TILED>
 __device__ __forceinline__ void cell_body(const fvm_mesh_t& m, const Phys& p, const float* __restrict__ prims,
                                           const float* __restrict__ bcv, float* __restrict__ grads,
                                           int32_t* __restrict__ has_grads, int waves) {
@@ -455,11 +473,14 @@ __device__ __forceinline__ void cell_body(const fvm_mesh_t& m, const Phys& p, co
     if (blockIdx.x == 0 && threadIdx.x == 0) *has_grads = 1;
     const bool skip_frozen = frozen_skip(m, NA - lo, stride);
     int cols[KG], own;
-    next_cols<DIM>(m, i, NA, cols, own, skip_frozen);
+    next_cols<DIM, TILED>(m, i, NA, cols, own, skip_frozen);
     for (int64_t tile = blockIdx.x; i < NA; i += stride, tile += gridDim.x) {
-        if (waves > 0) prefetch_tile(m.cell_rec + (int64_t)lo * Ly::CR, NA - lo, Ly::CR, tile + (int64_t)waves * gridDim.x);
+        if (waves > 0 && (!TILED || lo == 0)) {
+            if constexpr (TILED) prefetch_tile(m.cell_tiles, (NA + 31) & ~31, 4 * Ly::CQ, tile + (int64_t)waves * gridDim.x);
+            else prefetch_tile(m.cell_rec + (int64_t)lo * Ly::CR, NA - lo, Ly::CR, tile + (int64_t)waves * gridDim.x);
+        }
         if (m.case_active && !case_on(m, m.cell_case, i)) {
-            next_cols<DIM>(m, i + stride, NA, cols, own, skip_frozen);
+            next_cols<DIM, TILED>(m, i + stride, NA, cols, own, skip_frozen);
             continue;
         }
         float X[KG][RS];
@@ -477,8 +498,14 @@ __device__ __forceinline__ void cell_body(const fvm_mesh_t& m, const Phys& p, co
             for (int k = 1; k < KG; ++k) U[c] = own == k ? X[k][c] : U[c];
         }
         float rec[Ly::CR];
-        ld_vec<Ly::CR>(m.cell_rec + (int64_t)i * Ly::CR, rec);
-        next_cols<DIM>(m, i + stride, NA, cols, own, skip_frozen);
+        if constexpr (TILED) {
+            const float* r = quad_ptr<Ly::CQ>(m.cell_tiles, i);
+#pragma unroll
+            for (int q = 1; q < Ly::CQ; ++q) ld4_nc(r + 128 * q, rec + 4 * q);
+        } else {
+            ld_vec<Ly::CR>(m.cell_rec + (int64_t)i * Ly::CR, rec);
+        }
+        next_cols<DIM, TILED>(m, i + stride, NA, cols, own, skip_frozen);
         float g[DIM][C];
 #pragma unroll
         for (int d = 0; d < DIM; ++d)
@@ -645,12 +672,12 @@ __global__ void __launch_bounds__(kBlock) k_cell_wide(fvm_mesh_t m, Phys p, cons
 // Register budget of the cell kernel: left to ptxas it settles on 64 with a spill in the loop;
 // the budget trades resident warps against registers for the one-ahead loads and the unrolled
 // stencil (chosen by timing on the 1.97 M-tet box).
-template <int DIM>
+template <int DIM, bool TILED>
 __global__ void __maxnreg__(FVM_CELL_MAXNREG) k_cell(fvm_mesh_t m, Phys p, const float* __restrict__ prims,
                                                   const float* __restrict__ bcv, float* __restrict__ grads,
                                                   int32_t* __restrict__ has_grads, int waves) {
     dependency_wait();
-    cell_body<DIM, false>(m, p, prims, bcv, grads, has_grads, waves);
+    cell_body<DIM, false, TILED>(m, p, prims, bcv, grads, has_grads, waves);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -660,9 +687,9 @@ __global__ void __maxnreg__(FVM_CELL_MAXNREG) k_cell(fvm_mesh_t m, Phys p, const
 // ca / cb and both sides' primitives P0, P1 and limited gradients G0, G1 (cell sides; a boundary
 // side's value is read here): the arithmetic of every facet kernel, so all of them give the same
 // bits.
-template <int DIM>
+template <int DIM, int NR>
 __device__ __forceinline__ void face_eval(const fvm_mesh_t& m, const Phys& p, const float* __restrict__ bcv,
-                                          int f, int ca, int cb, const float (&rec)[L<DIM>::FR],
+                                          int f, int ca, int cb, const float (&rec)[NR],
                                           const float (&P0)[L<DIM>::RS], const float (&P1)[L<DIM>::RS],
                                           const float (&G0)[L<DIM>::GS], const float (&G1)[L<DIM>::GS],
                                           float (&F)[L<DIM>::RS]) {
@@ -873,6 +900,52 @@ __device__ __forceinline__ void face_body(const fvm_mesh_t& m, const Phys& p, co
     }
 }
 
+// The same from the tiled table.  (The gathered rows stay whole 256-bit accesses: 64-byte rows in
+// four 128-bit pieces are cheaper for the L1 alone but took 57 against 48 us here, twice the requests
+// in flight for the same bytes; facets sorted by their lower cell measured no faster.)
+template <int DIM>
+__device__ __forceinline__ void face_body_tiled(const fvm_mesh_t& m, const Phys& p, const float* __restrict__ prims,
+                                                const float* __restrict__ bcv, const float* __restrict__ grads,
+                                                float* __restrict__ flux, int waves) {
+    using Ly = L<DIM>;
+    constexpr int RS = Ly::RS, GS = Ly::GS;
+    const int nF = m.n_facets;                            // facets this launch evaluates: [lo, nF)
+    const int lo = m.facet_lo;
+    const int stride = gridDim.x * blockDim.x;
+    int f = lo + blockIdx.x * blockDim.x + threadIdx.x;
+    const bool skip_frozen = frozen_skip(m, nF - lo, stride);
+    float head[4];
+    auto fetch_head = [&](int j) {
+        if (j < nF && (!skip_frozen || case_on(m, m.face_case, j))) ld4_nc(quad_ptr<Ly::FQ>(m.face_tiles, j), head);
+        else head[0] = head[1] = head[2] = head[3] = 0.f;
+    };
+    fetch_head(f);
+    for (int64_t tile = blockIdx.x; f < nF; f += stride, tile += gridDim.x) {
+        if (waves > 0 && lo == 0) prefetch_tile(m.face_tiles, ((int64_t)nF + 31) & ~31, 4 * Ly::FQ, tile + (int64_t)waves * gridDim.x);
+        const int ca = as_int(head[Ly::FA]), cb = as_int(head[Ly::FB]);
+        if (m.case_active && !case_on(m, m.face_case, f)) {
+            fetch_head(f + stride);
+            continue;
+        }
+        const int cell0 = ca >= 0 ? ca : cb;
+        const int cell1 = cb >= 0 ? cb : ca;
+        float P0[RS], P1[RS], G0[GS], G1[GS], rec[4 * Ly::FQ];
+        ld_vec<RS>(prims + (int64_t)cell0 * RS, P0);
+        ld_vec<RS>(prims + (int64_t)cell1 * RS, P1);
+        ld_vec_cg<GS>(grads + (int64_t)cell0 * GS, G0);
+        ld_vec_cg<GS>(grads + (int64_t)cell1 * GS, G1);
+        const float* r = quad_ptr<Ly::FQ>(m.face_tiles, f);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) rec[q] = head[q];
+#pragma unroll
+        for (int q = 1; q < Ly::FQ; ++q) ld4_nc(r + 128 * q, rec + 4 * q);
+        fetch_head(f + stride);
+        float F[RS];
+        face_eval<DIM>(m, p, bcv, f, ca, cb, rec, P0, P1, G0, G1, F);
+        st_vec<RS>(flux + (int64_t)f * RS, F);
+    }
+}
+
 // Facet records staged by the bulk-copy unit.  Each block walks tiles of blockDim.x facets; thread
 // 0 has the next tile's records (one contiguous range) copied into the other half of a two-stage
 // shared-memory ring with cp.async.bulk, completion counted on that stage's mbarrier, while the
@@ -988,13 +1061,14 @@ __global__ void __launch_bounds__(kMaxBlock) k_face_staged(fvm_mesh_t m, Phys p,
 #else
 #define FVM_FACE_BOUNDS __launch_bounds__(kMaxBlock)
 #endif
-template <int DIM>
+template <int DIM, bool TILED>
 __global__ void FVM_FACE_BOUNDS k_face(fvm_mesh_t m, Phys p, const float* __restrict__ prims,
                                                   const float* __restrict__ bcv,
                                                   const float* __restrict__ grads, float* __restrict__ flux,
                                                   int waves) {
     dependency_wait();
-    face_body<DIM, false>(m, p, prims, bcv, grads, flux, waves);
+    if constexpr (TILED) face_body_tiled<DIM>(m, p, prims, bcv, grads, flux, waves);
+    else face_body<DIM, false>(m, p, prims, bcv, grads, flux, waves);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1181,7 +1255,34 @@ enum DivMode { DIV_RESIDUAL = 0, DIV_STAGE = 1, DIV_FINAL = 2, DIV_FINAL_ADAPT =
 // batched reductions may shuffle): each thread loads the next cell's divergence record one iteration
 // ahead, so the flux gathers of a cell start at the top of its iteration.  Single-mesh reductions
 // are accumulated per thread and combined once per block after the loop.
-template <int DIM, int MODE, bool COH>
+// A cell's divergence weights and facet indices.  The tiled form stores 1 / vol once and the signs in
+// the indices' top bits: 2D one quad (three indices, 1 / vol); 3D a quad of indices per cell and the
+// tile's 32 values of 1 / vol after them.
+template <int DIM, bool TILED>
+struct DivRec {
+    float v[TILED ? (DIM == 2 ? 4 : 5) : L<DIM>::DR];
+    __device__ __forceinline__ void load(const fvm_mesh_t& m, int i) {
+        if constexpr (TILED) {
+            const float* t = m.div_tiles + (int64_t)(i >> 5) * (32 * L<DIM>::DT);
+            ld4_nc(t + 4 * (i & 31), v);
+            if constexpr (DIM == 3) v[4] = __ldg(t + 128 + (i & 31));
+        } else {
+            ld_vec<L<DIM>::DR>(m.div_rec + (int64_t)i * L<DIM>::DR, v);
+        }
+    }
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (float& x : v) x = 0.f;
+    }
+    __device__ __forceinline__ int facet(int k) const {
+        return TILED ? as_int(v[k]) & 0x7fffffff : as_int(v[TILED ? 0 : L<DIM>::K + k]);
+    }
+    __device__ __forceinline__ float weight(int k) const {
+        return TILED ? (as_int(v[k]) < 0 ? -v[DIM == 2 ? 3 : 4] : v[DIM == 2 ? 3 : 4]) : v[k];
+    }
+};
+
+template <int DIM, int MODE, bool COH, bool TILED>
 __device__ __forceinline__ void div_body(const fvm_mesh_t& m, const Phys& p, const float* __restrict__ flux,
                                          const StageArgs& a, float* __restrict__ state, float* __restrict__ prims,
                                          float* __restrict__ kbuf, const float* __restrict__ dt,
@@ -1200,40 +1301,36 @@ __device__ __forceinline__ void div_body(const fvm_mesh_t& m, const Phys& p, con
 #pragma unroll
     for (int c = 0; c < (ADAPT ? 3 * C : 1); ++c) ad_acc[c] = 0.0;
     int i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31);
-    float nxt[Ly::DR];
+    DivRec<DIM, TILED> nxt;
     const bool skip_frozen = frozen_skip(m, NA, stride);
-    if (i0 + lane < NA && (!skip_frozen || case_on(m, m.cell_case, i0 + lane)))
-        ld_vec<Ly::DR>(m.div_rec + (int64_t)(i0 + lane) * Ly::DR, nxt);
-    else
-#pragma unroll
-        for (int q = 0; q < Ly::DR; ++q) nxt[q] = 0.f;
+    if (i0 + lane < NA && (!skip_frozen || case_on(m, m.cell_case, i0 + lane))) nxt.load(m, i0 + lane);
+    else nxt.clear();
     for (int64_t tile = blockIdx.x; i0 < NA; i0 += stride, tile += gridDim.x) {
         if (waves > 0) {
-            prefetch_tile(m.div_rec, NA, Ly::DR, tile + (int64_t)waves * gridDim.x);
+            if constexpr (TILED) prefetch_tile(m.div_tiles, (NA + 31) & ~31, Ly::DT, tile + (int64_t)waves * gridDim.x);
+            else prefetch_tile(m.div_rec, NA, Ly::DR, tile + (int64_t)waves * gridDim.x);
             if (MODE != DIV_RESIDUAL) prefetch_tile(state, NA, C, tile + (int64_t)waves * gridDim.x);
         }
         const int i = i0 + lane;
         const bool live = i < NA && (m.case_active == nullptr || case_on(m, m.cell_case, i));
-        float rec[Ly::DR];
-#pragma unroll
-        for (int q = 0; q < Ly::DR; ++q) rec[q] = nxt[q];
+        const DivRec<DIM, TILED> rec = nxt;
         float r[C];
 #pragma unroll
         for (int c = 0; c < C; ++c) r[c] = 0.f;
         if (live) {
 #pragma unroll
             for (int k = 0; k < Ly::K; ++k) {
-                if (k < m.kf) {
-                    const float w = rec[k];
+                if (TILED || k < m.kf) {
+                    const float w = rec.weight(k);
                     float Fk[RS];
-                    ld_vec_cg<RS>(flux + (int64_t)as_int(rec[Ly::K + k]) * RS, Fk);
+                    if constexpr (TILED) ld_vec<RS>(flux + (int64_t)rec.facet(k) * RS, Fk);
+                    else ld_vec_cg<RS>(flux + (int64_t)rec.facet(k) * RS, Fk);
 #pragma unroll
                     for (int c = 0; c < C; ++c) r[c] = fmaf(w, Fk[c], r[c]);
                 }
             }
         }
-        if (i + stride < NA && (!skip_frozen || case_on(m, m.cell_case, i + stride)))
-            ld_vec<Ly::DR>(m.div_rec + (int64_t)(i + stride) * Ly::DR, nxt);
+        if (i + stride < NA && (!skip_frozen || case_on(m, m.cell_case, i + stride))) nxt.load(m, i + stride);
         if (MODE == DIV_RESIDUAL) {
             if (live) store_state<C>(dudt + (int64_t)i * C, r);
             continue;
@@ -1322,7 +1419,7 @@ __device__ __forceinline__ void div_body(const fvm_mesh_t& m, const Phys& p, con
     }
 }
 
-template <int DIM, int MODE>
+template <int DIM, int MODE, bool TILED>
 __global__ void __launch_bounds__(kMaxBlock) k_div_stage(fvm_mesh_t m, Phys p, const float* __restrict__ flux,
                                                        StageArgs a, float* __restrict__ state,
                                                        float* __restrict__ prims, float* __restrict__ kbuf,
@@ -1330,7 +1427,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_div_stage(fvm_mesh_t m, Phys p, c
                                                        double* __restrict__ red,
                                                        float* __restrict__ dudt, int waves) {
     dependency_wait();
-    div_body<DIM, MODE, false>(m, p, flux, a, state, prims, kbuf, dt, red, dudt, waves);
+    div_body<DIM, MODE, false, TILED>(m, p, flux, a, state, prims, kbuf, dt, red, dudt, waves);
 }
 
 // Step-end bookkeeping: adaptive dt (integrators.py:42-62) or CFL dt, conservation sums.
@@ -1497,17 +1594,17 @@ __global__ void __launch_bounds__(kBlock) k_step_fused(fvm_mesh_t m, Phys p, Fus
                 bc_item<DIM, true>(m, p, f.prims, f.grads, f.has_grads, f.bcv, f.red, b, scale);
             grid_barrier(f.bar, f.status);
         }
-        if (m.kg == DIM + 2) cell_body<DIM, true>(m, p, f.prims, f.bcv, f.grads, f.has_grads, 0);
+        if (m.kg == DIM + 2) cell_body<DIM, true, false>(m, p, f.prims, f.bcv, f.grads, f.has_grads, 0);
         else cell_wide_body<DIM, true>(m, p, f.prims, f.bcv, f.grads, f.has_grads);
         grid_barrier(f.bar, f.status);
         face_body<DIM, true>(m, p, f.prims, f.bcv, f.grads, f.flux, 0);
         grid_barrier(f.bar, f.status);
         if (!a.final_)
-            div_body<DIM, DIV_STAGE, true>(m, p, f.flux, a, f.state, f.prims, f.k, f.dt, f.red, nullptr, 0);
+            div_body<DIM, DIV_STAGE, true, false>(m, p, f.flux, a, f.state, f.prims, f.k, f.dt, f.red, nullptr, 0);
         else if (a.adaptive)
-            div_body<DIM, DIV_FINAL_ADAPT, true>(m, p, f.flux, a, f.state, f.prims, f.k, f.dt, f.red, nullptr, 0);
+            div_body<DIM, DIV_FINAL_ADAPT, true, false>(m, p, f.flux, a, f.state, f.prims, f.k, f.dt, f.red, nullptr, 0);
         else
-            div_body<DIM, DIV_FINAL, true>(m, p, f.flux, a, f.state, f.prims, f.k, f.dt, f.red, nullptr, 0);
+            div_body<DIM, DIV_FINAL, true, false>(m, p, f.flux, a, f.state, f.prims, f.k, f.dt, f.red, nullptr, 0);
         grid_barrier(f.bar, f.status);
         if (a.final_ && f.need_final) {
             finalize_body(DIM + 2, f.adaptive, f.atol, f.rtol, f.mtol, f.alpha_hi, f.alpha_lo, f.order, f.cfl, a.cons,
@@ -1694,6 +1791,8 @@ static bool mesh_ok(const fvm_mesh_t* m) {
         return false;
     if (m->n_char > 0 && (!m->ch_cell || !m->ch_normal || !m->ch_rho || !m->ch_vn || !m->ch_p || !m->ch_vt))
         return false;
+    for (const float* t : {m->cell_tiles, m->face_tiles, m->div_tiles})   // read in 16-byte quads
+        if ((uintptr_t)t & 15u) return false;
     if (m->n_cases < 0) return false;
     if (m->n_owned < 0 || m->n_owned > m->n_cells || m->char_scale_given < 0 || m->char_scale_given > 1) return false;
     if (m->n_cases > 0 && (m->n_owned > 0 || m->char_scale_given)) return false;
@@ -1714,8 +1813,9 @@ static inline unsigned blocks_for(int64_t n) { return (unsigned)((n + kBlock - 1
 
 // Threads per block of the cell, facet and divergence kernels (set by the autotuner through
 // fvm_set_block_size).  The boundary kernels keep kBlock: their per-block reduction order must not
-// change between single-mesh and batched runs.
-static int g_block_cell = kBlock, g_block_face = kBlock, g_block_div = kBlock;
+// change between single-mesh and batched runs.  The cell kernel's 96 registers leave 20 warps per SM
+// in blocks of 128 and 16 in blocks of 256 (39.3 against 41.4 us at 855 k cells in 3D).
+static int g_block_cell = 128, g_block_face = kBlock, g_block_div = kBlock;
 // Record prefetch distance in waves of resident blocks per kernel: -1 = default (off: with the
 // persistent kernels' index look-ahead it measured slower on the 2M-tet box), 0 = off.
 static int g_pf_cell = -1, g_pf_face = -1, g_pf_div = -1;
@@ -1760,6 +1860,10 @@ static inline unsigned fin_blocks(const fvm_mesh_t* m) {
     return m->n_cases > 0 ? (unsigned)((m->n_cases + 127) / 128) : 1u;
 }
 
+// The kernels read the tiled tables where the mesh has them (same items, order and bits).
+static inline bool cell_tiled(const fvm_mesh_t* m) { return m->cell_tiles && m->kg == m->dim + 2; }
+static inline bool div_tiled(const fvm_mesh_t* m) { return m->div_tiles && m->kf == m->dim + 1; }
+
 // Boundary values and limited cell gradients for the padded primitives `prims`.
 template <int DIM>
 static int launch_begin(const fvm_mesh_t* m, const Phys& p, const float* prims, float* grads,
@@ -1776,10 +1880,13 @@ static int launch_begin(const fvm_mesh_t* m, const Phys& p, const float* prims, 
         FVM_LAUNCH(KID_CELL, s, launch(k_cell_wide<DIM>, dim3(gw), dim3(kBlock), 0, s, *m, p, prims, w->bc_vals, grads, has_grads));
         return launch_status();
     }
-    const unsigned gc =
-        persistent_grid(owned_cells(m) - m->cell_lo, g_block_cell, wave_blocks(k_cell<DIM>, g_block_cell));
-    FVM_LAUNCH(KID_CELL, s, launch(k_cell<DIM>, dim3(gc), dim3(g_block_cell), 0, s, *m, p, prims, w->bc_vals, grads, has_grads,
-                                                                    waves_of(g_pf_cell)));
+    auto cells = [&](auto kernel) {
+        const unsigned gc = persistent_grid(owned_cells(m) - m->cell_lo, g_block_cell, wave_blocks(kernel, g_block_cell));
+        FVM_LAUNCH(KID_CELL, s, launch(kernel, dim3(gc), dim3(g_block_cell), 0, s, *m, p, prims, w->bc_vals, grads,
+                                       has_grads, waves_of(g_pf_cell)));
+    };
+    if (cell_tiled(m)) cells(k_cell<DIM, true>);
+    else cells(k_cell<DIM, false>);
     return launch_status();
 }
 
@@ -1824,10 +1931,13 @@ static int launch_face(const fvm_mesh_t* m, const Phys& p, const float* prims, c
                                                                                   w->flux));
         return launch_status();
     }
-    const unsigned gf =
-        persistent_grid(m->n_facets - m->facet_lo, g_block_face, wave_blocks(k_face<DIM>, g_block_face));
-    FVM_LAUNCH(KID_FACE, s, launch(k_face<DIM>, dim3(gf), dim3(g_block_face), 0, s, *m, p, prims, w->bc_vals, grads, w->flux,
-                                                                    waves_of(g_pf_face)));
+    auto faces = [&](auto kernel) {
+        const unsigned gf = persistent_grid(m->n_facets - m->facet_lo, g_block_face, wave_blocks(kernel, g_block_face));
+        FVM_LAUNCH(KID_FACE, s, launch(kernel, dim3(gf), dim3(g_block_face), 0, s, *m, p, prims, w->bc_vals, grads, w->flux,
+                                       waves_of(g_pf_face)));
+    };
+    if (m->face_tiles) faces(k_face<DIM, true>);
+    else faces(k_face<DIM, false>);
     return launch_status();
 }
 
@@ -1839,27 +1949,24 @@ static int launch_fluxes(const fvm_mesh_t* m, const Phys& p, const float* prims,
     return rc ? rc : launch_face<DIM>(m, p, prims, grads, w, s);
 }
 
-template <int DIM, int MODE>
-static void launch_div_mode(const fvm_mesh_t* m, const Phys& p, const float* flux, const StageArgs& a, float* state,
-                            float* prims, float* kbuf, const float* dt, double* red, float* dudt, cudaStream_t s) {
-    const unsigned grid =
-        persistent_grid(owned_cells(m), g_block_div, wave_blocks(k_div_stage<DIM, MODE>, g_block_div));
-    FVM_LAUNCH(KID_DIV_STAGE, s, launch(k_div_stage<DIM, MODE>, dim3(grid), dim3(g_block_div), 0, s, 
-                                     *m, p, flux, a, state, prims, kbuf, dt, red, dudt, waves_of(g_pf_div)));
-}
-
 // Divergence (+ stage combination): picks the kernel variant for what the launch must do.
 template <int DIM>
 static int launch_div(const fvm_mesh_t* m, const Phys& p, const float* flux, const StageArgs& a, float* state,
                       float* prims, float* kbuf, const float* dt, double* red, float* dudt, cudaStream_t s) {
-    if (dudt)
-        launch_div_mode<DIM, DIV_RESIDUAL>(m, p, flux, a, state, prims, kbuf, dt, red, dudt, s);
-    else if (!a.final_)
-        launch_div_mode<DIM, DIV_STAGE>(m, p, flux, a, state, prims, kbuf, dt, red, dudt, s);
-    else if (a.adaptive)
-        launch_div_mode<DIM, DIV_FINAL_ADAPT>(m, p, flux, a, state, prims, kbuf, dt, red, dudt, s);
-    else
-        launch_div_mode<DIM, DIV_FINAL>(m, p, flux, a, state, prims, kbuf, dt, red, dudt, s);
+    auto div = [&](auto kernel) {
+        const unsigned grid = persistent_grid(owned_cells(m), g_block_div, wave_blocks(kernel, g_block_div));
+        FVM_LAUNCH(KID_DIV_STAGE, s, launch(kernel, dim3(grid), dim3(g_block_div), 0, s, *m, p, flux, a, state, prims, kbuf,
+                                            dt, red, dudt, waves_of(g_pf_div)));
+    };
+    auto mode = [&](auto t) {
+        constexpr bool T = decltype(t)::value;
+        if (dudt) div(k_div_stage<DIM, DIV_RESIDUAL, T>);
+        else if (!a.final_) div(k_div_stage<DIM, DIV_STAGE, T>);
+        else if (a.adaptive) div(k_div_stage<DIM, DIV_FINAL_ADAPT, T>);
+        else div(k_div_stage<DIM, DIV_FINAL, T>);
+    };
+    if (div_tiled(m)) mode(std::true_type{});
+    else mode(std::false_type{});
     return launch_status();
 }
 

@@ -20,7 +20,7 @@ from .config import ConfigFVM
 from .fvm_mesh import FVMMesh, FVMMesh2D, FVMMesh3D
 from types import SimpleNamespace
 
-from .tables import FVMTables, KernelTables, grad_index, row_sizes
+from .tables import FVMTables, KernelTables, grad_index, row_sizes, tiled_records
 
 
 class FluidConstitution:
@@ -86,7 +86,7 @@ class DeviceMesh:
 
     _struct_fields = [f for f in _lib.MESH_PTR_FIELDS if f not in
                       ("cell_rec", "div_rec", "face_rec", "cell_case", "face_case", "bc_case", "ch_off",
-                       "case_mu", "case_mu_b", "case_kappa", "case_active")]
+                       "case_mu", "case_mu_b", "case_kappa", "case_active", "cell_tiles", "face_tiles", "div_tiles")]
 
     def __init__(self, kt: KernelTables, device, records: dict | None = None):
         """``records``: precomputed device records (default ``kt.records()``)."""
@@ -97,6 +97,7 @@ class DeviceMesh:
         up = {k: v.contiguous().to(self.device) for k, v in (records or kt.records()).items()}
         for f in self._struct_fields:
             up[f] = getattr(kt, f).contiguous().to(self.device)
+        up.update(tiled_records(kt.dim, kt.kg, kt.kf, up))
         self.t = SimpleNamespace(**up)
         m = _lib.Mesh(dim=kt.dim, n_comp=kt.n_comp, n_cells=kt.n_cells, n_facets=kt.n_facets,
                       n_bc=kt.n_bc, n_char=kt.n_char, kg=kt.kg, kf=kt.kf)

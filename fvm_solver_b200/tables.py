@@ -290,6 +290,37 @@ class KernelTables:
         return dict(cell_rec=cell, div_rec=div, face_rec=face)
 
 
+def _tile(rows: torch.Tensor) -> torch.Tensor:
+    """[n][4 Q] -> tiles of 32 items, quad by quad: [ceil(n / 32)][Q][32][4]."""
+    n, w = rows.shape
+    t = torch.zeros(((n + 31) // 32 * 32, w), dtype=torch.float32, device=rows.device)
+    t[:n] = rows
+    return t.view(-1, 32, w // 4, 4).permute(0, 2, 1, 3).contiguous()
+
+
+def tiled_records(dim: int, kg: int, kf: int, rec: dict) -> dict:
+    """The tiled tables of ``include/fvm_b200.h`` from the row records (any device): ``cell_tiles``
+    (the reference's stencil only), ``face_tiles``, and ``div_tiles`` (if every cell has dim + 1 facets
+    and one 1/vol)."""
+    K = dim + 1
+    bits = lambda t: t.to(torch.int32).view(torch.float32)
+    out = {"face_tiles": _tile(rec["face_rec"][:, :4 + 4 * dim])}
+    if kg == dim + 2:
+        out["cell_tiles"] = _tile(rec["cell_rec"])
+    w, ids = rec["div_rec"][:, :K], rec["div_rec"][:, K:2 * K].contiguous().view(torch.int32).long()
+    vol = w[:, :1].abs()
+    if kf == K and bool((w.abs() == vol).all()):
+        ids = ids - (w < 0).long() * (1 << 31)                 # bit 31: the weight's sign
+        if dim == 2:
+            out["div_tiles"] = _tile(torch.cat([bits(ids), vol], 1))
+        else:
+            q = _tile(bits(ids)).view(-1, 128)
+            v = torch.zeros(q.shape[0] * 32, dtype=torch.float32, device=q.device)
+            v[:vol.shape[0]] = vol[:, 0]
+            out["div_tiles"] = torch.cat([q, v.view(-1, 32)], 1).contiguous()
+    return out
+
+
 def record_sizes(dim: int, kg: int | None = None):
     """(cell record, facet record, divergence record) widths in floats.  The reference's stencil
     (kg = dim + 2) has the compact cell record FVM_CELL_REC(dim) (20 / 32); a widened stencil the

@@ -56,6 +56,10 @@ extern "C" {
 #define FVM_CELL_REC_KG(dim, kg) ((((dim) * (kg) + (kg) + ((dim) + 1) * (dim) + 2) + 7) / 8 * 8)
 #define FVM_FACE_REC(dim) ((dim) == 2 ? 16 : 16)
 #define FVM_DIV_REC 8
+/* Tiled tables: 16-byte quads per cell / facet record, floats per cell of the divergence table. */
+#define FVM_CELL_QUADS(dim) ((dim) == 2 ? 5 : 8)
+#define FVM_FACE_QUADS(dim) ((dim) == 2 ? 3 : 4)
+#define FVM_DIV_TILE(dim) ((dim) == 2 ? 4 : 5)
 
 /* Mesh tables (built by fvm_solver_b200/tables.py).  N cells, F facets, Fb boundary facets,
  * Fc characteristic facets, K = dim + 1 facets per cell, KG = kg gradient slots: dim + 2 (the
@@ -124,6 +128,15 @@ typedef struct fvm_mesh {
      * e.g. a part's inner cells and facets while its halo exchange is in flight. */
     int32_t cell_lo;
     int32_t facet_lo;
+    /* Tiled copies of the tables (optional, each may be NULL: the kernels then read the rows above; same
+     * results).  Items come in tiles of 32: quad q (16 bytes) of item i lies at float
+     * ((i / 32) * Q + q) * 128 + 4 * (i % 32), the last tile padded with zeros; 16-byte aligned.
+     *   cell_tiles (read when kg = dim + 2), Q = FVM_CELL_QUADS: the compact cell record.
+     *   face_tiles, Q = FVM_FACE_QUADS: the facet record without its padding.
+     *   div_tiles (read when kf = dim + 1; one 1/vol per cell), FVM_DIV_TILE floats per cell: the
+     *     facet indices with the sign of the weight in bit 31 (2D: three and 1/vol, one quad per
+     *     cell; 3D: four, a quad per cell, and the tile's 32 values of 1/vol after its quads). */
+    const float *cell_tiles, *face_tiles, *div_tiles;
 } fvm_mesh_t;
 
 /* Gas and scheme constants (ConfigFVM fields, time_fvm/config_fvm.py:52-63). */
