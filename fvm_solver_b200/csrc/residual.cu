@@ -320,29 +320,55 @@ __device__ __forceinline__ float limiter_phi(int p, float delta, float dU, float
 // additions is that of 256 threads striding over the facets and a block reduction, whatever the block
 // size (a thread of a smaller block takes several of the 256 parts), so every caller agrees bitwise:
 // single and batched meshes, the boundary kernel, the cell kernel's boundary blocks, the fused step.
-// Four elements of a part are in flight at a time (one dependent pair of loads each).
+// Four elements of a thread are in flight at a time, their cells fetched one step ahead.  (Small on
+// purpose: on small meshes the kernel is bound by latency, and sixteen at a time or prefetches cost
+// it 0.5 us per launch.)
+template <int DIM, bool COH, int NP>
+__device__ __forceinline__ void char_parts(const fvm_mesh_t& m, const Phys& p, const float* prims, int first, int hi,
+                                           int stride, double (&acc)[4]) {
+    constexpr int U = 4;
+    int cell[U];
+    auto fetch = [&](int t) {
+#pragma unroll
+        for (int q = 0; q < U; ++q) cell[q] = t + q * stride < hi ? __ldg(m.ch_cell + t + q * stride) : -1;
+    };
+    fetch(first);
+    for (int t = first; t < hi; t += U * stride) {
+        float T[U];
+        bool on[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) {
+            on[q] = cell[q] >= 0;
+            T[q] = on[q] ? ld1_mut<COH>(prims + (int64_t)cell[q] * L<DIM>::RS + DIM + 1) : 0.f;
+        }
+        fetch(t + U * stride);
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+            if (on[q]) acc[q % NP] += (double)sqrtf(p.gR * T[q]);
+    }
+}
+
 template <int DIM, bool COH = false>
 __device__ __forceinline__ double char_c_sum(const fvm_mesh_t& m, const Phys& p, const float* prims, int lo,
                                              int hi, double* red /* [32] */) {
     constexpr int V = 256;
-    const int lane = threadIdx.x & 31;
-    for (int v = threadIdx.x; v < V; v += blockDim.x) {   // whole warps: blockDim.x is a multiple of 32
-        double acc = 0.0;
-        for (int t = lo + v; t < hi; t += 4 * V) {
-            float T[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int u = t + q * V;
-                T[q] = 0.f;
-                if (u < hi) T[q] = ld1_mut<COH>(prims + (int64_t)__ldg(m.ch_cell + u) * L<DIM>::RS + DIM + 1);
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (t + q * V < hi) acc += (double)sqrtf(p.gR * T[q]);
-        }
+    const int lane = threadIdx.x & 31, B = blockDim.x;
+    auto put = [&](double acc, int v) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
         if (lane == 0) red[v >> 5] = acc;
+    };
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    if (B == 128) {   // element j of thread t: part (t + 128 j) mod 256
+        char_parts<DIM, COH, 2>(m, p, prims, lo + threadIdx.x, hi, B, acc);
+        put(acc[0], threadIdx.x);
+        put(acc[1], threadIdx.x + B);
+    } else {
+        for (int v = threadIdx.x; v < V; v += B) {        // whole warps: B is a multiple of 32
+            acc[0] = 0.0;
+            char_parts<DIM, COH, 1>(m, p, prims, lo + v, hi, V, acc);
+            put(acc[0], v);
+        }
     }
     __syncthreads();
     double x = 0.0;
@@ -1374,6 +1400,100 @@ __device__ __forceinline__ void reduce_batched_item(const fvm_mesh_t& m, const P
     }
 }
 
+// Step-end bookkeeping: adaptive dt (integrators.py:42-62) or CFL dt, conservation sums, by threads
+// `tid` of `nth`.  Batched meshes (n_cases > 0): one thread per case handles its CFL dt and sums.
+// The sums were accumulated by atomics of other blocks (also of the same launch): read through L2,
+// all of a thread's before the first is cleared.
+struct FinArgs {
+    int adaptive, cons, n_cases;
+    float atol, rtol, mtol, alpha_hi, alpha_lo, order, cfl;
+    float* dt;
+    double* cons_out;
+    const uint8_t* active;
+};
+template <int C, bool ADAPT>
+__device__ __forceinline__ void finalize_body(const FinArgs& f, double* red, int tid, int nth) {
+    if (f.n_cases > 0) {
+        for (int c = tid; c < f.n_cases; c += nth) {
+            if (f.active && !f.active[c]) continue;
+            double* slot = red + FVM_RED_DOUBLES + 8 * c;
+            double v[C + 1];
+#pragma unroll
+            for (int k = 0; k <= C; ++k) v[k] = __ldcg(slot + k);
+            if (f.cfl > 0.f) {
+                if (v[0] > 0.0) f.dt[c] = (float)((double)f.cfl / v[0]);
+                slot[0] = 0.0;
+            }
+            if (f.cons) {
+#pragma unroll
+                for (int k = 0; k < C; ++k) {
+                    if (f.cons_out) f.cons_out[c * C + k] = v[1 + k];
+                    slot[1 + k] = 0.0;
+                }
+            }
+        }
+        return;
+    }
+    if (tid != 0) return;
+    double cons[C];
+    const double smax = __ldcg(red + 16);
+#pragma unroll
+    for (int c = 0; c < C; ++c) cons[c] = f.cons ? __ldcg(red + 24 + c) : 0.0;
+    if (ADAPT && f.adaptive) {
+        double s[3 * C], E = 0.0;
+#pragma unroll
+        for (int c = 0; c < 3 * C; ++c) s[c] = __ldcg(red + c);
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            const double nd = sqrt(s[c]), nh = sqrt(s[C + c]), nu = sqrt(s[2 * C + c]);
+            E += nd / ((double)f.atol + (double)f.rtol * nh + (double)f.mtol * nu);
+            red[c] = red[C + c] = red[2 * C + c] = 0.0;
+        }
+        E /= C;
+        const float Ef = (float)E;
+        const float factor = 0.9f * powf(Ef, -1.f / f.order);
+        const float alpha = Ef > 1.f ? f.alpha_hi : f.alpha_lo;
+        f.dt[0] = f.dt[0] * (alpha + (1.f - alpha) * factor);
+        red[40] = E;
+    }
+    if (f.cfl > 0.f) {
+        if (smax > 0.0) f.dt[0] = (float)((double)f.cfl / smax);
+        red[16] = 0.0;
+    }
+    if (f.cons) {
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            if (f.cons_out) f.cons_out[c] = cons[c];
+            red[24 + c] = 0.0;
+        }
+    }
+}
+
+// The last block of a launch to come here (an arrival counter in red[62], left at zero) does the
+// bookkeeping, after every block's atomics.  For the state reductions, whose callers launch them plainly
+// (reduction and k_finalize of 16 cases took 19 us, now 11); the stage kernels keep the overlapped
+// k_finalize, their fence and arrival behind all the state stores cost more than its launch.
+// Block-wide call.
+template <int C>
+__device__ __forceinline__ void finalize_last_block(const FinArgs& f, double* red) {
+    __shared__ int s_last;
+    unsigned* arrived = reinterpret_cast<unsigned*>(red + 62);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(arrived, 1u) + 1u == gridDim.x;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    finalize_body<C, false>(f, red, threadIdx.x, blockDim.x);
+    if (threadIdx.x == 0) *arrived = 0u;
+}
+
+template <int C>
+__global__ void k_finalize(FinArgs f, double* red) {
+    dependency_wait();
+    finalize_body<C, true>(f, red, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+
 // What one k_div_stage launch does after the divergence.
 enum DivMode { DIV_RESIDUAL = 0, DIV_STAGE = 1, DIV_FINAL = 2, DIV_FINAL_ADAPT = 3 };
 
@@ -1556,68 +1676,6 @@ __global__ void __launch_bounds__(kMaxBlock) k_div_stage(fvm_mesh_t m, Phys p, c
     div_body<DIM, MODE, false, TILED>(m, p, flux, a, state, prims, kbuf, dt, red, dudt, waves);
 }
 
-// Step-end bookkeeping: adaptive dt (integrators.py:42-62) or CFL dt, conservation sums.
-// Batched meshes (n_cases > 0): one thread per case handles its CFL dt and sums.
-// The sums were accumulated by atomics of other blocks (in the fused step, of the same launch):
-// read them through L2.
-__device__ __forceinline__ void finalize_body(int C, int adaptive, float atol, float rtol, float mtol,
-                                              float alpha_hi, float alpha_lo, float order, float cfl, int cons,
-                                              double* red, float* dt, double* cons_out, int n_cases,
-                                              const uint8_t* __restrict__ active) {
-    if (n_cases > 0) {
-        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n_cases; c += gridDim.x * blockDim.x) {
-            if (active && !active[c]) continue;
-            double* slot = red + FVM_RED_DOUBLES + 8 * c;
-            if (cfl > 0.f) {
-                const double smax = __ldcg(slot);
-                if (smax > 0.0) dt[c] = (float)((double)cfl / smax);
-                slot[0] = 0.0;
-            }
-            if (cons) {
-                for (int k = 0; k < C; ++k) {
-                    if (cons_out) cons_out[c * C + k] = __ldcg(slot + 1 + k);
-                    slot[1 + k] = 0.0;
-                }
-            }
-        }
-        return;
-    }
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (adaptive) {
-        double E = 0.0;
-        for (int c = 0; c < C; ++c) {
-            const double nd = sqrt(__ldcg(red + c)), nh = sqrt(__ldcg(red + C + c)), nu = sqrt(__ldcg(red + 2 * C + c));
-            E += nd / ((double)atol + (double)rtol * nh + (double)mtol * nu);
-            red[c] = red[C + c] = red[2 * C + c] = 0.0;
-        }
-        E /= C;
-        const float Ef = (float)E;
-        const float factor = 0.9f * powf(Ef, -1.f / order);
-        const float alpha = Ef > 1.f ? alpha_hi : alpha_lo;
-        dt[0] = dt[0] * (alpha + (1.f - alpha) * factor);
-        red[40] = E;
-    }
-    if (cfl > 0.f) {
-        const double smax = __ldcg(red + 16);
-        if (smax > 0.0) dt[0] = (float)((double)cfl / smax);
-        red[16] = 0.0;
-    }
-    if (cons) {
-        for (int c = 0; c < C; ++c) {
-            if (cons_out) cons_out[c] = __ldcg(red + 24 + c);
-            red[24 + c] = 0.0;
-        }
-    }
-}
-
-__global__ void k_finalize(int C, int adaptive, float atol, float rtol, float mtol, float alpha_hi,
-                           float alpha_lo, float order, float cfl, int cons, double* red, float* dt,
-                           double* cons_out, int n_cases, const uint8_t* __restrict__ active) {
-    dependency_wait();
-    finalize_body(C, adaptive, atol, rtol, mtol, alpha_hi, alpha_lo, order, cfl, cons, red, dt, cons_out, n_cases,
-                  active);
-}
-
 // ------------------------------------------------------------------------------------------
 // Fused step: every phase of every stage of one step in one cooperative launch.
 //
@@ -1733,8 +1791,9 @@ __global__ void __launch_bounds__(kBlock) k_step_fused(fvm_mesh_t m, Phys p, Fus
             div_body<DIM, DIV_FINAL, true, false>(m, p, f.flux, a, f.state, f.prims, f.k, f.dt, f.red, nullptr, 0);
         grid_barrier(f.bar, f.status);
         if (a.final_ && f.need_final) {
-            finalize_body(DIM + 2, f.adaptive, f.atol, f.rtol, f.mtol, f.alpha_hi, f.alpha_lo, f.order, f.cfl, a.cons,
-                          f.red, f.dt, f.cons, m.n_cases, m.case_active);
+            const FinArgs fa{f.adaptive, a.cons, m.n_cases, f.atol, f.rtol, f.mtol, f.alpha_hi, f.alpha_lo, f.order,
+                             f.cfl, f.dt, f.cons, m.case_active};
+            finalize_body<DIM + 2, true>(fa, f.red, tid, nth);
             grid_barrier(f.bar, f.status);
         }
     }
@@ -1773,7 +1832,7 @@ __global__ void __launch_bounds__(kBlock) k_pad_prims(int N, const float* __rest
 // into the per-case slots (reduce_batched_item).
 template <int DIM>
 __global__ void __launch_bounds__(kBlock) k_reduce_state(fvm_mesh_t m, Phys p, const float* __restrict__ state,
-                                                          int want_cfl, int want_cons, double* red) {
+                                                          int want_cfl, int want_cons, double* red, FinArgs fin) {
     constexpr int C = DIM + 2;
     const int NA = m.n_owned > 0 ? m.n_owned : m.n_cells;
     const int stride = gridDim.x * blockDim.x;
@@ -1803,6 +1862,7 @@ __global__ void __launch_bounds__(kBlock) k_reduce_state(fvm_mesh_t m, Phys p, c
             sp = block_max(sp, smem);
             if (threadIdx.x == 0) atomic_max_pos(red + 16, sp);
         }
+        finalize_last_block<C>(fin, red);
         return;
     }
     // Batched: each warp takes one contiguous chunk of cells and accumulates per lane while the
@@ -1874,6 +1934,7 @@ __global__ void __launch_bounds__(kBlock) k_reduce_state(fvm_mesh_t m, Phys p, c
         }
     }
     flush();
+    finalize_last_block<C>(fin, red);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -2189,12 +2250,29 @@ static StageArgs stage_args(const fvm_tableau_t* tab, int s) {
     return a;
 }
 
-static int finalize_impl(const fvm_mesh_t* m, const fvm_tableau_t* tab, const fvm_solver_bufs_t* b,
-                         const fvm_work_t* w, int cons, cudaStream_t st) {
-    FVM_LAUNCH(KID_FINALIZE, st,
-               launch(k_finalize, dim3(fin_blocks(m)), dim3(128), 0, st, m->n_comp, tab->adaptive, tab->atol, tab->rtol, tab->mtol,
-                                                         tab->alpha_hi_err, tab->alpha_lo_err, tab->order, tab->cfl,
-                                                         cons, w->red, b->dt, b->cons, m->n_cases, m->case_active));
+static FinArgs fin_args(const fvm_mesh_t* m, const fvm_tableau_t* tab, const fvm_solver_bufs_t* b, int cons) {
+    FinArgs f{};
+    f.adaptive = tab->adaptive;
+    f.cons = cons;
+    f.n_cases = m->n_cases;
+    f.atol = tab->atol;
+    f.rtol = tab->rtol;
+    f.mtol = tab->mtol;
+    f.alpha_hi = tab->alpha_hi_err;
+    f.alpha_lo = tab->alpha_lo_err;
+    f.order = tab->order;
+    f.cfl = tab->cfl;
+    f.dt = b->dt;
+    f.cons_out = b->cons;
+    f.active = m->case_active;
+    return f;
+}
+
+static int finalize_impl(const fvm_mesh_t* m, const FinArgs& f, double* red, cudaStream_t st) {
+    if (m->dim == 2)
+        FVM_LAUNCH(KID_FINALIZE, st, launch(k_finalize<4>, dim3(fin_blocks(m)), dim3(128), 0, st, f, red));
+    else
+        FVM_LAUNCH(KID_FINALIZE, st, launch(k_finalize<5>, dim3(fin_blocks(m)), dim3(128), 0, st, f, red));
     return launch_status();
 }
 
@@ -2209,7 +2287,8 @@ static int stage_finish(const fvm_mesh_t* m, const Phys& p, const fvm_tableau_t*
     a.cons = a.final_ && b->cons != nullptr;
     rc = launch_div<DIM>(m, p, w->flux, a, b->state, b->prims, b->k, b->dt, w->red, nullptr, st);
     if (rc) return rc;
-    if (finalize && a.final_ && (a.adaptive || a.cfl || a.cons)) rc = finalize_impl(m, tab, b, w, a.cons, st);
+    if (finalize && a.final_ && (a.adaptive || a.cfl || a.cons))
+        rc = finalize_impl(m, fin_args(m, tab, b, a.cons), w->red, st);
     return rc;
 }
 
@@ -2237,7 +2316,8 @@ static int stage_phase_impl(const fvm_mesh_t* m, const Phys& p, const fvm_tablea
         a.cons = a.final_ && b->cons != nullptr;
         rc = launch_div<DIM>(&mm, p, w->flux, a, b->state, b->prims, b->k, b->dt, w->red, nullptr, st);
         if (rc) return rc;
-        if (finalize && a.final_ && (a.adaptive || a.cfl || a.cons)) rc = finalize_impl(&mm, tab, b, w, a.cons, st);
+        if (finalize && a.final_ && (a.adaptive || a.cfl || a.cons))
+            rc = finalize_impl(&mm, fin_args(&mm, tab, b, a.cons), w->red, st);
     }
     return rc;
 }
@@ -2279,14 +2359,15 @@ static int multistep_impl(const fvm_mesh_t* m, const Phys& p, int store, int n_t
     }
     a.cons = b->cons != nullptr;
     rc = launch_div<DIM>(m, p, w->flux, a, b->state, b->prims, b->k, b->dt, w->red, nullptr, st);
-    if (rc) return rc;
-    if (a.cons) {
-        FVM_LAUNCH(KID_FINALIZE, st, launch(k_finalize, dim3(fin_blocks(m)), dim3(128), 0, st, m->n_comp, 0, 0.f, 0.f, 0.f, 0.f, 0.f,
-                                                                              1.f, 0.f, 1, w->red, b->dt, b->cons,
-                                                                              m->n_cases, m->case_active));
-        rc = launch_status();
-    }
-    return rc;
+    if (rc || !a.cons) return rc;
+    FinArgs fin{};
+    fin.cons = 1;
+    fin.n_cases = m->n_cases;
+    fin.order = 1.f;
+    fin.dt = b->dt;
+    fin.cons_out = b->cons;
+    fin.active = m->case_active;
+    return finalize_impl(m, fin, w->red, st);
 }
 
 }  // namespace fvm
@@ -2463,7 +2544,7 @@ extern "C" int fvm_stage_finalize(const fvm_mesh_t* mesh, const fvm_tableau_t* t
                                   const fvm_work_t* work, void* stream) {
     if (!mesh_ok(mesh) || !tab_ok(tab) || !bufs_ok(bufs) || !work || !work->red) return FVM_E_ARG;
     if (!(tab->adaptive || tab->cfl > 0.f || bufs->cons)) return FVM_OK;
-    return finalize_impl(mesh, tab, bufs, work, bufs->cons != nullptr, (cudaStream_t)stream);
+    return finalize_impl(mesh, fin_args(mesh, tab, bufs, bufs->cons != nullptr), work->red, (cudaStream_t)stream);
 }
 
 extern "C" int fvm_multistep(const fvm_mesh_t* mesh, const fvm_physics_t* phys, int32_t store,
@@ -2622,42 +2703,38 @@ extern "C" int fvm_state_to_prims(const fvm_mesh_t* mesh, const fvm_physics_t* p
     return launch_status();
 }
 
+// The state's CFL maximum and / or conservation sums, and the bookkeeping that turns them into dt / sums.
+static int reduce_impl(const fvm_mesh_t* mesh, const Phys& p, const float* state, const FinArgs& f, double* red,
+                       cudaStream_t st) {
+    if (mesh->dim == 2)
+        FVM_LAUNCH(KID_REDUCE_STATE, st, k_reduce_state<2><<<reduce_grid<2>(mesh), kBlock, 0, st>>>(
+                                             *mesh, p, state, f.cfl > 0.f, f.cons, red, f));
+    else
+        FVM_LAUNCH(KID_REDUCE_STATE, st, k_reduce_state<3><<<reduce_grid<3>(mesh), kBlock, 0, st>>>(
+                                             *mesh, p, state, f.cfl > 0.f, f.cons, red, f));
+    return launch_status();
+}
+
 extern "C" int fvm_cfl_dt(const fvm_mesh_t* mesh, const fvm_physics_t* phys, const float* state, float cfl,
                           float* dt, const fvm_work_t* work, void* stream) {
     if (!mesh_ok(mesh) || !phys || !state || !dt || !work || !work->red || !(cfl > 0.f)) return FVM_E_ARG;
-    const Phys p = make_phys(phys);
-    cudaStream_t st = (cudaStream_t)stream;
-    if (mesh->dim == 2)
-        FVM_LAUNCH(KID_REDUCE_STATE, st, k_reduce_state<2><<<reduce_grid<2>(mesh), kBlock, 0, st>>>(
-                                             *mesh, p, state, 1, 0, work->red));
-    else
-        FVM_LAUNCH(KID_REDUCE_STATE, st, k_reduce_state<3><<<reduce_grid<3>(mesh), kBlock, 0, st>>>(
-                                             *mesh, p, state, 1, 0, work->red));
-    int rc = launch_status();
-    if (rc) return rc;
-    FVM_LAUNCH(KID_FINALIZE, st, launch(k_finalize, dim3(fin_blocks(mesh)), dim3(128), 0, st, mesh->n_comp, 0, 0.f, 0.f, 0.f, 0.f,
-                                                                             0.f, 1.f, cfl, 0, work->red, dt,
-                                                                             nullptr, mesh->n_cases, nullptr));
-    return launch_status();
+    FinArgs f{};
+    f.n_cases = mesh->n_cases;
+    f.order = 1.f;
+    f.cfl = cfl;
+    f.dt = dt;
+    return reduce_impl(mesh, make_phys(phys), state, f, work->red, (cudaStream_t)stream);
 }
 
 extern "C" int fvm_conservation(const fvm_mesh_t* mesh, const float* state, double* out, const fvm_work_t* work,
                                 void* stream) {
     if (!mesh_ok(mesh) || !state || !out || !work || !work->red) return FVM_E_ARG;
-    Phys p{};
-    cudaStream_t st = (cudaStream_t)stream;
-    if (mesh->dim == 2)
-        FVM_LAUNCH(KID_REDUCE_STATE, st, k_reduce_state<2><<<reduce_grid<2>(mesh), kBlock, 0, st>>>(
-                                             *mesh, p, state, 0, 1, work->red));
-    else
-        FVM_LAUNCH(KID_REDUCE_STATE, st, k_reduce_state<3><<<reduce_grid<3>(mesh), kBlock, 0, st>>>(
-                                             *mesh, p, state, 0, 1, work->red));
-    int rc = launch_status();
-    if (rc) return rc;
-    FVM_LAUNCH(KID_FINALIZE, st, launch(k_finalize, dim3(fin_blocks(mesh)), dim3(128), 0, st, mesh->n_comp, 0, 0.f, 0.f, 0.f, 0.f,
-                                                                             0.f, 1.f, 0.f, 1, work->red, nullptr,
-                                                                             out, mesh->n_cases, nullptr));
-    return launch_status();
+    FinArgs f{};
+    f.cons = 1;
+    f.n_cases = mesh->n_cases;
+    f.order = 1.f;
+    f.cons_out = out;
+    return reduce_impl(mesh, Phys{}, state, f, work->red, (cudaStream_t)stream);
 }
 
 extern "C" int fvm_residual_noalloc(const fvm_mesh_t* mesh, const fvm_physics_t* phys, const float* prims,
