@@ -15,72 +15,157 @@
 
 namespace fvm {
 
-// Every kernel is templated on an upper bound KT of the slot count (4, 8 or 16) and unrolls the
+// Every kernel is templated on an upper bound KT of the slot count (2, 4, 5, 8 or 16; five slots are the
+// widest rows of the residual's operators) and unrolls the
 // slot loop, so the values, columns and gathers of all slots of a row are in flight together (one
-// dependent round trip per row instead of K); slots are summed in order k = 0, 1, ... as before.
-template <int KT>
-__global__ void __launch_bounds__(kBlock) k_ell_spmv(const float* __restrict__ vals,
-                                                      const int32_t* __restrict__ cols, int64_t M,
-                                                      int K, const float* __restrict__ x,
-                                                      int64_t incx, const float* __restrict__ bias,
-                                                      float* __restrict__ y, int64_t incy) {
-    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (r >= M) return;
-    float v[KT], xv[KT];
+// dependent round trip per row instead of K); slots are summed in order k = 0, 1, ...
+//
+// The products are bound by memory (8 K bytes of values and columns per row), but with a row or two
+// per thread and one block after the other they ran at the pace of the two round trips: 22 us for
+// 1.3 M rows of five slots whose bytes take 9.  So one wave of blocks walks the rows (kEllBlocks per SM)
+// and a thread loads the values and columns of its next RT rows (a block apart, so that each access
+// stays contiguous over the warp) before it gathers for the current ones.  On the operators of a
+// 438 k-tet box: facet gradient (4.4 M rows of two slots) 41 -> 22 us, cell gradient (1.3 M rows of
+// five) 21 -> 14 us, with five columns 26 -> 19 us, divergence with five columns 14 -> 11 us.
+constexpr int kEllBlocks = 4;
+
+template <int KT, int RT>
+struct EllRows {
+    float v[RT][KT];
+    int c[RT][KT];
+    __device__ __forceinline__ void load(const float* __restrict__ vals, const int32_t* __restrict__ cols, int64_t M,
+                                         int K, int64_t r0) {
 #pragma unroll
-    for (int k = 0; k < KT; ++k) {
-        v[k] = 0.f;
-        xv[k] = 0.f;
-        if (k < K) {
-            v[k] = __ldg(vals + k * M + r);
-            xv[k] = __ldg(x + (int64_t)__ldg(cols + k * M + r) * incx);
+        for (int j = 0; j < RT; ++j)
+#pragma unroll
+            for (int k = 0; k < KT; ++k) {
+                const int64_t r = r0 + j * kBlock;
+                const bool on = k < K && r < M;
+                v[j][k] = on ? __ldg(vals + k * M + r) : 0.f;
+                c[j][k] = on ? __ldg(cols + k * M + r) : 0;
+            }
+    }
+};
+
+template <int KT, int RT>
+__global__ void __launch_bounds__(kBlock, kEllBlocks) k_ell_spmv(const float* __restrict__ vals,
+                                                                  const int32_t* __restrict__ cols, int64_t M,
+                                                                  int K, const float* __restrict__ x,
+                                                                  int64_t incx, const float* __restrict__ bias,
+                                                                  float* __restrict__ y, int64_t incy) {
+    const int64_t step = (int64_t)gridDim.x * (kBlock * RT);
+    int64_t r0 = blockIdx.x * (int64_t)(kBlock * RT) + threadIdx.x;
+    EllRows<KT, RT> next;
+    next.load(vals, cols, M, K, r0);
+    for (; r0 < M; r0 += step) {
+        const EllRows<KT, RT> cur = next;
+        float xv[RT][KT], b[RT];
+#pragma unroll
+        for (int j = 0; j < RT; ++j) {
+            const bool on = r0 + j * kBlock < M;
+            b[j] = on && bias ? __ldg(bias + r0 + j * kBlock) : 0.f;
+#pragma unroll
+            for (int k = 0; k < KT; ++k) xv[j][k] = on && k < K ? __ldg(x + (int64_t)cur.c[j][k] * incx) : 0.f;
+        }
+        next.load(vals, cols, M, K, r0 + step);
+#pragma unroll
+        for (int j = 0; j < RT; ++j) {
+            const int64_t r = r0 + j * kBlock;
+            if (r >= M) break;
+            float acc = 0.f;
+#pragma unroll
+            for (int k = 0; k < KT; ++k)
+                if (k < K) acc = fmaf(cur.v[j][k], xv[j][k], acc);
+            if (bias) acc += b[j];
+            y[r * incy] = acc;
         }
     }
-    float acc = 0.f;
-#pragma unroll
-    for (int k = 0; k < KT; ++k)
-        if (k < K) acc = fmaf(v[k], xv[k], acc);
-    if (bias) acc += __ldg(bias + r);
-    y[r * incy] = acc;
 }
 
 // One thread per (row, group of CB columns).
 template <int KT, int CB>
-__global__ void __launch_bounds__(kBlock) k_ell_spmm(const float* __restrict__ vals,
+__global__ void __launch_bounds__(kBlock, KT <= 8 ? kEllBlocks : 1) k_ell_spmm(const float* __restrict__ vals,
                                                       const int32_t* __restrict__ cols, int64_t M,
                                                       int K, const float* __restrict__ X,
                                                       int64_t ldx, int B,
                                                       const float* __restrict__ bias,
                                                       float* __restrict__ Y, int64_t ldy) {
-    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (r >= M) return;
+    const int64_t step = (int64_t)gridDim.x * kBlock;
+    int64_t r = blockIdx.x * (int64_t)kBlock + threadIdx.x;
     const int c0 = blockIdx.y * CB;
     const int nb = min(CB, B - c0);
-    float v[KT];
-    int64_t xo[KT];
+    EllRows<KT, 1> next;
+    next.load(vals, cols, M, K, r);
+    for (; r < M; r += step) {
+        const EllRows<KT, 1> cur = next;
+        next.load(vals, cols, M, K, r + step);
+        float acc[CB];
 #pragma unroll
-    for (int k = 0; k < KT; ++k) {
-        v[k] = k < K ? __ldg(vals + k * M + r) : 0.f;
-        xo[k] = k < K ? (int64_t)__ldg(cols + k * M + r) * ldx + c0 : 0;
-    }
-    float acc[CB];
+        for (int j = 0; j < CB; ++j) acc[j] = 0.f;
 #pragma unroll
-    for (int j = 0; j < CB; ++j) acc[j] = 0.f;
+        for (int k = 0; k < KT; ++k) {
+            if (k >= K) break;
+            float xr[CB];
+            const float* xk = X + (int64_t)cur.c[0][k] * ldx + c0;
 #pragma unroll
-    for (int k = 0; k < KT; ++k) {
-        if (k >= K) break;
-        float xr[CB];
+            for (int j = 0; j < CB; ++j) xr[j] = j < nb ? __ldg(xk + j) : 0.f;
 #pragma unroll
-        for (int j = 0; j < CB; ++j) xr[j] = j < nb ? __ldg(X + xo[k] + j) : 0.f;
+            for (int j = 0; j < CB; ++j)
+                if (j < nb) acc[j] = fmaf(cur.v[0][k], xr[j], acc[j]);
+        }
+        const float b = bias ? __ldg(bias + r) : 0.f;
+        float* yr = Y + r * ldy + c0;
 #pragma unroll
         for (int j = 0; j < CB; ++j)
-            if (j < nb) acc[j] = fmaf(v[k], xr[j], acc[j]);
+            if (j < nb) yr[j] = bias ? acc[j] + b : acc[j];
     }
-    float b = bias ? __ldg(bias + r) : 0.f;
-    float* yr = Y + r * ldy + c0;
+}
+
+// Five columns (the 3D variables).  A slot's five floats start on any 4-byte boundary; they lie in two
+// consecutive 16-byte words, which are loaded whole and shifted into place: five scalar gathers per
+// slot cost the L1 41-70 cycles per warp (rows in random order), the two words 17-21.  Both words hold
+// at least one of the five floats, so neither leaves the memory the row itself lies in.
+constexpr int spmm5_blocks(int KT) { return KT <= 4 ? 3 : 2; }   // per SM: 40 gathered floats of a row in registers
+
+template <int KT>
+__global__ void __launch_bounds__(kBlock, spmm5_blocks(KT)) k_ell_spmm5(const float* __restrict__ vals,
+                                                         const int32_t* __restrict__ cols, int64_t M,
+                                                         int K, const float* __restrict__ X, int64_t ldx,
+                                                         const float* __restrict__ bias,
+                                                         float* __restrict__ Y, int64_t ldy) {
+    const int64_t step = (int64_t)gridDim.x * kBlock;
+    int64_t r = blockIdx.x * (int64_t)kBlock + threadIdx.x;
+    EllRows<KT, 1> next;
+    next.load(vals, cols, M, K, r);
+    for (; r < M; r += step) {
+        const EllRows<KT, 1> cur = next;
+        float4 w[KT][2];
+        int sh[KT];
 #pragma unroll
-    for (int j = 0; j < CB; ++j)
-        if (j < nb) yr[j] = bias ? acc[j] + b : acc[j];
+        for (int k = 0; k < KT; ++k) {
+            const uintptr_t a = reinterpret_cast<uintptr_t>(X + (int64_t)cur.c[0][k] * ldx);
+            const float4* q = reinterpret_cast<const float4*>(a & ~(uintptr_t)15);
+            sh[k] = (int)(a >> 2) & 3;
+            w[k][0] = k < K ? __ldg(q) : make_float4(0.f, 0.f, 0.f, 0.f);
+            w[k][1] = k < K ? __ldg(q + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        next.load(vals, cols, M, K, r + step);
+        const float b = bias ? __ldg(bias + r) : 0.f;
+        float acc[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int k = 0; k < KT; ++k) {
+            if (k >= K) break;
+            const float f[8] = {w[k][0].x, w[k][0].y, w[k][0].z, w[k][0].w, w[k][1].x, w[k][1].y, w[k][1].z, w[k][1].w};
+            float t[7];
+#pragma unroll
+            for (int j = 0; j < 7; ++j) t[j] = sh[k] & 1 ? f[j + 1] : f[j];
+#pragma unroll
+            for (int j = 0; j < 5; ++j) acc[j] = fmaf(cur.v[0][k], sh[k] & 2 ? t[j + 2] : t[j], acc[j]);
+        }
+        float* yr = Y + r * ldy;
+#pragma unroll
+        for (int j = 0; j < 5; ++j) yr[j] = bias ? acc[j] + b : acc[j];
+    }
 }
 
 // Specialisation for 4 contiguous, 16-byte aligned columns: one float4 gather per slot.
@@ -217,19 +302,41 @@ extern "C" const char* fvm_version(void) { return "fvm_b200 1.0 sm_100a"; }
 
 using fvm::launch_status;
 
+// One wave of blocks over M rows, `rows` per thread (0: no device).
+static int64_t ell_grid(int64_t M, int rows, int per_sm) {
+    static int sms[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if (!sms[dev] && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    const int64_t all = (M + (int64_t)fvm::kBlock * rows - 1) / ((int64_t)fvm::kBlock * rows), wave = (int64_t)sms[dev] * per_sm;
+    return all < wave ? all : wave;
+}
+
 extern "C" int fvm_ell_spmv(const float* vals, const int32_t* cols, int64_t M, int32_t K,
                             const float* x, int64_t incx, const float* bias, float* y, int64_t incy,
                             void* stream) {
     if (M < 0 || K < 0 || (M > 0 && (!vals && K > 0)) || (M > 0 && (!x || !y))) return FVM_E_ARG;
     if (M == 0) return FVM_OK;
     if (K > FVM_MAX_ELL_K) return FVM_E_UNSUPPORTED;
-    const int64_t grid = (M + fvm::kBlock - 1) / fvm::kBlock;
     cudaStream_t s = (cudaStream_t)stream;
-#define FVM_SPMV(KT) FVM_LAUNCH(fvm::KID_ELL_SPMV, s, fvm::k_ell_spmv<KT><<<(unsigned)grid, fvm::kBlock, 0, s>>>( \
-                                    vals, cols, M, K, x, incx, bias, y, incy))
-    if (K <= 4) FVM_SPMV(4);
-    else if (K <= 8) FVM_SPMV(8);
-    else FVM_SPMV(16);
+    if (ell_grid(M, 1, 1) < 1) {
+        launch_status();
+        return FVM_E_CUDA;
+    }
+    // several rows per thread only where every SM still gets its blocks
+#define FVM_SPMV_R(KT, RT) FVM_LAUNCH(fvm::KID_ELL_SPMV, s, fvm::k_ell_spmv<KT, RT><<<(unsigned)ell_grid(M, RT, fvm::kEllBlocks), \
+                                      fvm::kBlock, 0, s>>>(vals, cols, M, K, x, incx, bias, y, incy))
+#define FVM_SPMV(KT, RT)                                                                                \
+    do {                                                                                                \
+        if (RT > 1 && M >= 148LL * fvm::kEllBlocks * fvm::kBlock * RT) FVM_SPMV_R(KT, RT);              \
+        else FVM_SPMV_R(KT, 1);                                                                         \
+    } while (0)
+    if (K <= 2) FVM_SPMV(2, 4);
+    else if (K <= 4) FVM_SPMV(4, 2);
+    else if (K <= 5) FVM_SPMV(5, 1);
+    else if (K <= 8) FVM_SPMV(8, 1);
+    else FVM_SPMV(16, 1);
+#undef FVM_SPMV_R
 #undef FVM_SPMV
     return launch_status();
 }
@@ -243,6 +350,11 @@ extern "C" int fvm_ell_spmm(const float* vals, const int32_t* cols, int64_t M, i
     const int64_t gx = (M + fvm::kBlock - 1) / fvm::kBlock;
     cudaStream_t s = (cudaStream_t)stream;
     if (K > FVM_MAX_ELL_K) return FVM_E_UNSUPPORTED;
+    const int64_t gw = ell_grid(M, 1, fvm::kEllBlocks);
+    if (gw < 1) {
+        launch_status();
+        return FVM_E_CUDA;
+    }
     const bool aligned = ((uintptr_t)X % 16 == 0) && ((uintptr_t)Y % 16 == 0);
     if (B == 4 && ldx == 4 && ldy == 4 && aligned) {
 #define FVM_SPMM4(KT) FVM_LAUNCH(fvm::KID_ELL_SPMM, s, fvm::k_ell_spmm4<KT><<<(unsigned)gx, fvm::kBlock, 0, s>>>( \
@@ -251,9 +363,15 @@ extern "C" int fvm_ell_spmm(const float* vals, const int32_t* cols, int64_t M, i
         else if (K <= 8) FVM_SPMM4(8);
         else FVM_SPMM4(16);
 #undef FVM_SPMM4
+    } else if (B == 5 && K <= 5) {
+#define FVM_SPMM5(KT) FVM_LAUNCH(fvm::KID_ELL_SPMM, s, fvm::k_ell_spmm5<KT><<<(unsigned)ell_grid(M, 1, fvm::spmm5_blocks(KT)), \
+                                     fvm::kBlock, 0, s>>>(vals, cols, M, K, X, ldx, bias, Y, ldy))
+        if (K <= 4) FVM_SPMM5(4);
+        else FVM_SPMM5(5);
+#undef FVM_SPMM5
     } else {
         const unsigned gy = (unsigned)((B + 7) / 8);
-#define FVM_SPMM(KT) FVM_LAUNCH(fvm::KID_ELL_SPMM, s, fvm::k_ell_spmm<KT, 8><<<dim3((unsigned)gx, gy), fvm::kBlock, 0, s>>>( \
+#define FVM_SPMM(KT) FVM_LAUNCH(fvm::KID_ELL_SPMM, s, fvm::k_ell_spmm<KT, 8><<<dim3((unsigned)gw, gy), fvm::kBlock, 0, s>>>( \
                                     vals, cols, M, K, X, ldx, B, bias, Y, ldy))
         if (K <= 4) FVM_SPMM(4);
         else if (K <= 8) FVM_SPMM(8);
