@@ -185,5 +185,8 @@ def ptr(t) -> int | None:
 
 
 def stream_ptr(stream=None) -> int | None:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream or None
+    """The raw handle of ``stream``, or of the current stream of the current device (asked for directly:
+    building a ``torch.cuda.Stream`` object costs more than the rest of a small product's call)."""
+    if stream is not None:
+        return stream.cuda_stream or None
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()) or None

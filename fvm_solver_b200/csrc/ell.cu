@@ -302,14 +302,18 @@ extern "C" const char* fvm_version(void) { return "fvm_b200 1.0 sm_100a"; }
 
 using fvm::launch_status;
 
-// One wave of blocks over M rows, `rows` per thread (0: no device).
-static int64_t ell_grid(int64_t M, int rows, int per_sm) {
+// SMs of the current device (0: no device).
+static int64_t ell_wave() {
     static int sms[64];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
     if (!sms[dev] && cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    const int64_t all = (M + (int64_t)fvm::kBlock * rows - 1) / ((int64_t)fvm::kBlock * rows), wave = (int64_t)sms[dev] * per_sm;
-    return all < wave ? all : wave;
+    return sms[dev];
+}
+// One wave of `per_sm` blocks on each of `sms` SMs over M rows, `rows` per thread.
+static unsigned ell_grid(int64_t M, int rows, int64_t sms, int per_sm) {
+    const int64_t all = (M + (int64_t)fvm::kBlock * rows - 1) / ((int64_t)fvm::kBlock * rows);
+    return (unsigned)(all < sms * per_sm ? all : sms * per_sm);
 }
 
 extern "C" int fvm_ell_spmv(const float* vals, const int32_t* cols, int64_t M, int32_t K,
@@ -319,16 +323,17 @@ extern "C" int fvm_ell_spmv(const float* vals, const int32_t* cols, int64_t M, i
     if (M == 0) return FVM_OK;
     if (K > FVM_MAX_ELL_K) return FVM_E_UNSUPPORTED;
     cudaStream_t s = (cudaStream_t)stream;
-    if (ell_grid(M, 1, 1) < 1) {
+    const int64_t wave = ell_wave();
+    if (wave < 1) {
         launch_status();
         return FVM_E_CUDA;
     }
     // several rows per thread only where every SM still gets its blocks
-#define FVM_SPMV_R(KT, RT) FVM_LAUNCH(fvm::KID_ELL_SPMV, s, fvm::k_ell_spmv<KT, RT><<<(unsigned)ell_grid(M, RT, fvm::kEllBlocks), \
+#define FVM_SPMV_R(KT, RT) FVM_LAUNCH(fvm::KID_ELL_SPMV, s, fvm::k_ell_spmv<KT, RT><<<ell_grid(M, RT, wave, fvm::kEllBlocks), \
                                       fvm::kBlock, 0, s>>>(vals, cols, M, K, x, incx, bias, y, incy))
 #define FVM_SPMV(KT, RT)                                                                                \
     do {                                                                                                \
-        if (RT > 1 && M >= 148LL * fvm::kEllBlocks * fvm::kBlock * RT) FVM_SPMV_R(KT, RT);              \
+        if (RT > 1 && M >= wave * fvm::kEllBlocks * fvm::kBlock * RT) FVM_SPMV_R(KT, RT);              \
         else FVM_SPMV_R(KT, 1);                                                                         \
     } while (0)
     if (K <= 2) FVM_SPMV(2, 4);
@@ -350,8 +355,8 @@ extern "C" int fvm_ell_spmm(const float* vals, const int32_t* cols, int64_t M, i
     const int64_t gx = (M + fvm::kBlock - 1) / fvm::kBlock;
     cudaStream_t s = (cudaStream_t)stream;
     if (K > FVM_MAX_ELL_K) return FVM_E_UNSUPPORTED;
-    const int64_t gw = ell_grid(M, 1, fvm::kEllBlocks);
-    if (gw < 1) {
+    const int64_t wave = ell_wave();
+    if (wave < 1) {
         launch_status();
         return FVM_E_CUDA;
     }
@@ -364,14 +369,14 @@ extern "C" int fvm_ell_spmm(const float* vals, const int32_t* cols, int64_t M, i
         else FVM_SPMM4(16);
 #undef FVM_SPMM4
     } else if (B == 5 && K <= 5) {
-#define FVM_SPMM5(KT) FVM_LAUNCH(fvm::KID_ELL_SPMM, s, fvm::k_ell_spmm5<KT><<<(unsigned)ell_grid(M, 1, fvm::spmm5_blocks(KT)), \
+#define FVM_SPMM5(KT) FVM_LAUNCH(fvm::KID_ELL_SPMM, s, fvm::k_ell_spmm5<KT><<<ell_grid(M, 1, wave, fvm::spmm5_blocks(KT)), \
                                      fvm::kBlock, 0, s>>>(vals, cols, M, K, X, ldx, bias, Y, ldy))
         if (K <= 4) FVM_SPMM5(4);
         else FVM_SPMM5(5);
 #undef FVM_SPMM5
     } else {
         const unsigned gy = (unsigned)((B + 7) / 8);
-#define FVM_SPMM(KT) FVM_LAUNCH(fvm::KID_ELL_SPMM, s, fvm::k_ell_spmm<KT, 8><<<dim3((unsigned)gw, gy), fvm::kBlock, 0, s>>>( \
+#define FVM_SPMM(KT) FVM_LAUNCH(fvm::KID_ELL_SPMM, s, fvm::k_ell_spmm<KT, 8><<<dim3(ell_grid(M, 1, wave, fvm::kEllBlocks), gy), fvm::kBlock, 0, s>>>( \
                                     vals, cols, M, K, X, ldx, B, bias, Y, ldy))
         if (K <= 4) FVM_SPMM(4);
         else if (K <= 8) FVM_SPMM(8);

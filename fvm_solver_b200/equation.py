@@ -266,7 +266,9 @@ class FVMEquation:
 
     def forward(self, primatives: torch.Tensor) -> torch.Tensor:
         """dU/dt [N, C] of the primitives [N, C] (V, rho, T)."""
-        prims = primatives.to(device=self.device, dtype=torch.float32).contiguous()
+        prims = primatives
+        if not (prims.is_cuda and prims.dtype == torch.float32 and prims.device == self.grads.device and prims.is_contiguous()):
+            prims = primatives.to(device=self.device, dtype=torch.float32).contiguous()
         assert prims.shape == (self.mesh.n_cells, self.n_comp), f"bad primatives shape {tuple(prims.shape)}"
         out = torch.empty_like(prims)
         _lib.check(self.lib.fvm_residual(ct.byref(self.dev.struct), ct.byref(self.phys), _lib.ptr(prims),

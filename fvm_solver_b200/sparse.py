@@ -74,10 +74,11 @@ class SPMB200(SPM):
             return self.spMM(x, b)
         if b is not None:
             b = b.contiguous()
-        y = torch.empty(self.M, device=x.device, dtype=x.dtype)
-        _lib.check(self.lib.fvm_ell_spmv(_lib.ptr(self.vals), _lib.ptr(self.cols), self.M, self.K,
-                                         x.data_ptr(), x.stride(0), _lib.ptr(b), _lib.ptr(y), 1,
-                                         _lib.stream_ptr()), "fvm_ell_spmv")
+        y = x.new_empty(self.M)
+        rc = self.lib.fvm_ell_spmv(_lib.ptr(self.vals), _lib.ptr(self.cols), self.M, self.K, x.data_ptr(), x.stride(0), _lib.ptr(b), _lib.ptr(y), 1,
+                                   _lib.stream_ptr())
+        if rc:
+            _lib.check(rc, "fvm_ell_spmv")
         return y
 
     def spMM(self, X: torch.Tensor, b: torch.Tensor = None) -> torch.Tensor:
@@ -88,17 +89,19 @@ class SPMB200(SPM):
         if b is not None:
             b = b.contiguous()
         if B == 1:
-            y = torch.empty((self.M, 1), device=X.device, dtype=X.dtype)
-            _lib.check(self.lib.fvm_ell_spmv(_lib.ptr(self.vals), _lib.ptr(self.cols), self.M, self.K,
-                                             X.data_ptr(), X.stride(0), _lib.ptr(b), _lib.ptr(y), 1,
-                                             _lib.stream_ptr()), "fvm_ell_spmv")
+            y = X.new_empty((self.M, 1))
+            rc = self.lib.fvm_ell_spmv(_lib.ptr(self.vals), _lib.ptr(self.cols), self.M, self.K, X.data_ptr(), X.stride(0), _lib.ptr(b), _lib.ptr(y), 1,
+                                       _lib.stream_ptr())
+            if rc:
+                _lib.check(rc, "fvm_ell_spmv")
             return y
         if X.stride(1) != 1:
             X = X.contiguous()
-        Y = torch.empty((self.M, B), device=X.device, dtype=X.dtype)
-        _lib.check(self.lib.fvm_ell_spmm(_lib.ptr(self.vals), _lib.ptr(self.cols), self.M, self.K,
-                                         X.data_ptr(), X.stride(0), B, _lib.ptr(b), _lib.ptr(Y), B,
-                                         _lib.stream_ptr()), "fvm_ell_spmm")
+        Y = X.new_empty((self.M, B))
+        rc = self.lib.fvm_ell_spmm(_lib.ptr(self.vals), _lib.ptr(self.cols), self.M, self.K, X.data_ptr(), X.stride(0), B, _lib.ptr(b), _lib.ptr(Y), B,
+                                   _lib.stream_ptr())
+        if rc:
+            _lib.check(rc, "fvm_ell_spmm")
         return Y
 
 
