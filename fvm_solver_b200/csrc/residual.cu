@@ -588,11 +588,14 @@ __device__ __forceinline__ void cell_eval(const Phys& p, const float (&X)[L<DIM>
 // gradient-stencil columns one iteration ahead, so the neighbour gathers of a cell are issued at
 // the top of its iteration together with its record, one memory round trip instead of two.  TILED: the
 // record comes from the tiled table, else from the row table.  INNER: cells with a boundary column
-// are left to the launch's boundary blocks (boundary_cells).  Block `bid` of `nblk`.
+// are left to the launch's boundary blocks (boundary_cells).  Block `bid` of `nblk`.  `copy` (2D, or
+// null) receives the cells' primitives: where `prims` are the caller's, the padded copy in the
+// workspace is filled on the way instead of by a kernel before.
 template <int DIM, bool COH, bool TILED, bool INNER>
 __device__ __forceinline__ void cell_body(const fvm_mesh_t& m, const Phys& p, const float* __restrict__ prims,
                                           const float* __restrict__ bcv, float* __restrict__ grads,
-                                          int32_t* __restrict__ has_grads, int waves, int bid, int nblk) {
+                                          int32_t* __restrict__ has_grads, int waves, int bid, int nblk,
+                                          float* __restrict__ copy) {
     using Ly = L<DIM>;
     constexpr int C = Ly::C, KG = Ly::KG, RS = Ly::RS;
     const int N = m.n_cells;                              // columns < N are cells (halo included)
@@ -635,6 +638,8 @@ __device__ __forceinline__ void cell_body(const fvm_mesh_t& m, const Phys& p, co
         float rec[Ly::CR];
         cell_record<DIM, TILED>(m, i, rec);
         next_cols<DIM, TILED>(m, i + stride, NA, cols, own, skip_frozen);
+        if constexpr (RS == C)
+            if (copy) st_vec<RS>(copy + (int64_t)i * RS, U);
         cell_eval<DIM>(p, X, U, rec, grads + (int64_t)i * Ly::GS);
     }
 }
@@ -647,7 +652,7 @@ __device__ __forceinline__ void cell_body(const fvm_mesh_t& m, const Phys& p, co
 template <int DIM, bool TILED>
 __device__ __forceinline__ void boundary_cells(const fvm_mesh_t& m, const Phys& p, const float* __restrict__ prims,
                                                float* __restrict__ bcv, float* __restrict__ grads,
-                                               const int32_t* __restrict__ has_grads) {
+                                               const int32_t* __restrict__ has_grads, float* __restrict__ copy) {
     using Ly = L<DIM>;
     constexpr int C = Ly::C, KG = Ly::KG, RS = Ly::RS;
     __shared__ double red[32];
@@ -693,6 +698,8 @@ __device__ __forceinline__ void boundary_cells(const fvm_mesh_t& m, const Phys& 
     float V[C], rec[Ly::CR];
 #pragma unroll
     for (int c = 0; c < C; ++c) V[c] = U[c];
+    if constexpr (RS == C)
+        if (copy) st_vec<RS>(copy + (int64_t)cell * RS, U);
     cell_record<DIM, TILED>(m, cell, rec);
     cell_eval<DIM>(p, X, V, rec, grads + (int64_t)cell * Ly::GS);
 }
@@ -705,7 +712,7 @@ __device__ __forceinline__ void boundary_cells(const fvm_mesh_t& m, const Phys& 
 template <int DIM, bool COH>
 __device__ __forceinline__ void cell_wide_body(const fvm_mesh_t& m, const Phys& p, const float* __restrict__ prims,
                                                const float* __restrict__ bcv, float* __restrict__ grads,
-                                               int32_t* __restrict__ has_grads) {
+                                               int32_t* __restrict__ has_grads, float* __restrict__ copy) {
     using Ly = L<DIM>;
     constexpr int C = Ly::C, K = Ly::K, RS = Ly::RS;
     const int kg = m.kg;
@@ -726,6 +733,7 @@ __device__ __forceinline__ void cell_wide_body(const fvm_mesh_t& m, const Phys& 
         for (int j = 0; j < K; ++j) face |= 1u << ((meta >> (4 * j)) & 15);
         float U[RS];
         ld_mut<COH, RS>(prims + (int64_t)i * RS, U);
+        if (copy) st_vec<RS>(copy + (int64_t)i * RS, U);
         float g[DIM][C];
 #pragma unroll
         for (int d = 0; d < DIM; ++d)
@@ -799,9 +807,9 @@ __device__ __forceinline__ void cell_wide_body(const fvm_mesh_t& m, const Phys& 
 template <int DIM>
 __global__ void __launch_bounds__(kBlock) k_cell_wide(fvm_mesh_t m, Phys p, const float* __restrict__ prims,
                                                        const float* __restrict__ bcv, float* __restrict__ grads,
-                                                       int32_t* __restrict__ has_grads) {
+                                                       int32_t* __restrict__ has_grads, float* __restrict__ copy) {
     dependency_wait();
-    cell_wide_body<DIM, false>(m, p, prims, bcv, grads, has_grads);
+    cell_wide_body<DIM, false>(m, p, prims, bcv, grads, has_grads, copy);
 }
 
 #ifndef FVM_CELL_MAXNREG
@@ -813,9 +821,10 @@ __global__ void __launch_bounds__(kBlock) k_cell_wide(fvm_mesh_t m, Phys p, cons
 template <int DIM, bool TILED>
 __global__ void __maxnreg__(FVM_CELL_MAXNREG) k_cell(fvm_mesh_t m, Phys p, const float* __restrict__ prims,
                                                   const float* __restrict__ bcv, float* __restrict__ grads,
-                                                  int32_t* __restrict__ has_grads, int waves) {
+                                                  int32_t* __restrict__ has_grads, int waves,
+                                                  float* __restrict__ copy) {
     dependency_wait();
-    cell_body<DIM, false, TILED, false>(m, p, prims, bcv, grads, has_grads, waves, blockIdx.x, gridDim.x);
+    cell_body<DIM, false, TILED, false>(m, p, prims, bcv, grads, has_grads, waves, blockIdx.x, gridDim.x, copy);
 }
 
 // Boundary values and limited gradients in one launch: the first `nb` blocks take the boundary cells
@@ -825,10 +834,11 @@ __global__ void __maxnreg__(FVM_CELL_MAXNREG) k_cell(fvm_mesh_t m, Phys p, const
 template <int DIM, bool TILED>
 __global__ void __maxnreg__(FVM_CELL_MAXNREG) k_cell_bc(fvm_mesh_t m, Phys p, const float* __restrict__ prims,
                                                      float* __restrict__ bcv, float* __restrict__ grads,
-                                                     const int32_t* __restrict__ has_grads, int waves, int nb) {
+                                                     const int32_t* __restrict__ has_grads, int waves, int nb,
+                                                     float* __restrict__ copy) {
     dependency_wait();
-    if ((int)blockIdx.x < nb) boundary_cells<DIM, TILED>(m, p, prims, bcv, grads, has_grads);
-    else cell_body<DIM, false, TILED, true>(m, p, prims, bcv, grads, nullptr, waves, blockIdx.x - nb, gridDim.x - nb);
+    if ((int)blockIdx.x < nb) boundary_cells<DIM, TILED>(m, p, prims, bcv, grads, has_grads, copy);
+    else cell_body<DIM, false, TILED, true>(m, p, prims, bcv, grads, nullptr, waves, blockIdx.x - nb, gridDim.x - nb, copy);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1778,8 +1788,8 @@ __global__ void __launch_bounds__(kBlock) k_step_fused(fvm_mesh_t m, Phys p, Fus
                 bc_item<DIM, true>(m, p, f.prims, f.grads, f.has_grads, f.bcv, f.red, b, scale);
             grid_barrier(f.bar, f.status);
         }
-        if (m.kg == DIM + 2) cell_body<DIM, true, false, false>(m, p, f.prims, f.bcv, f.grads, f.has_grads, 0, blockIdx.x, gridDim.x);
-        else cell_wide_body<DIM, true>(m, p, f.prims, f.bcv, f.grads, f.has_grads);
+        if (m.kg == DIM + 2) cell_body<DIM, true, false, false>(m, p, f.prims, f.bcv, f.grads, f.has_grads, 0, blockIdx.x, gridDim.x, nullptr);
+        else cell_wide_body<DIM, true>(m, p, f.prims, f.bcv, f.grads, f.has_grads, nullptr);
         grid_barrier(f.bar, f.status);
         face_body<DIM, true>(m, p, f.prims, f.bcv, f.grads, f.flux, 0);
         grid_barrier(f.bar, f.status);
@@ -2063,14 +2073,15 @@ static inline bool fuse_bc(const fvm_mesh_t* m) {
 
 template <int DIM>
 static int launch_begin(const fvm_mesh_t* m, const Phys& p, const float* prims, float* grads,
-                        int32_t* has_grads, const fvm_work_t* w, bool with_faces, cudaStream_t s) {
+                        int32_t* has_grads, const fvm_work_t* w, bool with_faces, cudaStream_t s,
+                        float* copy = nullptr) {
     if (with_faces && fuse_bc(m)) {
         auto cells = [&](auto kernel) {
             const unsigned nb = blocks_of(m->n_bc, g_block_cell);
             const int wave = wave_blocks(kernel, g_block_cell);
             const unsigned gc = persistent_grid(m->n_cells, g_block_cell, std::max(wave - (int)nb, wave / 2));
             FVM_LAUNCH(KID_CELL, s, launch(kernel, dim3(nb + gc), dim3(g_block_cell), 0, s, *m, p, prims, w->bc_vals, grads,
-                                           has_grads, waves_of(g_pf_cell), (int)nb));
+                                           has_grads, waves_of(g_pf_cell), (int)nb, copy));
         };
         if (cell_tiled(m)) cells(k_cell_bc<DIM, true>);
         else cells(k_cell_bc<DIM, false>);
@@ -2085,13 +2096,13 @@ static int launch_begin(const fvm_mesh_t* m, const Phys& p, const float* prims, 
     if (owned_cells(m) - m->cell_lo <= 0) return launch_status();   // empty range: nothing to launch
     if (m->kg != DIM + 2) {
         const unsigned gw = persistent_grid(owned_cells(m) - m->cell_lo, kBlock, wave_blocks(k_cell_wide<DIM>, kBlock));
-        FVM_LAUNCH(KID_CELL, s, launch(k_cell_wide<DIM>, dim3(gw), dim3(kBlock), 0, s, *m, p, prims, w->bc_vals, grads, has_grads));
+        FVM_LAUNCH(KID_CELL, s, launch(k_cell_wide<DIM>, dim3(gw), dim3(kBlock), 0, s, *m, p, prims, w->bc_vals, grads, has_grads, copy));
         return launch_status();
     }
     auto cells = [&](auto kernel) {
         const unsigned gc = persistent_grid(owned_cells(m) - m->cell_lo, g_block_cell, wave_blocks(kernel, g_block_cell));
         FVM_LAUNCH(KID_CELL, s, launch(kernel, dim3(gc), dim3(g_block_cell), 0, s, *m, p, prims, w->bc_vals, grads,
-                                       has_grads, waves_of(g_pf_cell)));
+                                       has_grads, waves_of(g_pf_cell), copy));
     };
     if (cell_tiled(m)) cells(k_cell<DIM, true>);
     else cells(k_cell<DIM, false>);
@@ -2152,8 +2163,8 @@ static int launch_face(const fvm_mesh_t* m, const Phys& p, const float* prims, c
 // bc -> cell -> face for the padded primitives `prims`; leaves fluxes in work->flux.
 template <int DIM>
 static int launch_fluxes(const fvm_mesh_t* m, const Phys& p, const float* prims, float* grads,
-                         int32_t* has_grads, const fvm_work_t* w, cudaStream_t s) {
-    const int rc = launch_begin<DIM>(m, p, prims, grads, has_grads, w, true, s);
+                         int32_t* has_grads, const fvm_work_t* w, cudaStream_t s, float* copy = nullptr) {
+    const int rc = launch_begin<DIM>(m, p, prims, grads, has_grads, w, true, s, copy);
     return rc ? rc : launch_face<DIM>(m, p, prims, grads, w, has_grads, s);
 }
 
@@ -2178,21 +2189,23 @@ static int launch_div(const fvm_mesh_t* m, const Phys& p, const float* flux, con
     return launch_status();
 }
 
-// dU/dt from the padded primitives in work->prims: bc -> cell -> face -> divergence, or with the
-// owner-computes variant bc -> cell -> k_face_div (whole meshes; same bits).
+// dU/dt from the padded primitives `prims` (work->prims, or rows of the caller's that the cell kernel
+// copies there): bc -> cell -> face -> divergence, or with the owner-computes variant bc -> cell ->
+// k_face_div (whole meshes; same bits).
 template <int DIM>
-static int launch_residual(const fvm_mesh_t* m, const Phys& p, float* grads, int32_t* has_grads, float* dudt,
-                           const fvm_work_t* w, cudaStream_t s) {
+static int launch_residual(const fvm_mesh_t* m, const Phys& p, const float* prims, float* grads, int32_t* has_grads,
+                           float* dudt, const fvm_work_t* w, cudaStream_t s) {
+    float* copy = prims == w->prims ? nullptr : w->prims;
     if (g_div_variant == 1 && m->cell_lo == 0 && m->facet_lo == 0 && owned_cells(m) > 0) {
-        const int rc = launch_begin<DIM>(m, p, w->prims, grads, has_grads, w, false, s);
+        const int rc = launch_begin<DIM>(m, p, prims, grads, has_grads, w, false, s, copy);
         if (rc) return rc;
         const unsigned g = persistent_grid(4 * (int64_t)owned_cells(m), g_block_face,
                                            wave_blocks(k_face_div<DIM>, g_block_face));
-        FVM_LAUNCH(KID_DIV_STAGE, s, launch(k_face_div<DIM>, dim3(g), dim3(g_block_face), 0, s, *m, p, w->prims, w->bc_vals, grads,
+        FVM_LAUNCH(KID_DIV_STAGE, s, launch(k_face_div<DIM>, dim3(g), dim3(g_block_face), 0, s, *m, p, prims, w->bc_vals, grads,
                                                                                 dudt));
         return launch_status();
     }
-    const int rc = launch_fluxes<DIM>(m, p, w->prims, grads, has_grads, w, s);
+    const int rc = launch_fluxes<DIM>(m, p, prims, grads, has_grads, w, s, copy);
     if (rc) return rc;
     StageArgs a{};
     return launch_div<DIM>(m, p, w->flux, a, nullptr, nullptr, nullptr, nullptr, nullptr, dudt, s);
@@ -2201,9 +2214,12 @@ static int launch_residual(const fvm_mesh_t* m, const Phys& p, float* grads, int
 template <int DIM>
 static int residual_impl(const fvm_mesh_t* m, const Phys& p, const float* prims_user, float* grads,
                          int32_t* has_grads, float* dudt, const fvm_work_t* w, cudaStream_t s) {
+    // 2D rows need no padding: aligned primitives are read where they are (a launch and a pass less)
+    if (DIM == 2 && ((uintptr_t)prims_user & 15u) == 0 && owned_cells(m) == m->n_cells && m->cell_lo == 0 && !m->case_active)
+        return launch_residual<DIM>(m, p, prims_user, grads, has_grads, dudt, w, s);
     FVM_LAUNCH(KID_STATE_TO_PRIMS, s, launch(k_pad_prims<DIM>, dim3(blocks_for(m->n_cells)), dim3(kBlock), 0, s, 
                                           m->n_cells, prims_user, w->prims));
-    return launch_residual<DIM>(m, p, grads, has_grads, dudt, w, s);
+    return launch_residual<DIM>(m, p, w->prims, grads, has_grads, dudt, w, s);
 }
 
 // dU/dt of a conserved state: one kernel writes the padded primitives into work->prims (the
@@ -2213,7 +2229,7 @@ static int residual_state_impl(const fvm_mesh_t* m, const Phys& p, const float* 
                                int32_t* has_grads, float* dudt, const fvm_work_t* w, cudaStream_t s) {
     FVM_LAUNCH(KID_STATE_TO_PRIMS, s, launch(k_state_to_prims<DIM>, dim3(blocks_for(m->n_cells)), dim3(kBlock), 0, s, 
                                           m->n_cells, p.inv_Cv, state, w->prims));
-    return launch_residual<DIM>(m, p, grads, has_grads, dudt, w, s);
+    return launch_residual<DIM>(m, p, w->prims, grads, has_grads, dudt, w, s);
 }
 
 static StageArgs stage_args(const fvm_tableau_t* tab, int s) {

@@ -75,8 +75,8 @@ class SPMB200(SPM):
         if b is not None:
             b = b.contiguous()
         y = x.new_empty(self.M)
-        rc = self.lib.fvm_ell_spmv(_lib.ptr(self.vals), _lib.ptr(self.cols), self.M, self.K, x.data_ptr(), x.stride(0), _lib.ptr(b), _lib.ptr(y), 1,
-                                   _lib.stream_ptr())
+        rc = self.lib.fvm_ell_spmv(_lib.ptr(self.vals), _lib.ptr(self.cols), self.M, self.K, x.data_ptr(),
+                                   x.stride(0), _lib.ptr(b), _lib.ptr(y), 1, _lib.stream_ptr())
         if rc:
             _lib.check(rc, "fvm_ell_spmv")
         return y
@@ -90,16 +90,16 @@ class SPMB200(SPM):
             b = b.contiguous()
         if B == 1:
             y = X.new_empty((self.M, 1))
-            rc = self.lib.fvm_ell_spmv(_lib.ptr(self.vals), _lib.ptr(self.cols), self.M, self.K, X.data_ptr(), X.stride(0), _lib.ptr(b), _lib.ptr(y), 1,
-                                       _lib.stream_ptr())
+            rc = self.lib.fvm_ell_spmv(_lib.ptr(self.vals), _lib.ptr(self.cols), self.M, self.K, X.data_ptr(),
+                                       X.stride(0), _lib.ptr(b), _lib.ptr(y), 1, _lib.stream_ptr())
             if rc:
                 _lib.check(rc, "fvm_ell_spmv")
             return y
         if X.stride(1) != 1:
             X = X.contiguous()
         Y = X.new_empty((self.M, B))
-        rc = self.lib.fvm_ell_spmm(_lib.ptr(self.vals), _lib.ptr(self.cols), self.M, self.K, X.data_ptr(), X.stride(0), B, _lib.ptr(b), _lib.ptr(Y), B,
-                                   _lib.stream_ptr())
+        rc = self.lib.fvm_ell_spmm(_lib.ptr(self.vals), _lib.ptr(self.cols), self.M, self.K, X.data_ptr(),
+                                   X.stride(0), B, _lib.ptr(b), _lib.ptr(Y), B, _lib.stream_ptr())
         if rc:
             _lib.check(rc, "fvm_ell_spmm")
         return Y
