@@ -197,12 +197,19 @@ class CorrectorNet:
         the pre-activations and the operands for the backward pass; inference does not.  Both forms
         give bitwise the same output."""
         b = self._bufs
+        _lib.check(self.lib.fvm_in_layer(b["X"].data_ptr(), b["N"], self.bf["W_in"].data_ptr(),
+                                         self.params["b_in"].data_ptr(), b["hf"][0].data_ptr(),
+                                         b["Z"][0].data_ptr() if store_pre else None, self.err.data_ptr(),
+                                         _lib.stream_ptr()), "fvm_in_layer")
+        return self._layers(nbr, store_pre)
+
+    def _layers(self, nbr: torch.Tensor, store_pre: bool) -> torch.Tensor:
+        """The message-passing layers and the decoder from the input layer's activations."""
+        b = self._bufs
         N, L = b["N"], self.L
         p, s = self.params, _lib.stream_ptr()
         err = self.err.data_ptr()
         Z = [z.data_ptr() for z in b["Z"]] if store_pre else [None] * (L + 1)
-        _lib.check(self.lib.fvm_in_layer(b["X"].data_ptr(), N, self.bf["W_in"].data_ptr(), p["b_in"].data_ptr(),
-                                         b["hf"][0].data_ptr(), Z[0], err, s), "fvm_in_layer")
         for l in range(L):
             last = l == L - 1
             keep = store_pre or not last
@@ -344,7 +351,6 @@ class CorrectorModel:
         self.cell_case32 = batch.dev.case["cell_case"]
         self.kdt_case = torch.empty(batch.n_cases, device=dev)
         self.S = torch.empty((batch.n_cases, C), dtype=torch.float64, device=dev)
-        self.shift = torch.zeros((batch.n_cases, C), device=dev)
         self.base = torch.empty((N, C), device=dev)
         self.fmean = torch.zeros(2 * C, device=dev)
         self.finv = torch.ones(2 * C, device=dev)
@@ -390,25 +396,26 @@ class CorrectorModel:
             self.base.data_ptr(), b["X"].data_ptr(), XW, _lib.stream_ptr()), "fvm_corrector_inputs")
         return b["X"]
 
-    def _shift(self, out: torch.Tensor) -> torch.Tensor:
-        """Per-case offsets that remove the volume-weighted mean of the mass and energy parts of
-        scale * out (the other components get no offset)."""
-        b = self.batch
-        _lib.check(self.net.lib.fvm_conservation(ct.byref(b.dev.struct), out.data_ptr(), self.S.data_ptr(),
-                                                 ct.byref(b.work.struct), _lib.stream_ptr()), "fvm_conservation")
-        mean = self.S[:, self.cons] / self.case_vol.unsqueeze(1) * self.scale[self.cons].double()
-        self.shift[:, self.cons] = mean.float()
-        return self.shift
-
     def predict(self, state: torch.Tensor, out_state: torch.Tensor, r0: torch.Tensor):
-        """out_state = proposal for U_{t+k} from state = U_t with residual r0 = dU/dt(U_t)."""
-        self.inputs(state, r0)
-        out = self.net.forward(self.nbr, store_pre=False)
-        shift = self._shift(out)
-        _lib.check(self.net.lib.fvm_corrector_combine(
-            state.data_ptr(), self.base.data_ptr(), out.data_ptr(), self.scale.data_ptr(), shift.data_ptr(),
-            self.cell_case32.data_ptr(), state.shape[0], self.C, out_state.data_ptr(), _lib.stream_ptr()),
-            "fvm_corrector_combine")
+        """out_state = proposal for U_{t+k} from state = U_t with residual r0 = dU/dt(U_t).
+
+        The input features are formed inside the input layer (the network's X buffer, which training
+        reads, is left alone), and the offsets that remove the volume-weighted mean of the mass and
+        energy parts of scale * out inside the kernel that adds the proposal up."""
+        net, b, N = self.net, self.batch, state.shape[0]
+        lib, s, bufs = net.lib, _lib.stream_ptr(), net._alloc(state.shape[0])
+        _lib.check(lib.fvm_corrector_in_layer(
+            state.data_ptr(), r0.data_ptr(), b.t_solver.dt.data_ptr(), self.k, self.cell_case32.data_ptr(), N, self.C,
+            self.fmean.data_ptr(), self.finv.data_ptr(), self.geo.data_ptr(), self.geo.shape[1], self.base.data_ptr(),
+            net.bf["W_in"].data_ptr(), net.params["b_in"].data_ptr(), bufs["hf"][0].data_ptr(), net.err.data_ptr(), s),
+            "fvm_corrector_in_layer")
+        out = net._layers(self.nbr, store_pre=False)
+        _lib.check(lib.fvm_conservation(ct.byref(b.dev.struct), out.data_ptr(), self.S.data_ptr(),
+                                        ct.byref(b.work.struct), s), "fvm_conservation")
+        _lib.check(lib.fvm_corrector_propose(
+            state.data_ptr(), self.base.data_ptr(), out.data_ptr(), self.scale.data_ptr(), self.S.data_ptr(),
+            self.case_vol.data_ptr(), self.cons.start, self.cell_case32.data_ptr(), N, self.C, out_state.data_ptr(), s),
+            "fvm_corrector_propose")
         return out_state
 
 

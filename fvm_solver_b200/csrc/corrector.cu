@@ -539,6 +539,33 @@ __global__ void k_corrector_combine(const float* __restrict__ state, const float
     prop[t] = v;
 }
 
+// The same with the shift formed from the cases' sums of vol * out: the components from `first` on lose
+// the volume-weighted mean of scale * out, (float)(sums / case_vol * scale).  One thread per cell.
+template <int C>
+__global__ void __launch_bounds__(256) k_corrector_propose(const float* __restrict__ state, const float* __restrict__ base,
+                                                           const float* __restrict__ out, const float* __restrict__ scale,
+                                                           const double* __restrict__ sums,
+                                                           const double* __restrict__ case_vol, int first,
+                                                           const int32_t* __restrict__ cell_case, int N,
+                                                           float* __restrict__ prop) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    const int cs = cell_case ? __ldg(cell_case + i) : 0;
+    const double vol = __ldg(case_vol + cs);
+    float u[C], b[C], o[C];
+    load_row<C>(state + (int64_t)i * C, u);
+    load_row<C>(base + (int64_t)i * C, b);
+    load_row<C>(out + (int64_t)i * C, o);
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        const float sc = __ldg(scale + c);
+        float v = u[c] + b[c] + sc * o[c];
+        v -= c >= first ? (float)(__ldg(sums + (int64_t)cs * C + c) / vol * (double)sc) : 0.f;
+        u[c] = v;
+    }
+    store_row<C>(prop + (int64_t)i * C, u);
+}
+
 static inline unsigned nblk(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
 }  // namespace corr
@@ -644,6 +671,22 @@ extern "C" int fvm_corrector_combine(const float* state, const float* base, cons
     return launch_status();
 }
 
+extern "C" int fvm_corrector_propose(const float* state, const float* base, const float* out, const float* scale,
+                                     const double* sums, const double* case_vol, int32_t first,
+                                     const int32_t* cell_case, int32_t N, int32_t C, float* prop, void* stream) {
+    if (!state || !base || !out || !scale || !sums || !case_vol || !prop || N <= 0 || first < 0) return FVM_E_ARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    const bool rows16 = (((uintptr_t)state | (uintptr_t)base | (uintptr_t)out | (uintptr_t)prop) & 15u) == 0;
+    if (C == 4 && rows16)
+        FVM_LAUNCH(KID_CORRECTOR, s, corr::k_corrector_propose<4><<<corr::nblk(N, 256), 256, 0, s>>>(
+                                         state, base, out, scale, sums, case_vol, first, cell_case, N, prop));
+    else if (C == 5)
+        FVM_LAUNCH(KID_CORRECTOR, s, corr::k_corrector_propose<5><<<corr::nblk(N, 256), 256, 0, s>>>(
+                                         state, base, out, scale, sums, case_vol, first, cell_case, N, prop));
+    else
+        return C == 4 ? FVM_E_ARG : FVM_E_UNSUPPORTED;
+    return launch_status();
+}
 
 // ------------------------------------------------------------------------------------------
 // Message-passing layer on an fp32 residual stream (fvm_mp_layer, fvm_mp_layer_train) and the
@@ -657,9 +700,9 @@ extern "C" int fvm_corrector_combine(const float* state, const float* base, cons
 // neighbours of the Morton-ordered cells are mostly in the same tile, so the gathers hit L1 (72 %)
 // and the floor is the 512 bytes of DRAM traffic.  What bounds it is latency: a tile is a chain of
 // neighbour list -> gathers -> MMA -> epilogue.  One CTA of 128 rows therefore runs that chain without
-// any role split, small enough (64 registers, 54 KB of shared memory, 64 TMEM columns) that four CTAs
-// share an SM and fill each other's waits; one CTA per SM with gather and epilogue warps side by side
-// left 12 warps per SM and took 111 us per layer at 278 k rows of 64 (now 55 us).  The
+// any role split, small enough (256 threads, 56 KB of shared memory, 64 TMEM columns) that three or four
+// CTAs share an SM and fill each other's waits; one CTA per SM with gather and epilogue warps side by side
+// left 12 warps per SM and took 111 us per layer at 278 k rows of 64 (now 50 us).  The
 // epilogue goes through shared memory (the operand's own buffer, free once the MMAs are done), so
 // the residual, the pre-activation and h' move as whole 128-byte lines instead of one line per lane.
 // The mbarrier wait is bounded; a wait that gives up sets *err and ends the CTA.
@@ -668,7 +711,9 @@ namespace fvm {
 namespace corr {
 
 constexpr int kLayerThreads = 256;
-constexpr int kLayerCtas = 4;                            // CTAs per SM
+// CTAs per SM: four of the input layer; three of the others, whose 80 registers hold a row's gathers
+// without spills (50 us per layer at 278 k rows of 64; four with 64 registers spill, 55 us).
+constexpr int layer_ctas(bool input) { return input ? 4 : 3; }
 constexpr int kLayerW = 64;                              // channels
 // One 8-channel unit of a tile's rows, 32 bytes apart from the next modulo 128: the 16-byte stores of
 // four units x two rows (eight lanes) then hit every bank once.
@@ -681,7 +726,12 @@ constexpr int kLayerSmem = kLayerWBytes + kLayerABytes;
 struct LayerArgs {
     const float* h;              // [M][64] fp32 residual stream (input)
     const int32_t* nbr;          // [M][KN]
-    const __nv_bfloat16* X;      // input layer: [M][64] features (h and nbr unused)
+    const __nv_bfloat16* X;      // input layer: [M][64] features (h and nbr unused), or null:
+    const float *state, *r0, *dt, *mean, *inv_std, *geo;   // the features of fvm_corrector_inputs, built
+    const int32_t* cell_case;                              // here (C, G columns; base [M][C] is stored)
+    float* base;
+    int C, G;
+    float k;
     int M, KN;
     const __nv_bfloat16* Wt;     // [64][128] (input layer: [64][64])
     const float* bias;           // [64]
@@ -740,8 +790,55 @@ __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
 // chunks both hit every bank once.
 __device__ __forceinline__ int epi_off(int r, int c) { return r * 256 + ((c ^ (r & 7)) << 4); }
 
+// A row of zeros: what a missing neighbour, or a row past M, reads (adding +0 leaves a sum that starts
+// at +0 unchanged), so the gather needs no selects on the data.
+__device__ __align__(256) float g_zero_row[kLayerW];
+
+// A row's features as k_corrector_inputs forms them -- normalised state and baseline k dt r0 (stored to
+// base), geometry, zeros -- into the operand tile: the row's thread of the block's first half takes the
+// first 16, that of the second half the others, so a thread's loads are all independent.
+template <int C>
+__device__ __forceinline__ void stage_features(const LayerArgs& g, uint8_t* sA, int64_t row, int r, bool second) {
+    const bool valid = row < g.M;
+    if (!second) {
+        float u[C], b[C], x[16];
+        float h = 0.f;
+        if (valid) {
+            load_row<C>(g.state + row * C, u);
+            load_row<C>(g.r0 + row * C, b);
+            h = g.k * __ldg(g.dt + (g.cell_case ? __ldg(g.cell_case + row) : 0));
+        }
+#pragma unroll
+        for (int c = 2 * C; c < 16; ++c) x[c] = valid && c < 2 * C + g.G ? __ldg(g.geo + row * g.G + c - 2 * C) : 0.f;
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            b[c] *= h;
+            x[c] = valid ? (u[c] - __ldg(g.mean + c)) * __ldg(g.inv_std + c) : 0.f;
+            x[C + c] = valid ? (b[c] - __ldg(g.mean + C + c)) * __ldg(g.inv_std + C + c) : 0.f;
+        }
+        if (valid) store_row<C>(g.base + row * C, b);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = x[8 * q + e];
+            *reinterpret_cast<uint4*>(sA + q * kUnitBytes + r * 16) = pack8(v);
+        }
+    } else {
+        for (int q = 2; q < 8; ++q) {
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const int c = 8 * q + e;
+                v[e] = valid && c < 2 * C + g.G ? __ldg(g.geo + row * g.G + c - 2 * C) : 0.f;
+            }
+            *reinterpret_cast<uint4*>(sA + q * kUnitBytes + r * 16) = pack8(v);
+        }
+    }
+}
+
 template <bool INPUT>
-__global__ void __launch_bounds__(kLayerThreads, kLayerCtas) k_mp_layer(LayerArgs g) {
+__global__ void __launch_bounds__(kLayerThreads, layer_ctas(INPUT)) k_mp_layer(LayerArgs g) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sW = smem;                                   // B operand
     uint8_t* sA = smem + kLayerWBytes;                    // A operand, then the epilogue tile
@@ -750,7 +847,7 @@ __global__ void __launch_bounds__(kLayerThreads, kLayerCtas) k_mp_layer(LayerArg
     __shared__ uint32_t s_taddr;
     __shared__ __align__(16) int s_nb[INPUT ? 4 : TM * 8];
     __shared__ float s_inv[INPUT ? 1 : TM];
-    __shared__ float s_bias[kLayerW];
+    __shared__ __align__(16) float s_bias[kLayerW];
     __shared__ __align__(16) float s_wo[INPUT ? 4 : 8 * kLayerW];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ntiles = (g.M + TM - 1) / TM;
@@ -812,36 +909,38 @@ __global__ void __launch_bounds__(kLayerThreads, kLayerCtas) k_mp_layer(LayerArg
             __syncthreads();
         }
         // A operand.  The neighbour mean is the fp32 sum over the valid neighbours in table order
-        // (starting at +0) times 1 / count.  With at most four neighbours all loads of a row's unit
-        // are issued before any is used: a missing neighbour reads the row itself and adds +0,
-        // which leaves the sum unchanged.  Rows past M are zeros.
+        // (starting at +0) times 1 / count; with at most four neighbours all loads of a row's unit
+        // are issued before any is used.
+        if (INPUT && !g.X) {
+            const int r = tid & (TM - 1);
+            if (g.C == 4) stage_features<4>(g, sA, (int64_t)m0 + r, r, tid >= TM);
+            else stage_features<5>(g, sA, (int64_t)m0 + r, r, tid >= TM);
+        } else
 #pragma unroll 1
         for (int q = 0; q < 4; ++q) {
             const int r = r0 + 32 * q;
             const int64_t row = (int64_t)m0 + r;
             const bool valid = row < g.M;
-            const int64_t self = valid ? row : 0;
             if constexpr (INPUT) {
                 uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                if (valid) v = *reinterpret_cast<const uint4*>(g.X + self * kLayerW + 8 * u);
+                if (valid) v = *reinterpret_cast<const uint4*>(g.X + row * kLayerW + 8 * u);
                 *reinterpret_cast<uint4*>(sA + u * kUnitBytes + r * 16) = v;
             } else {
+                auto src = [&](int64_t j, bool on) { return (on ? g.h + j * kLayerW : (const float*)g_zero_row) + 8 * u; };
                 float own[8], acc[8];
-                ld8(g.h + self * kLayerW + 8 * u, own);
+                ld8(src(row, valid), own);
                 if (g.KN <= 4) {
                     float nb[4][8];
                     const int4 jj = *reinterpret_cast<const int4*>(s_nb + r * 8);
-                    const int j[4] = {jj.x, jj.y, jj.z, jj.w};
+                    ld8(src(jj.x, jj.x >= 0), nb[0]);
+                    ld8(src(jj.y, jj.y >= 0), nb[1]);
+                    ld8(src(jj.z, jj.z >= 0), nb[2]);
+                    if (g.KN == 4) ld8(src(jj.w, jj.w >= 0), nb[3]);
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (e < 3 || g.KN == 4) ld8(g.h + (j[e] >= 0 ? (int64_t)j[e] : self) * kLayerW + 8 * u, nb[e]);
+                    for (int c = 0; c < 8; ++c) acc[c] = ((0.f + nb[0][c]) + nb[1][c]) + nb[2][c];
+                    if (g.KN == 4)
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) acc[c] = 0.f;
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (e < 3 || g.KN == 4)
-#pragma unroll
-                            for (int c = 0; c < 8; ++c) acc[c] += j[e] >= 0 ? nb[e][c] : 0.f;
+                        for (int c = 0; c < 8; ++c) acc[c] += nb[3][c];
                 } else {
 #pragma unroll
                     for (int c = 0; c < 8; ++c) acc[c] = 0.f;
@@ -856,10 +955,7 @@ __global__ void __launch_bounds__(kLayerThreads, kLayerCtas) k_mp_layer(LayerArg
                 }
                 const float inv = s_inv[r];
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    own[c] = valid ? own[c] : 0.f;
-                    acc[c] = valid ? acc[c] * inv : 0.f;
-                }
+                for (int c = 0; c < 8; ++c) acc[c] *= inv;
                 const uint4 a = pack8(own), b = pack8(acc);
                 *reinterpret_cast<uint4*>(sA + u * kUnitBytes + r * 16) = a;
                 *reinterpret_cast<uint4*>(sA + (8 + u) * kUnitBytes + r * 16) = b;
@@ -891,11 +987,12 @@ __global__ void __launch_bounds__(kLayerThreads, kLayerCtas) k_mp_layer(LayerArg
             tmem_ld32(taddr + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(32 * half), z);
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
+                const float4 bs = *reinterpret_cast<const float4*>(s_bias + 32 * half + 4 * c);
                 float4 v;
-                v.x = __uint_as_float(z[4 * c]) + s_bias[32 * half + 4 * c];
-                v.y = __uint_as_float(z[4 * c + 1]) + s_bias[32 * half + 4 * c + 1];
-                v.z = __uint_as_float(z[4 * c + 2]) + s_bias[32 * half + 4 * c + 2];
-                v.w = __uint_as_float(z[4 * c + 3]) + s_bias[32 * half + 4 * c + 3];
+                v.x = __uint_as_float(z[4 * c]) + bs.x;
+                v.y = __uint_as_float(z[4 * c + 1]) + bs.y;
+                v.z = __uint_as_float(z[4 * c + 2]) + bs.z;
+                v.w = __uint_as_float(z[4 * c + 3]) + bs.w;
                 *reinterpret_cast<float4*>(sA + epi_off(r, 8 * half + c)) = v;
             }
         }
@@ -969,7 +1066,7 @@ __global__ void __launch_bounds__(kLayerThreads, kLayerCtas) k_mp_layer(LayerArg
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(64u));
 }
 
-// Grid: one wave of resident CTAs (kLayerCtas per SM), or one per tile.
+// Grid: one wave of resident CTAs, or one per tile.
 template <bool INPUT>
 static int launch_layer(const LayerArgs& g, cudaStream_t s) {
     static int sms[64];
@@ -989,7 +1086,7 @@ static int launch_layer(const LayerArgs& g, cudaStream_t s) {
         sms[dev] = n;
     }
     const int ntiles = (g.M + TM - 1) / TM;
-    FVM_LAUNCH(KID_CORRECTOR, s, launch(k_mp_layer<INPUT>, dim3((unsigned)std::min(ntiles, kLayerCtas * sms[dev])),
+    FVM_LAUNCH(KID_CORRECTOR, s, launch(k_mp_layer<INPUT>, dim3((unsigned)std::min(ntiles, layer_ctas(INPUT) * sms[dev])),
                                         dim3(kLayerThreads), kLayerSmem, s, g));
     return launch_status();
 }
@@ -1118,6 +1215,35 @@ extern "C" int fvm_in_layer(const void* X, int32_t M, const void* Wt, const floa
     g.bias = bias;
     g.h_out = h_out;
     g.Z = Z;
+    g.err = err;
+    return corr::launch_layer<true>(g, (cudaStream_t)stream);
+}
+
+extern "C" int fvm_corrector_in_layer(const float* state, const float* r0, const float* dt, int32_t k,
+                                      const int32_t* cell_case, int32_t N, int32_t C, const float* mean,
+                                      const float* inv_std, const float* geo, int32_t G, float* base, const void* Wt,
+                                      const float* bias, float* h_out, int32_t* err, void* stream) {
+    if (!state || !r0 || !dt || !mean || !inv_std || (G > 0 && !geo) || !base || !Wt || !bias || !h_out || !err ||
+        N <= 0 || G < 0 || k < 1 || (C != 4 && C != 5) || 2 * C + G > corr::kLayerW)
+        return FVM_E_ARG;
+    if (((uintptr_t)h_out & 31u) || (uintptr_t)Wt % 16) return FVM_E_ARG;
+    if (C == 4 && (((uintptr_t)state | (uintptr_t)r0 | (uintptr_t)base) & 15u)) return FVM_E_ARG;   // 128-bit rows
+    corr::LayerArgs g{};
+    g.M = N;
+    g.state = state;
+    g.r0 = r0;
+    g.dt = dt;
+    g.mean = mean;
+    g.inv_std = inv_std;
+    g.geo = geo;
+    g.cell_case = cell_case;
+    g.base = base;
+    g.C = C;
+    g.G = G;
+    g.k = (float)k;
+    g.Wt = static_cast<const __nv_bfloat16*>(Wt);
+    g.bias = bias;
+    g.h_out = h_out;
     g.err = err;
     return corr::launch_layer<true>(g, (cudaStream_t)stream);
 }

@@ -390,6 +390,18 @@ int fvm_mp_layer_train(const float *h, const int32_t *nbr, int32_t M, int32_t KN
  * Z (or NULL) receives the pre-activations.  Bitwise equal to fvm_gemm_bf16 with bias and SiLU. */
 int fvm_in_layer(const void *X, int32_t M, const void *Wt, const float *bias, float *h_out, float *Z, int32_t *err,
                  void *stream);
+/* The input layer straight from the corrector's inputs: h_out_i = SiLU(X_i . Wt^T + bias) with the feature
+ * rows X of fvm_corrector_inputs for kdt = k * dt[case], formed in the kernel; also stores base = k dt r0
+ * [N][C].  C = 4 (state, r0 and base 16-byte aligned) or 5, 2C + G <= 64.  Bitwise equal to fvm_corrector_inputs + fvm_in_layer. */
+int fvm_corrector_in_layer(const float *state, const float *r0, const float *dt, int32_t k, const int32_t *cell_case,
+                           int32_t N, int32_t C, const float *mean, const float *inv_std, const float *geo, int32_t G,
+                           float *base, const void *Wt, const float *bias, float *h_out, int32_t *err, void *stream);
+/* prop = state + base + scale[c] * out - shift, where the components c >= first lose their case's
+ * volume-weighted mean of scale * out: shift = (float)(sums[case][c] / case_vol[case] * scale[c]) with
+ * sums = fvm_conservation(out) (FP64), and 0 below.  C = 4 (rows 16-byte aligned) or 5. */
+int fvm_corrector_propose(const float *state, const float *base, const float *out, const float *scale,
+                          const double *sums, const double *case_vol, int32_t first, const int32_t *cell_case, int32_t N,
+                          int32_t C, float *prop, void *stream);
 /* Backward pass of the network (64 channels; fp32 rows 8-byte, bf16 rows 16-byte aligned, dA 32-byte).
  * Sums over the cells use workspace sets of FVM_BACK_SET floats (8-byte aligned, no clearing needed):
  * one for each bias gradient and O + 1 consecutive ones (`dec`) for the decoder.  A set is filled by a

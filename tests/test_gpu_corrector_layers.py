@@ -124,3 +124,33 @@ def test_backward_kernels(N, KN, O):
     for got, t in [(db[0], grad(dh0, Z0)), (db[1], grad(dh, Z1)), (dbo, dout)] + \
             [(dWo[o], dout[:, o:o + 1] * h) for o in range(O)]:
         assert float(((got.cpu() - run(t)).abs() / t.abs().sum(0).cpu()).max()) < 1e-5
+
+
+@pytest.mark.parametrize("N,C,G,cases", [(1, 4, 0, 1), (129, 4, 11, 2), (1000, 5, 18, 3)])
+def test_inputs_in_the_input_layer_and_proposal(N, C, G, cases):
+    """fvm_corrector_in_layer against fvm_corrector_inputs + fvm_in_layer, fvm_corrector_propose against
+    fvm_corrector_combine with the shift formed in torch: bitwise."""
+    from fvm_solver_b200 import _lib
+    lib, s = _lib.load(), _lib.stream_ptr()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    U, r0, mean, inv = _rand(N, C, seed=1), _rand(N, C, seed=2), _rand(2 * C, seed=3), _rand(2 * C, seed=4).abs()
+    geo, W, bias = _rand(N, max(G, 1), seed=5), _rand(64, 64, seed=6, scale=0.1, bf=True), _rand(64, seed=7)
+    dt, k = _rand(cases, seed=8).abs(), 8
+    cc = torch.sort(torch.randint(0, cases, (N,), device="cuda", dtype=torch.int32)).values
+    kdt = dt * float(k)
+    P = lambda t: t.data_ptr()
+    X, base = torch.zeros(N, 64, dtype=torch.bfloat16, device="cuda"), torch.empty(N, C, device="cuda")
+    _lib.check(lib.fvm_corrector_inputs(P(U), P(r0), P(kdt), P(cc), N, C, P(mean), P(inv), P(geo), G, P(base), P(X), 64, s), "inputs")
+    want, got, base2 = torch.empty(N, 64, device="cuda"), torch.empty(N, 64, device="cuda"), torch.empty(N, C, device="cuda")
+    _lib.check(lib.fvm_in_layer(P(X), N, P(W), P(bias), P(want), None, P(err), s), "in_layer")
+    _lib.check(lib.fvm_corrector_in_layer(P(U), P(r0), P(dt), k, P(cc), N, C, P(mean), P(inv), P(geo), G, P(base2), P(W),
+                                          P(bias), P(got), P(err), s), "corrector_in_layer")
+    assert torch.equal(got, want) and torch.equal(base2, base) and int(err.item()) == 0
+    out, scale = _rand(N, C, seed=9), _rand(C, seed=10).abs()
+    sums, vol = _rand(cases, C, seed=11).double(), _rand(cases, seed=12).double().abs() + 0.1
+    shift = torch.zeros(cases, C, device="cuda")
+    shift[:, C - 2:] = (sums[:, C - 2:] / vol[:, None] * scale[C - 2:].double()).float()
+    a, b = torch.empty(N, C, device="cuda"), torch.empty(N, C, device="cuda")
+    _lib.check(lib.fvm_corrector_combine(P(U), P(base), P(out), P(scale), P(shift), P(cc), N, C, P(a), s), "combine")
+    _lib.check(lib.fvm_corrector_propose(P(U), P(base), P(out), P(scale), P(sums), P(vol), C - 2, P(cc), N, C, P(b), s), "propose")
+    assert torch.equal(a, b)
