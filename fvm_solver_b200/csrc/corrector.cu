@@ -17,6 +17,7 @@
 //     fp32 and/or bf16.
 // Split-K (for weight gradients, K = number of cells): `k_splits` > 1 makes each CTA handle one
 // K range and atomically add its fp32 tile into D (no epilogue other than the add).
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
 
@@ -776,6 +777,20 @@ __device__ __forceinline__ void tmem_ld32(uint32_t addr, uint32_t (&r)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// 16 TMEM lanes x 32 columns as 16x256b blocks: register 4 g + 2 j + e of lane t holds lane 8 j + t / 4,
+// column 8 g + 2 (t % 4) + e.  With the operand's columns stored in the order of frag_col, a lane has
+// eight neighbouring logical columns of a row and the row's 32 columns lie on four consecutive lanes.
+__device__ __forceinline__ void tmem_ld_frag(uint32_t addr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr));
+}
+__device__ __forceinline__ int frag_col(int m) {   // TMEM column of logical column m
+    return (m & ~31) | ((m >> 1) & 3) << 3 | ((m >> 3) & 3) << 1 | (m & 1);
+}
+
 // Operand layout of a tile: 16-byte unit u (8 channels) of row r at u * kUnitBytes + 16 r.  Eight
 // consecutive rows of a unit are one core matrix, so the tile reads as a K-major operand with the
 // channels as K (core matrices of a K step LBO = kUnitBytes apart, 8-row groups SBO = 128 apart).
@@ -1283,14 +1298,15 @@ extern "C" int fvm_decoder_back_f32(const float* h, const float* Wo, const float
 //     neighbour count) and dW += dZ^T A, both on tcgen05 from one staged copy of the tile;
 //   * k_back_gather: dh_l = dh_{l+1} + dA[:, :64] + sum over neighbours of dA[:, 64:], then
 //     dZ = dh_l SiLU'(Z_l) for the layer below.
-// All of them are bound by memory: 0.9 kB and 1.7 kB per cell and layer.  They replace a SiLU kernel
+// Both are bound by memory: 0.9 kB and 1.7 kB per cell and layer (57 and 100 us at 278 k cells, 4.4 and
+// 4.6 TB/s).  They replace a SiLU kernel
 // with one atomic per element (1178 us per layer at 278 k cells), two transposes, two GEMMs with
 // their operands read again and a scatter that counted every neighbour's neighbours.
 //
 // Column sums (the gradients of the biases and of the decoder) keep the value of one running fp32 sum
 // over the cells in order: with terms of one sign that sum's rounding is systematic (1.6e-4 of the
 // decoder's gradient at 278 k cells), so summing pieces from zero would move the results.  Rounding
-// a + t to fp32 depends on a only through its binade, so each warp walks a contiguous range of rows
+// a + t to fp32 depends on a only through its binade, so each half-warp walks a contiguous range of rows
 // with an accumulator that starts at the sum of everything before it, taken from a first pass over the
 // same terms, and what it added is exact: the first pass runs in the kernel that produces the terms,
 // the second in the next kernel that reads them, the ranges' increments are added up once at the
@@ -1299,8 +1315,11 @@ extern "C" int fvm_decoder_back_f32(const float* h, const float* Wo, const float
 namespace fvm {
 namespace corr {
 
-constexpr int kSumBlocks = 2 * 148, kSumWarps = 16, kSumThreads = 32 * kSumWarps;
-constexpr int kSumSegs = kSumBlocks * kSumWarps;         // row ranges, one per warp
+// Row ranges belong to half-warps: 16 lanes with four channels each read a row as one 256-byte piece, and
+// a warp has two rows in flight per load (two channels per lane and a row per warp took 118 us per
+// gather at 278 k cells).
+constexpr int kSumBlocks = 2 * 148, kSumThreads = 384, kSumParts = kSumThreads / 16;
+constexpr int kSumSegs = kSumBlocks * kSumParts;         // row ranges, one per half-warp
 // One set of 64 column sums: the ranges' sums, the blocks' sums, the blocks' increments.
 constexpr int kSumSet = (kSumSegs + 2 * kSumBlocks) * kLayerW;
 static_assert(kSumSet == FVM_BACK_SET, "workspace size");
@@ -1310,64 +1329,66 @@ __host__ __device__ __forceinline__ constexpr int set_delta(int b) { return (kSu
 struct Rows {
     int64_t lo, hi;
 };
-__device__ __forceinline__ Rows warp_rows(int N) {
+__device__ __forceinline__ Rows part_rows(int N) {
     const int64_t per = ((int64_t)N + kSumSegs - 1) / kSumSegs;
-    const int64_t lo = ((int64_t)blockIdx.x * kSumWarps + (threadIdx.x >> 5)) * per;
+    const int64_t lo = ((int64_t)blockIdx.x * kSumParts + (threadIdx.x >> 4)) * per;
     return Rows{min(lo, (int64_t)N), min(lo + per, (int64_t)N)};
 }
-__device__ __forceinline__ float2 ldf2(const float* p, int64_t i) { return __ldg(reinterpret_cast<const float2*>(p) + i); }
+__device__ __forceinline__ float4 ldf4(const float* p, int64_t i) { return __ldg(reinterpret_cast<const float4*>(p) + i); }
+__device__ __forceinline__ float4 f4(float v) { return make_float4(v, v, v, v); }
+__device__ __forceinline__ float4 add4(float4 a, float4 b) {
+    return make_float4(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y), __fadd_rn(a.z, b.z), __fadd_rn(a.w, b.w));
+}
+__device__ __forceinline__ float4 mul4(float d, float4 b) {
+    return make_float4(__fmul_rn(d, b.x), __fmul_rn(d, b.y), __fmul_rn(d, b.z), __fmul_rn(d, b.w));
+}
+__device__ __forceinline__ float4 fma4(float d, float4 b, float4 c) {
+    return make_float4(fmaf(d, b.x, c.x), fmaf(d, b.y, c.y), fmaf(d, b.z, c.z), fmaf(d, b.w, c.w));
+}
 
-// First pass: this warp's sums of channels 2 lane, 2 lane + 1 -> the set; block-wide call.
-__device__ __forceinline__ void put_sums(float* set, float2 v, float (*smem)[kLayerW]) {
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    reinterpret_cast<float2*>(set + ((int64_t)blockIdx.x * kSumWarps + w) * kLayerW)[lane] = v;
+// First pass: this range's sums of channels 4 l .. 4 l + 3 -> the set; block-wide call.
+__device__ __forceinline__ void put_sums(float* set, float4 v, float (*smem)[kLayerW]) {
+    const int h = threadIdx.x >> 4, l = threadIdx.x & 15;
+    reinterpret_cast<float4*>(set + ((int64_t)blockIdx.x * kSumParts + h) * kLayerW)[l] = v;
     __syncthreads();
-    reinterpret_cast<float2*>(smem[w])[lane] = v;
+    reinterpret_cast<float4*>(smem[h])[l] = v;
     __syncthreads();
     if (threadIdx.x < kLayerW) {
         float t = 0.f;
-#pragma unroll
-        for (int q = 0; q < kSumWarps; ++q) t += smem[q][threadIdx.x];
+#pragma unroll 8
+        for (int q = 0; q < kSumParts; ++q) t += smem[q][threadIdx.x];
         set[set_block(blockIdx.x) + threadIdx.x] = t;
     }
 }
-// Second pass: the sum of everything before this warp's range; block-wide call.
-__device__ __forceinline__ float2 get_prefix(const float* set, float (*smem)[kLayerW]) {
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float2 t = make_float2(0.f, 0.f);
+// Second pass: the sum of everything before this range; block-wide call.
+__device__ __forceinline__ float4 get_prefix(const float* set, float (*smem)[kLayerW]) {
+    const int h = threadIdx.x >> 4, l = threadIdx.x & 15;
+    float4 t = f4(0.f);
 #pragma unroll 4
-    for (int b = w; b < (int)blockIdx.x; b += kSumWarps) {
-        const float2 v = __ldcg(reinterpret_cast<const float2*>(set + set_block(b)) + lane);
-        t.x += v.x;
-        t.y += v.y;
-    }
+    for (int b = h; b < (int)blockIdx.x; b += kSumParts)
+        t = add4(t, __ldcg(reinterpret_cast<const float4*>(set + set_block(b)) + l));
     __syncthreads();
-    reinterpret_cast<float2*>(smem[w])[lane] = t;
+    reinterpret_cast<float4*>(smem[h])[l] = t;
     __syncthreads();
-    t = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int q = 0; q < kSumWarps; ++q) {
-        const float2 v = reinterpret_cast<const float2*>(smem[q])[lane];
-        t.x += v.x;
-        t.y += v.y;
-    }
-    for (int q = 0; q < w; ++q) {
-        const float2 v = __ldcg(reinterpret_cast<const float2*>(set + ((int64_t)blockIdx.x * kSumWarps + q) * kLayerW) + lane);
-        t.x += v.x;
-        t.y += v.y;
-    }
+    t = f4(0.f);
+#pragma unroll 8
+    for (int q = 0; q < kSumParts; ++q) t = add4(t, reinterpret_cast<const float4*>(smem[q])[l]);
+#pragma unroll 4
+    for (int q = 0; q < h; ++q)
+        t = add4(t, __ldcg(reinterpret_cast<const float4*>(set + ((int64_t)blockIdx.x * kSumParts + q) * kLayerW) + l));
     return t;
 }
-// Second pass: what this warp's accumulator gained (exact) -> the block's increment; block-wide call.
-__device__ __forceinline__ void put_delta(float* set, float2 acc, float2 start, float (*smem)[kLayerW]) {
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+// Second pass: what this range's accumulator gained (exact) -> the block's increment; block-wide call.
+__device__ __forceinline__ void put_delta(float* set, float4 acc, float4 start, float (*smem)[kLayerW]) {
+    const int h = threadIdx.x >> 4, l = threadIdx.x & 15;
     __syncthreads();
-    reinterpret_cast<float2*>(smem[w])[lane] = make_float2(acc.x - start.x, acc.y - start.y);
+    reinterpret_cast<float4*>(smem[h])[l] =
+        make_float4(acc.x - start.x, acc.y - start.y, acc.z - start.z, acc.w - start.w);
     __syncthreads();
     if (threadIdx.x < kLayerW) {
         double t = 0.0;
-#pragma unroll
-        for (int q = 0; q < kSumWarps; ++q) t += (double)smem[q][threadIdx.x];
+#pragma unroll 8
+        for (int q = 0; q < kSumParts; ++q) t += (double)smem[q][threadIdx.x];
         set[set_delta(blockIdx.x) + threadIdx.x] = (float)t;
     }
 }
@@ -1377,140 +1398,146 @@ __device__ __forceinline__ float silu_grad(float dh, float z) {
     const float s = 1.f / (1.f + __expf(-z));
     return dh * s * (1.f + z * (1.f - s));
 }
-__device__ __forceinline__ float2 silu_grad2(float2 dh, float2 z) {
-    return make_float2(silu_grad(dh.x, z.x), silu_grad(dh.y, z.y));
+__device__ __forceinline__ float4 silu_grad4(float4 dh, float4 z) {
+    return make_float4(silu_grad(dh.x, z.x), silu_grad(dh.y, z.y), silu_grad(dh.z, z.z), silu_grad(dh.w, z.w));
 }
-__device__ __forceinline__ void st_bf2(__nv_bfloat16* p, int64_t i, float2 v) {
-    reinterpret_cast<__nv_bfloat162*>(p)[i] = __floats2bfloat162_rn(v.x, v.y);
+__device__ __forceinline__ void st_bf4(__nv_bfloat16* p, int64_t i, float4 v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    reinterpret_cast<uint2*>(p)[i] =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+// Lane l's value of column l (l < 16) <-> columns 4 l .. 4 l + 3 of a set (the others are zero).
+__device__ __forceinline__ float4 spread(float v) {
+    const int lane = threadIdx.x & 31, l = lane & 15, base = lane & 16;
+    float t[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        t[e] = __shfl_sync(0xffffffffu, v, base | ((4 * l + e) & 15));
+        if (4 * l + e >= 16) t[e] = 0.f;
+    }
+    return make_float4(t[0], t[1], t[2], t[3]);
+}
+__device__ __forceinline__ float pick(float4 v) {
+    const int lane = threadIdx.x & 31, l = lane & 15, src = (lane & 16) | (l >> 2);
+    const float x = __shfl_sync(0xffffffffu, v.x, src), y = __shfl_sync(0xffffffffu, v.y, src);
+    const float z = __shfl_sync(0xffffffffu, v.z, src), w = __shfl_sync(0xffffffffu, v.w, src);
+    return (l & 2) ? ((l & 1) ? w : z) : ((l & 1) ? y : x);
 }
 
 // Decoder backward and the last layer's dZ: dh = dOut Wo, dZ = dh SiLU'(Z); first pass of the sums of
 // dOut^T h, dOut (sets [O] and [1] at `dec`) and dZ (`bias`).
 template <int O>
-__global__ void __launch_bounds__(kSumThreads) k_back_top(const float* __restrict__ h, const float* __restrict__ Wo,
+__global__ void __launch_bounds__(kSumThreads, 2) k_back_top(const float* __restrict__ h, const float* __restrict__ Wo,
                                                           const float* __restrict__ dOut, const float* __restrict__ Z,
                                                           int N, float* __restrict__ dh, __nv_bfloat16* __restrict__ dZ,
                                                           float* __restrict__ dec, float* __restrict__ bias) {
-    __shared__ __align__(16) float smem[kSumWarps][kLayerW];
-    const int lane = threadIdx.x & 31;
-    float2 w[O], aw[O], ao = make_float2(0.f, 0.f), ab = make_float2(0.f, 0.f);
+    __shared__ __align__(16) float smem[kSumParts][kLayerW];
+    __shared__ __align__(16) float s_wo[O][kLayerW];
+    const int l = threadIdx.x & 15;
+    for (int t = threadIdx.x; t < O * kLayerW; t += kSumThreads) s_wo[t / kLayerW][t % kLayerW] = __ldg(Wo + t);
+    __syncthreads();
+    float4 aw[O], ab = f4(0.f);
+    float ao = 0.f;                                          // column l of dOut
 #pragma unroll
-    for (int o = 0; o < O; ++o) {
-        w[o] = make_float2(__ldg(Wo + o * kLayerW + 2 * lane), __ldg(Wo + o * kLayerW + 2 * lane + 1));
-        aw[o] = make_float2(0.f, 0.f);
-    }
-    const Rows r = warp_rows(N);
-#pragma unroll 4
+    for (int o = 0; o < O; ++o) aw[o] = f4(0.f);
+    const Rows r = part_rows(N);
+#pragma unroll 2
     for (int64_t i = r.lo; i < r.hi; ++i) {
-        const float2 x = ldf2(h, i * 32 + lane), z = ldf2(Z, i * 32 + lane);
-        float2 v = make_float2(0.f, 0.f);
+        const float4 x = ldf4(h, i * 16 + l), z = ldf4(Z, i * 16 + l);
+        float4 v = f4(0.f);
 #pragma unroll
         for (int o = 0; o < O; ++o) {
             const float d = __ldg(dOut + i * O + o);
-            v.x = fmaf(d, w[o].x, v.x);
-            v.y = fmaf(d, w[o].y, v.y);
-            aw[o].x += d * x.x;
-            aw[o].y += d * x.y;
-            if (2 * lane == o) ao.x += d;
-            if (2 * lane + 1 == o) ao.y += d;
+            v = fma4(d, reinterpret_cast<const float4*>(s_wo[o])[l], v);
+            aw[o] = fma4(d, x, aw[o]);
         }
-        reinterpret_cast<float2*>(dh)[i * 32 + lane] = v;
-        const float2 g = silu_grad2(v, z);
-        st_bf2(dZ, i * 32 + lane, g);
-        ab.x += g.x;
-        ab.y += g.y;
+        if (l < O) ao += __ldg(dOut + i * O + l);
+        reinterpret_cast<float4*>(dh)[i * 16 + l] = v;
+        const float4 g = silu_grad4(v, z);
+        st_bf4(dZ, i * 16 + l, g);
+        ab = add4(ab, g);
     }
 #pragma unroll
     for (int o = 0; o < O; ++o) put_sums(dec + (int64_t)o * kSumSet, aw[o], smem);
-    put_sums(dec + (int64_t)O * kSumSet, ao, smem);
+    put_sums(dec + (int64_t)O * kSumSet, spread(ao), smem);
     put_sums(bias, ab, smem);
 }
 
 // Second pass of the decoder's sums.
 template <int O>
-__global__ void __launch_bounds__(kSumThreads) k_back_decoder(const float* __restrict__ h,
+__global__ void __launch_bounds__(kSumThreads, 2) k_back_decoder(const float* __restrict__ h,
                                                               const float* __restrict__ dOut, int N,
                                                               float* __restrict__ dec) {
-    __shared__ __align__(16) float smem[kSumWarps][kLayerW];
-    const int lane = threadIdx.x & 31;
-    float2 s0[O + 1], a[O + 1];
+    __shared__ __align__(16) float smem[kSumParts][kLayerW];
+    const int l = threadIdx.x & 15;
+    float4 s0[O], a[O];
 #pragma unroll
-    for (int o = 0; o <= O; ++o) a[o] = s0[o] = get_prefix(dec + (int64_t)o * kSumSet, smem);
-    const Rows r = warp_rows(N);
-#pragma unroll 4
+    for (int o = 0; o < O; ++o) a[o] = s0[o] = get_prefix(dec + (int64_t)o * kSumSet, smem);
+    const float so = pick(get_prefix(dec + (int64_t)O * kSumSet, smem));
+    float ao = so;                                           // column l of dOut
+    const Rows r = part_rows(N);
+#pragma unroll 2
     for (int64_t i = r.lo; i < r.hi; ++i) {
-        const float2 x = ldf2(h, i * 32 + lane);
+        const float4 x = ldf4(h, i * 16 + l);
 #pragma unroll
-        for (int o = 0; o < O; ++o) {
-            const float d = __ldg(dOut + i * O + o);
-            a[o].x = __fadd_rn(a[o].x, __fmul_rn(d, x.x));
-            a[o].y = __fadd_rn(a[o].y, __fmul_rn(d, x.y));
-            if (2 * lane == o) a[O].x = __fadd_rn(a[O].x, d);
-            if (2 * lane + 1 == o) a[O].y = __fadd_rn(a[O].y, d);
-        }
+        for (int o = 0; o < O; ++o) a[o] = add4(a[o], mul4(__ldg(dOut + i * O + o), x));
+        if (l < O) ao = __fadd_rn(ao, __ldg(dOut + i * O + l));
     }
 #pragma unroll
-    for (int o = 0; o <= O; ++o) put_delta(dec + (int64_t)o * kSumSet, a[o], s0[o], smem);
+    for (int o = 0; o < O; ++o) put_delta(dec + (int64_t)o * kSumSet, a[o], s0[o], smem);
+    put_delta(dec + (int64_t)O * kSumSet, spread(ao), spread(so), smem);
 }
 
 // Second pass of a bias gradient on its own (the input layer's).
-__global__ void __launch_bounds__(kSumThreads) k_back_bias(const float* __restrict__ dh, const float* __restrict__ Z,
+__global__ void __launch_bounds__(kSumThreads, 2) k_back_bias(const float* __restrict__ dh, const float* __restrict__ Z,
                                                            int N, float* __restrict__ bias) {
-    __shared__ __align__(16) float smem[kSumWarps][kLayerW];
-    const int lane = threadIdx.x & 31;
-    const float2 s0 = get_prefix(bias, smem);
-    float2 a = s0;
-    const Rows r = warp_rows(N);
+    __shared__ __align__(16) float smem[kSumParts][kLayerW];
+    const int l = threadIdx.x & 15;
+    const float4 s0 = get_prefix(bias, smem);
+    float4 a = s0;
+    const Rows r = part_rows(N);
 #pragma unroll 4
-    for (int64_t i = r.lo; i < r.hi; ++i) {
-        const float2 g = silu_grad2(ldf2(dh, i * 32 + lane), ldf2(Z, i * 32 + lane));
-        a.x = __fadd_rn(a.x, g.x);
-        a.y = __fadd_rn(a.y, g.y);
-    }
+    for (int64_t i = r.lo; i < r.hi; ++i) a = add4(a, silu_grad4(ldf4(dh, i * 16 + l), ldf4(Z, i * 16 + l)));
     put_delta(bias, a, s0, smem);
 }
 
 // dh = dh_in + dA[:, :64] + sum_{j in nbr} dA[j][64:], in that order; dZ = dh SiLU'(Z) with the first
 // pass of its column sums (bias), and the second pass of the layer above's (dh_in, Z_in, bias_in).
-// A warp per row, two channels per lane: every access is a whole 256-byte half row.  DEEP: the
-// neighbour count as a compile-time bound, so the gathers of several rows are in flight.
+// KM bounds the neighbour count at compile time; the lists are fetched a row ahead.
 template <int KM>
 __global__ void __launch_bounds__(kSumThreads, 2) k_back_gather(
     const float* __restrict__ dA, const int32_t* __restrict__ nbr, int N, int KN, const float* __restrict__ dh_in,
     const float* __restrict__ Z_in, float* __restrict__ bias_in, const float* __restrict__ Z, float* __restrict__ dh,
     __nv_bfloat16* __restrict__ dZ, float* __restrict__ bias) {
-    __shared__ __align__(16) float smem[kSumWarps][kLayerW];
-    const int lane = threadIdx.x & 31;
-    const float2 s0 = get_prefix(bias_in, smem);
-    float2 a = s0, ab = make_float2(0.f, 0.f);
-    const Rows r = warp_rows(N);
-#pragma unroll 2
+    __shared__ __align__(16) float smem[kSumParts][kLayerW], s_start[kSumParts][kLayerW];
+    const int l = threadIdx.x & 15;
+    float4 a = get_prefix(bias_in, smem), ab = f4(0.f);
+    float4* start = reinterpret_cast<float4*>(s_start[threadIdx.x >> 4]) + l;   // this thread's own, out of the registers
+    *start = a;
+    const Rows r = part_rows(N);
+    int next[KM];
+    auto fetch = [&](int64_t i) {
+#pragma unroll
+        for (int q = 0; q < KM; ++q) next[q] = q < KN && i < r.hi ? __ldg(nbr + i * KN + q) : -1;
+    };
+    fetch(r.lo);
     for (int64_t i = r.lo; i < r.hi; ++i) {
-        int j[KM];
+        float4 nb[KM];
 #pragma unroll
-        for (int q = 0; q < KM; ++q) j[q] = q < KN ? __ldg(nbr + i * KN + q) : -1;
-        const float2 own = ldf2(dA, i * 64 + lane), up = ldf2(dh_in, i * 32 + lane);
-        const float2 zi = ldf2(Z_in, i * 32 + lane), z = ldf2(Z, i * 32 + lane);
-        float2 nb[KM];
+        for (int q = 0; q < KM; ++q) nb[q] = next[q] >= 0 ? ldf4(dA, (int64_t)next[q] * 32 + 16 + l) : f4(0.f);
+        const float4 own = ldf4(dA, i * 32 + l), up = ldf4(dh_in, i * 16 + l);
+        const float4 zi = ldf4(Z_in, i * 16 + l), z = ldf4(Z, i * 16 + l);
+        fetch(i + 1);
+        a = add4(a, silu_grad4(up, zi));
+        float4 v = add4(own, up);
 #pragma unroll
-        for (int q = 0; q < KM; ++q) nb[q] = j[q] >= 0 ? ldf2(dA, (int64_t)j[q] * 64 + 32 + lane) : make_float2(0.f, 0.f);
-        const float2 gi = silu_grad2(up, zi);
-        a.x = __fadd_rn(a.x, gi.x);
-        a.y = __fadd_rn(a.y, gi.y);
-        float2 v = make_float2(own.x + up.x, own.y + up.y);
-#pragma unroll
-        for (int q = 0; q < KM; ++q)
-            if (j[q] >= 0) {
-                v.x += nb[q].x;
-                v.y += nb[q].y;
-            }
-        reinterpret_cast<float2*>(dh)[i * 32 + lane] = v;
-        const float2 g = silu_grad2(v, z);
-        st_bf2(dZ, i * 32 + lane, g);
-        ab.x += g.x;
-        ab.y += g.y;
+        for (int q = 0; q < KM; ++q) v = add4(v, nb[q]);
+        reinterpret_cast<float4*>(dh)[i * 16 + l] = v;
+        const float4 g = silu_grad4(v, z);
+        st_bf4(dZ, i * 16 + l, g);
+        ab = add4(ab, g);
     }
-    put_delta(bias_in, a, s0, smem);
+    put_delta(bias_in, a, *start, smem);
     put_sums(bias, ab, smem);
 }
 
@@ -1534,44 +1561,48 @@ __global__ void __launch_bounds__(256) k_back_finish(FinishArgs f) {
 }
 
 // One layer's products over the cells, a persistent kernel (one CTA per SM, 128-row tiles):
-//   warps 8-11 copy the tile's dZ (128 x 64) and A (128 x 128) into a three-stage ring (cp.async) in
-//   the unit layout of the forward layer; one thread issues the MMAs
+//   warp 8 copies the tile's dZ (128 x 64) and A (128 x 128, two halves) into a four-stage ring with
+//   TMA in the 128-byte swizzle (64 channels of a row = one swizzled line; rows past N read as zero);
+//   warp 9 issues the MMAs
 //     dA  [128 x 128] = dZ . W       (K-major dZ and W^T; two accumulators)
 //     dW^T [128 x 64] += A^T . dZ    (the same copies read MN-major, the tile's rows as K; one
 //                                     accumulator in tensor memory for the CTA's whole run);
 //   warps 0-7 read dA (warp w: TMEM lanes 32 (w % 4), columns 64 (w / 4)), divide the neighbour half
-//   by the row's neighbour count and store it.  At the end the CTA adds its dW^T to dW.
+//   by the row's neighbour count and store it, a row's 32 columns on four lanes as one 128-byte line.
+//   At the end the CTA adds its dW^T to dW.
 // Without dA (the input layer) A is the [N][64] feature rows and only dW is formed.
-constexpr int kBackLoaders = 128, kBackThreads = 256 + kBackLoaders, kBackStages = 3;
-constexpr int kBackStage = 8 * kUnitBytes + kLayerABytes;                        // dZ and A of one tile
-constexpr int kBackSmem = kBackStages * kBackStage + 8 * kUnitBytes;             // + W^T (128 x 64)
+// Bound by memory, 0.9 kB per row.  Copies by four warps' cp.async into no-swizzle operands held the L1's
+// path for 3000 cycles per tile, and their warp also issued the MMAs (2200 cycles per tile); with stores
+// of one row per lane that took 75 us per layer at 278 k rows.
+constexpr int kBackThreads = 320, kBackStages = 4;
+constexpr int kBackHalf = TM * kLayerW * 2;                                      // 128 rows x 64 channels
+constexpr int kBackStage = 3 * kBackHalf;                                        // dZ and A of one tile
+constexpr int kBackSmem = 1024 + kBackStages * kBackStage + 8 * kUnitBytes;      // + alignment, W^T (128 x 64)
 
-__device__ __forceinline__ int loaders_or(int v) {       // named barrier of the loaders, with an OR
-    int r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.b32 p, %1, 0;\n\t"
-        "bar.red.or.pred q, 1, 128, p;\n\t"
-        "selp.b32 %0, 1, 0, q;\n\t}\n"
-        : "=r"(r)
-        : "r"(v)
-        : "memory");
-    return r;
+// 128-byte-swizzled operand: atoms of 8 rows x 128 bytes, 1024 bytes apart along the rows; `lbo` apart
+// along the channels (MN-major reads of more than 64 channels).
+__device__ __forceinline__ uint64_t make_desc_sw(uint32_t saddr, uint32_t lbo) {
+    return make_desc(saddr, lbo, 1024) | (uint64_t)2 << 61;
 }
-__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool valid) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+__device__ __forceinline__ void tma_tile(uint32_t dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            dst),
+        "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+        : "memory");
 }
 
 template <bool LAYER>
-__global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __nv_bfloat16* __restrict__ dZ,
-                                                                const __nv_bfloat16* __restrict__ A,
+__global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __grid_constant__ CUtensorMap map_z,
+                                                                const __grid_constant__ CUtensorMap map_a,
                                                                 const __nv_bfloat16* __restrict__ WT,
                                                                 const int32_t* __restrict__ nbr, int KN, int N,
                                                                 float* __restrict__ dA, float* __restrict__ dW,
                                                                 int* __restrict__ err) {
-    extern __shared__ __align__(1024) uint8_t smem[];
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
     uint8_t* sW = smem + kBackStages * kBackStage;
-    __shared__ __align__(8) uint64_t bar_free[kBackStages], bar_full[2], bar_empty[2];
+    __shared__ __align__(8) uint64_t bar_load[kBackStages], bar_free[kBackStages], bar_full[2], bar_empty[2];
     __shared__ uint32_t s_taddr;
     __shared__ int s_fail, s_last;
     constexpr int AU = LAYER ? 16 : 8;                    // 8-channel units of an A row
@@ -1584,7 +1615,10 @@ __global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __nv_bfloa
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        for (int b = 0; b < kBackStages; ++b) mbar_init(&bar_free[b], 1);
+        for (int b = 0; b < kBackStages; ++b) {
+            mbar_init(&bar_load[b], 1);
+            mbar_init(&bar_free[b], 1);
+        }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&bar_full[b], 1);
             mbar_init(&bar_empty[b], 8);
@@ -1595,12 +1629,12 @@ __global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __nv_bfloa
     }
     if (LAYER) {
         for (int t = tid; t < TM * 8; t += kBackThreads)
-            *reinterpret_cast<uint4*>(sW + (t & 7) * kUnitBytes + (t >> 3) * 16) =
+            *reinterpret_cast<uint4*>(sW + (t & 7) * kUnitBytes + frag_col(t >> 3) * 16) =
                 *reinterpret_cast<const uint4*>(WT + (int64_t)(t >> 3) * kLayerW + 8 * (t & 7));
     } else {   // rows 64..127 of the input layer's dW^T read zeros
         for (int st = 0; st < kBackStages; ++st)
-            for (int t = tid; t < 8 * kUnitBytes / 16; t += kBackThreads)
-                reinterpret_cast<uint4*>(smem + st * kBackStage + 16 * kUnitBytes)[t] = make_uint4(0u, 0u, 0u, 0u);
+            for (int t = tid; t < kBackHalf / 16; t += kBackThreads)
+                reinterpret_cast<uint4*>(smem + st * kBackStage + 2 * kBackHalf)[t] = make_uint4(0u, 0u, 0u, 0u);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -1610,95 +1644,98 @@ __global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __nv_bfloa
     const uint32_t id_a = make_idesc(TM);
     const uint32_t id_w = make_idesc(kLayerW) | (1u << 15) | (1u << 16);   // both operands MN-major
 
-    if (warp >= 8) {
-        const int lt = tid - 256;
-        auto load = [&](int k) {
-            if (k < nlocal) {
-                const int64_t m0 = (int64_t)((int)blockIdx.x + k * (int)gridDim.x) * TM;
-                const uint32_t sz = smem_u32(smem + (k % kBackStages) * kBackStage), sa = sz + 8 * kUnitBytes;
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const int t = lt + q * kBackLoaders, r = (t & 7) + 8 * (t >> 6), u = (t >> 3) & 7;
-                    const bool on = m0 + r < N;
-                    cp16(sz + u * kUnitBytes + r * 16, dZ + (on ? m0 + r : 0) * kLayerW + 8 * u, on);
+    if (warp == 8) {
+        if (lane == 0) {
+            int k = 0;
+            for (; k < nlocal; ++k) {
+                const int st = k % kBackStages, m0 = ((int)blockIdx.x + k * (int)gridDim.x) * TM;
+                if (k >= kBackStages && !mbar_wait(&bar_free[st], (uint32_t)((k / kBackStages - 1) & 1))) {
+                    atomicExch(&s_fail, 1);
+                    break;
                 }
-#pragma unroll
-                for (int q = 0; q < AU; ++q) {
-                    const int t = lt + q * kBackLoaders, r = (t & 7) + 8 * (t / (8 * AU)), u = (t >> 3) % AU;
-                    const bool on = m0 + r < N;
-                    cp16(sa + u * kUnitBytes + r * 16, A + (on ? m0 + r : 0) * (8 * AU) + 8 * u, on);
-                }
+                const uint32_t sz = smem_u32(smem + st * kBackStage);
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&bar_load[st])),
+                             "r"((LAYER ? 3 : 2) * kBackHalf)
+                             : "memory");
+                tma_tile(sz, &map_z, 0, m0, &bar_load[st]);
+                tma_tile(sz + kBackHalf, &map_a, 0, m0, &bar_load[st]);
+                if (LAYER) tma_tile(sz + 2 * kBackHalf, &map_a, kLayerW, m0, &bar_load[st]);
             }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-        load(0);
-        load(1);
-        int fail = 0;
-        for (int k = 0; k < nlocal; ++k) {
-            if (k >= 1 && !fail)                          // the MMAs of tile k - 1 read the stage of tile k + 2
-                fail = !mbar_wait(&bar_free[(k - 1) % kBackStages], (uint32_t)(((k - 1) / kBackStages) & 1));
-            if (!fail) load(k + 2);
-            else asm volatile("cp.async.commit_group;" ::: "memory");
-            asm volatile("cp.async.wait_group 2;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            fail = loaders_or(fail);
-            if (fail) break;
-            if (lt == 0) {
+            // no copy outlives the CTA, also when a wait gave up
+            for (int j = max(0, k - kBackStages); j < k; ++j)
+                if (!mbar_wait(&bar_load[j % kBackStages], (uint32_t)((j / kBackStages) & 1))) atomicExch(&s_fail, 1);
+        }
+    } else if (warp == 9) {
+        if (lane == 0) {
+            for (int k = 0; k < nlocal; ++k) {
                 const int a = k & 1, st = k % kBackStages;
-                if (LAYER && k >= 2) fail = !mbar_wait(&bar_empty[a], (uint32_t)(((k >> 1) - 1) & 1));
-                if (!fail) {
-                    asm volatile("tcgen05.fence::after_thread_sync;");
-                    const uint32_t sz = smem_u32(smem + st * kBackStage), sa = sz + 8 * kUnitBytes;
-                    if (LAYER)
-#pragma unroll
-                        for (int q = 0; q < kLayerW / 16; ++q)
-                            tc_mma(taddr + a * TM, make_desc(sz + 2 * q * kUnitBytes, kUnitBytes, 128),
-                                   make_desc(smem_u32(sW) + 2 * q * kUnitBytes, kUnitBytes, 128), id_a, q > 0);
-#pragma unroll
-                    for (int q = 0; q < TM / 16; ++q)
-                        tc_mma(tw, make_desc(sa + q * 256, 128, kUnitBytes), make_desc(sz + q * 256, 128, kUnitBytes),
-                               id_w, k > 0 || q > 0);
-                    tc_commit(&bar_free[st]);
-                    tc_commit(&bar_full[a]);
-                    s_last = k;
+                if (!mbar_wait(&bar_load[st], (uint32_t)((k / kBackStages) & 1)) ||
+                    (LAYER && k >= 2 && !mbar_wait(&bar_empty[a], (uint32_t)(((k >> 1) - 1) & 1)))) {
+                    atomicExch(&s_fail, 1);
+                    break;
                 }
+                asm volatile("tcgen05.fence::after_thread_sync;");
+                const uint32_t sz = smem_u32(smem + st * kBackStage), sa = sz + kBackHalf;
+                if (LAYER)
+#pragma unroll
+                    for (int q = 0; q < kLayerW / 16; ++q)
+                        tc_mma(taddr + a * TM, make_desc_sw(sz + 32 * q, 16),
+                               make_desc(smem_u32(sW) + 2 * q * kUnitBytes, kUnitBytes, 128), id_a, q > 0);
+#pragma unroll
+                for (int q = 0; q < TM / 16; ++q)
+                    tc_mma(tw, make_desc_sw(sa + 2048 * q, kBackHalf), make_desc_sw(sz + 2048 * q, kBackHalf), id_w,
+                           k > 0 || q > 0);
+                tc_commit(&bar_free[st]);
+                tc_commit(&bar_full[a]);
+                s_last = k;
             }
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        if (fail) atomicExch(&s_fail, 1);
     } else if (LAYER) {
         const int half = warp >> 2;
+        int next[8];                                      // row `lane`'s neighbours, fetched a tile ahead
+        auto fetch = [&](int k) {
+            const int64_t row = (int64_t)((int)blockIdx.x + k * (int)gridDim.x) * TM + 32 * (warp & 3) + lane;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) next[q] = half && k < nlocal && row < N && q < KN ? __ldg(nbr + row * KN + q) : -1;
+        };
+        fetch(0);
         for (int k = 0; k < nlocal; ++k) {
             const int a = k & 1;
-            const int64_t row = (int64_t)((int)blockIdx.x + k * (int)gridDim.x) * TM + 32 * (warp & 3) + lane;
+            const int64_t m0 = (int64_t)((int)blockIdx.x + k * (int)gridDim.x) * TM + 32 * (warp & 3);
             int deg = 0;
-            if (half && row < N)
-                for (int q = 0; q < KN; ++q) deg += __ldg(nbr + row * KN + q) >= 0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) deg += next[q] >= 0;
+            fetch(k + 1);
             const bool ok = mbar_wait(&bar_full[a], (uint32_t)((k >> 1) & 1));
             if (!__all_sync(0xffffffffu, ok)) {
                 if (lane == 0) atomicExch(&s_fail, 1);
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;");
-            uint32_t v[2][32];
+            uint32_t v[2][2][16];                         // 16-row group, 32-column group
             const uint32_t base = taddr + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(a * TM + 64 * half);
-            tmem_ld32(base, v[0]);
-            tmem_ld32(base + 32, v[1]);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) tmem_ld_frag(base + ((uint32_t)(16 * (t >> 1)) << 16) + 32 * (t & 1), v[t >> 1][t & 1]);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;");
             __syncwarp();
             if (lane == 0) mbar_arrive(&bar_empty[a]);
-            if (row < N) {
-                const float d = (float)max(deg, 1);
-                float* dst = dA + row * TM + 64 * half;
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    float x[8];
+            for (int t = 0; t < 4; ++t) {
+                const int r = 8 * t + (lane >> 2);
+                const float d = (float)max(__shfl_sync(0xffffffffu, deg, r), 1);
+                if (m0 + r < N) {
+                    float* dst = dA + (m0 + r) * TM + 64 * half + 8 * (lane & 3);
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        x[e] = __uint_as_float(v[q >> 2][8 * (q & 3) + e]);
-                        if (half) x[e] = x[e] / d;
+                    for (int c = 0; c < 2; ++c) {
+                        float x[8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            x[e] = __uint_as_float(v[t >> 1][c][4 * (e >> 1) + 2 * (t & 1) + (e & 1)]);
+                            if (half) x[e] = x[e] / d;
+                        }
+                        st8(dst + 32 * c, x);
                     }
-                    st8(dst + 8 * q, x);
                 }
             }
         }
@@ -1726,6 +1763,27 @@ __global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __nv_bfloa
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(512u));
 }
 
+// Tensor map of bf16 rows [N][cols] in boxes of 128 rows x 64 columns, 128-byte swizzle.
+static bool tile_map(CUtensorMap* map, const void* base, int cols, int N) {
+    using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return reinterpret_cast<Encode>(f);
+    }();
+    if (!encode) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)N}, strides[1] = {(cuuint64_t)cols * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)kLayerW, (cuuint32_t)TM}, step[2] = {1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, step,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <bool LAYER>
 static int launch_back_layer(const void* dZ, const void* A, const void* WT, const int32_t* nbr, int KN, int N,
                              float* dA, float* dW, int* err, cudaStream_t s) {
@@ -1745,10 +1803,11 @@ static int launch_back_layer(const void* dZ, const void* A, const void* WT, cons
         }
         sms[dev] = n;
     }
+    CUtensorMap map_z, map_a;
+    if (!tile_map(&map_z, dZ, kLayerW, N) || !tile_map(&map_a, A, LAYER ? 2 * kLayerW : kLayerW, N)) return FVM_E_CUDA;
     const unsigned grid = (unsigned)std::min((N + TM - 1) / TM, sms[dev]);
     FVM_LAUNCH(KID_CORRECTOR, s, k_back_layer<LAYER><<<grid, kBackThreads, kBackSmem, s>>>(
-                                     static_cast<const __nv_bfloat16*>(dZ), static_cast<const __nv_bfloat16*>(A),
-                                     static_cast<const __nv_bfloat16*>(WT), nbr, KN, N, dA, dW, err));
+                                     map_z, map_a, static_cast<const __nv_bfloat16*>(WT), nbr, KN, N, dA, dW, err));
     return launch_status();
 }
 
@@ -1772,8 +1831,8 @@ static inline bool aligned(const void* p, int b) { return ((uintptr_t)p & (b - 1
 extern "C" int fvm_back_top(const float* h, const float* Wo, const float* dOut, const float* Z, int32_t N, int32_t O,
                             float* dh, void* dZ, float* dec, float* bias, void* stream) {
     if (!h || !Wo || !dOut || !Z || !dh || !dZ || !dec || !bias || N <= 0 || O < 1 || O > 8) return FVM_E_ARG;
-    if (!corr::aligned(h, 8) || !corr::aligned(Z, 8) || !corr::aligned(dh, 8) || !corr::aligned(dZ, 4) ||
-        !corr::aligned(dec, 8) || !corr::aligned(bias, 8))
+    if (!corr::aligned(h, 16) || !corr::aligned(Z, 16) || !corr::aligned(dh, 16) || !corr::aligned(dZ, 8) ||
+        !corr::aligned(dec, 16) || !corr::aligned(bias, 16))
         return FVM_E_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     __nv_bfloat16* z = static_cast<__nv_bfloat16*>(dZ);
@@ -1785,7 +1844,7 @@ extern "C" int fvm_back_top(const float* h, const float* Wo, const float* dOut, 
 }
 
 extern "C" int fvm_back_decoder(const float* h, const float* dOut, int32_t N, int32_t O, float* dec, void* stream) {
-    if (!h || !dOut || !dec || N <= 0 || O < 1 || O > 8 || !corr::aligned(h, 8) || !corr::aligned(dec, 8))
+    if (!h || !dOut || !dec || N <= 0 || O < 1 || O > 8 || !corr::aligned(h, 16) || !corr::aligned(dec, 16))
         return FVM_E_ARG;
     cudaStream_t s = (cudaStream_t)stream;
 #define FVM_CALL(OO) FVM_LAUNCH(KID_CORRECTOR, s, corr::k_back_decoder<OO><<<corr::kSumBlocks, corr::kSumThreads, 0, s>>>( \
@@ -1810,8 +1869,8 @@ extern "C" int fvm_back_gather(const float* dA, const int32_t* nbr, int32_t N, i
     if (!dA || !nbr || !dh_in || !Z_in || !bias_in || !Z || !dh || !dZ || !bias || N <= 0 || KN <= 0 || KN > 8 ||
         dh == dh_in)
         return FVM_E_ARG;
-    if (!corr::aligned(dA, 8) || !corr::aligned(dh_in, 8) || !corr::aligned(Z_in, 8) || !corr::aligned(Z, 8) ||
-        !corr::aligned(dh, 8) || !corr::aligned(dZ, 4) || !corr::aligned(bias_in, 8) || !corr::aligned(bias, 8))
+    if (!corr::aligned(dA, 16) || !corr::aligned(dh_in, 16) || !corr::aligned(Z_in, 16) || !corr::aligned(Z, 16) ||
+        !corr::aligned(dh, 16) || !corr::aligned(dZ, 8) || !corr::aligned(bias_in, 16) || !corr::aligned(bias, 16))
         return FVM_E_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     __nv_bfloat16* z = static_cast<__nv_bfloat16*>(dZ);
@@ -1825,7 +1884,7 @@ extern "C" int fvm_back_gather(const float* dA, const int32_t* nbr, int32_t N, i
 }
 
 extern "C" int fvm_back_bias(const float* dh, const float* Z, int32_t N, float* bias, void* stream) {
-    if (!dh || !Z || !bias || N <= 0 || !corr::aligned(dh, 8) || !corr::aligned(Z, 8) || !corr::aligned(bias, 8))
+    if (!dh || !Z || !bias || N <= 0 || !corr::aligned(dh, 16) || !corr::aligned(Z, 16) || !corr::aligned(bias, 16))
         return FVM_E_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     FVM_LAUNCH(KID_CORRECTOR, s, corr::k_back_bias<<<corr::kSumBlocks, corr::kSumThreads, 0, s>>>(dh, Z, N, bias));

@@ -402,8 +402,8 @@ int fvm_corrector_in_layer(const float *state, const float *r0, const float *dt,
 int fvm_corrector_propose(const float *state, const float *base, const float *out, const float *scale,
                           const double *sums, const double *case_vol, int32_t first, const int32_t *cell_case, int32_t N,
                           int32_t C, float *prop, void *stream);
-/* Backward pass of the network (64 channels; fp32 rows 8-byte, bf16 rows 16-byte aligned, dA 32-byte).
- * Sums over the cells use workspace sets of FVM_BACK_SET floats (8-byte aligned, no clearing needed):
+/* Backward pass of the network (64 channels; rows 16-byte aligned, dA 32-byte).  Sums over the cells use
+ * workspace sets of FVM_BACK_SET floats (16-byte aligned, no clearing needed):
  * one for each bias gradient and O + 1 consecutive ones (`dec`) for the decoder.  A set is filled by a
  * first and a second pass over the same terms, and fvm_back_finish adds set q's n[q] column sums to
  * dst[q] (host arrays, at most 32 sets).  A column sum has the value of one fp32 accumulator that
@@ -416,7 +416,7 @@ int fvm_corrector_propose(const float *state, const float *base, const float *ou
  *   fvm_back_gather:  dh = dh_in + dA[:, :64] + sum_{j in nbr(i)} dA[j][64:]; dZ = dh SiLU'(Z) with the first
  *                     pass of bias; second pass of bias_in (dh_in, Z_in).  dh must not alias dh_in.
  *   fvm_back_bias:    second pass of bias alone (dh, Z) */
-#define FVM_BACK_SET ((296 * 16 + 2 * 296) * 64)
+#define FVM_BACK_SET ((296 * 24 + 2 * 296) * 64)
 int fvm_back_top(const float *h, const float *Wo, const float *dOut, const float *Z, int32_t N, int32_t O, float *dh,
                  void *dZ, float *dec, float *bias, void *stream);
 int fvm_back_decoder(const float *h, const float *dOut, int32_t N, int32_t O, float *dec, void *stream);

@@ -73,7 +73,7 @@ def test_forward_forms(N, KN, O):
     assert int(err.item()) == 0
 
 
-@pytest.mark.parametrize("N,KN,O", [(1, 1, 1), (127, 3, 4), (129, 4, 5), (700, 8, 8), (40_001, 3, 4)])
+@pytest.mark.parametrize("N,KN,O", [(1, 1, 1), (127, 3, 4), (129, 4, 5), (700, 8, 8), (40_001, 3, 4), (100_001, 4, 5)])
 def test_backward_kernels(N, KN, O):
     from fvm_solver_b200 import _lib
     lib, s = _lib.load(), _lib.stream_ptr()
