@@ -17,7 +17,7 @@ FVM_OK, FVM_E_ARG, FVM_E_CUDA, FVM_E_UNSUPPORTED, FVM_E_CAPACITY = 0, -1, -2, -3
 FVM_NOALLOC_SCRATCH_BYTES = 16 * 1024 * 1024
 FVM_MAX_STAGES = 12
 FVM_RED_DOUBLES = 64
-FVM_BACK_SET = (296 * 24 + 2 * 296) * 64
+FVM_BACK_SET = 2 * 296 * 64
 FVM_PHASE_BC, FVM_PHASE_CELLS, FVM_PHASE_FACES, FVM_PHASE_DIV = 1, 2, 4, 8
 
 _P = ct.c_void_p

@@ -1298,41 +1298,40 @@ extern "C" int fvm_decoder_back_f32(const float* h, const float* Wo, const float
 //     neighbour count) and dW += dZ^T A, both on tcgen05 from one staged copy of the tile;
 //   * k_back_gather: dh_l = dh_{l+1} + dA[:, :64] + sum over neighbours of dA[:, 64:], then
 //     dZ = dh_l SiLU'(Z_l) for the layer below.
-// Both are bound by memory: 0.9 kB and 1.7 kB per cell and layer (57 and 100 us at 278 k cells, 4.4 and
-// 4.6 TB/s).  They replace a SiLU kernel
+// Both are bound by memory: 0.9 kB and 1.7 kB per cell and layer (50 and 86 us at 278 k cells, 5.0 and
+// 5.4 TB/s).  They replace a SiLU kernel
 // with one atomic per element (1178 us per layer at 278 k cells), two transposes, two GEMMs with
 // their operands read again and a scatter that counted every neighbour's neighbours.
 //
 // Column sums (the gradients of the biases and of the decoder) keep the value of one running fp32 sum
 // over the cells in order: with terms of one sign that sum's rounding is systematic (1.6e-4 of the
 // decoder's gradient at 278 k cells), so summing pieces from zero would move the results.  Rounding
-// a + t to fp32 depends on a only through its binade, so each half-warp walks a contiguous range of rows
-// with an accumulator that starts at the sum of everything before it, taken from a first pass over the
-// same terms, and what it added is exact: the first pass runs in the kernel that produces the terms,
-// the second in the next kernel that reads them, the ranges' increments are added up once at the
+// a + t to fp32 depends on a only through its binade, so a block walks a contiguous range of rows with
+// accumulators that start at the sum of everything before it, taken from a first pass over the same
+// terms, and what they added is exact: the first pass runs in the kernel that produces the terms, the
+// second in the next kernel that reads them, the blocks' increments are added up once at the
 // end (k_back_finish).  The result does not depend on scheduling.
 // ------------------------------------------------------------------------------------------
 namespace fvm {
 namespace corr {
 
-// Row ranges belong to half-warps: 16 lanes with four channels each read a row as one 256-byte piece, and
-// a warp has two rows in flight per load (two channels per lane and a row per warp took 118 us per
-// gather at 278 k cells).
+// A block owns a contiguous range of rows; its half-warps (16 lanes with four channels each) take them in
+// turn, a row as one 256-byte piece, with the loads of two to four rows issued together.  At 278 k cells:
+// gather 86 us, input bias 29, decoder 31, top 51; with a range per warp and two channels per lane
+// (4736 streams, and the compiler's own unrolling) 116, 47, 45 and 65.
 constexpr int kSumBlocks = 2 * 148, kSumThreads = 384, kSumParts = kSumThreads / 16;
-constexpr int kSumSegs = kSumBlocks * kSumParts;         // row ranges, one per half-warp
-// One set of 64 column sums: the ranges' sums, the blocks' sums, the blocks' increments.
-constexpr int kSumSet = (kSumSegs + 2 * kSumBlocks) * kLayerW;
+// One set of 64 column sums: the blocks' sums, the blocks' increments.
+constexpr int kSumSet = 2 * kSumBlocks * kLayerW;
 static_assert(kSumSet == FVM_BACK_SET, "workspace size");
-__host__ __device__ __forceinline__ constexpr int set_block(int b) { return (kSumSegs + b) * kLayerW; }
-__host__ __device__ __forceinline__ constexpr int set_delta(int b) { return (kSumSegs + kSumBlocks + b) * kLayerW; }
+__host__ __device__ __forceinline__ constexpr int set_block(int b) { return b * kLayerW; }
+__host__ __device__ __forceinline__ constexpr int set_delta(int b) { return (kSumBlocks + b) * kLayerW; }
 
 struct Rows {
-    int64_t lo, hi;
+    int64_t lo, hi;                                      // lo, lo + kSumParts, ... below hi
 };
 __device__ __forceinline__ Rows part_rows(int N) {
-    const int64_t per = ((int64_t)N + kSumSegs - 1) / kSumSegs;
-    const int64_t lo = ((int64_t)blockIdx.x * kSumParts + (threadIdx.x >> 4)) * per;
-    return Rows{min(lo, (int64_t)N), min(lo + per, (int64_t)N)};
+    const int64_t per = ((int64_t)N + kSumBlocks - 1) / kSumBlocks, lo = (int64_t)blockIdx.x * per;
+    return Rows{lo + (threadIdx.x >> 4), min(lo + per, (int64_t)N)};
 }
 __device__ __forceinline__ float4 ldf4(const float* p, int64_t i) { return __ldg(reinterpret_cast<const float4*>(p) + i); }
 __device__ __forceinline__ float4 f4(float v) { return make_float4(v, v, v, v); }
@@ -1346,10 +1345,9 @@ __device__ __forceinline__ float4 fma4(float d, float4 b, float4 c) {
     return make_float4(fmaf(d, b.x, c.x), fmaf(d, b.y, c.y), fmaf(d, b.z, c.z), fmaf(d, b.w, c.w));
 }
 
-// First pass: this range's sums of channels 4 l .. 4 l + 3 -> the set; block-wide call.
+// First pass: this half-warp's sums of channels 4 l .. 4 l + 3 -> the set; block-wide call.
 __device__ __forceinline__ void put_sums(float* set, float4 v, float (*smem)[kLayerW]) {
     const int h = threadIdx.x >> 4, l = threadIdx.x & 15;
-    reinterpret_cast<float4*>(set + ((int64_t)blockIdx.x * kSumParts + h) * kLayerW)[l] = v;
     __syncthreads();
     reinterpret_cast<float4*>(smem[h])[l] = v;
     __syncthreads();
@@ -1360,25 +1358,30 @@ __device__ __forceinline__ void put_sums(float* set, float4 v, float (*smem)[kLa
         set[set_block(blockIdx.x) + threadIdx.x] = t;
     }
 }
-// Second pass: the sum of everything before this range; block-wide call.
-__device__ __forceinline__ float4 get_prefix(const float* set, float (*smem)[kLayerW]) {
+// Second pass: the sums of everything before this block's range, for S consecutive sets; block-wide call.
+template <int S>
+__device__ __forceinline__ void get_prefix(const float* set, float4 (&out)[S], float (*smem)[kLayerW]) {
     const int h = threadIdx.x >> 4, l = threadIdx.x & 15;
-    float4 t = f4(0.f);
-#pragma unroll 4
-    for (int b = h; b < (int)blockIdx.x; b += kSumParts)
-        t = add4(t, __ldcg(reinterpret_cast<const float4*>(set + set_block(b)) + l));
-    __syncthreads();
-    reinterpret_cast<float4*>(smem[h])[l] = t;
-    __syncthreads();
-    t = f4(0.f);
+    constexpr int kLoads = (kSumBlocks + kSumParts - 1) / kSumParts;
+#pragma unroll
+    for (int o = 0; o < S; ++o) {
+        float4 t = f4(0.f);
+#pragma unroll
+        for (int j = 0; j < kLoads; ++j) {
+            const int b = h + j * kSumParts;
+            if (b < (int)blockIdx.x)
+                t = add4(t, __ldcg(reinterpret_cast<const float4*>(set + (int64_t)o * kSumSet + set_block(b)) + l));
+        }
+        __syncthreads();
+        reinterpret_cast<float4*>(smem[h])[l] = t;
+        __syncthreads();
+        t = f4(0.f);
 #pragma unroll 8
-    for (int q = 0; q < kSumParts; ++q) t = add4(t, reinterpret_cast<const float4*>(smem[q])[l]);
-#pragma unroll 4
-    for (int q = 0; q < h; ++q)
-        t = add4(t, __ldcg(reinterpret_cast<const float4*>(set + ((int64_t)blockIdx.x * kSumParts + q) * kLayerW) + l));
-    return t;
+        for (int q = 0; q < kSumParts; ++q) t = add4(t, reinterpret_cast<const float4*>(smem[q])[l]);
+        out[o] = t;
+    }
 }
-// Second pass: what this range's accumulator gained (exact) -> the block's increment; block-wide call.
+// Second pass: what this half-warp's accumulator gained (exact) -> the block's increment; block-wide call.
 __device__ __forceinline__ void put_delta(float* set, float4 acc, float4 start, float (*smem)[kLayerW]) {
     const int h = threadIdx.x >> 4, l = threadIdx.x & 15;
     __syncthreads();
@@ -1441,21 +1444,37 @@ __global__ void __launch_bounds__(kSumThreads, 2) k_back_top(const float* __rest
 #pragma unroll
     for (int o = 0; o < O; ++o) aw[o] = f4(0.f);
     const Rows r = part_rows(N);
-#pragma unroll 2
-    for (int64_t i = r.lo; i < r.hi; ++i) {
-        const float4 x = ldf4(h, i * 16 + l), z = ldf4(Z, i * 16 + l);
-        float4 v = f4(0.f);
+    constexpr int kBatch = 2;                             // rows in flight; past the range they add +0
+    for (int64_t i0 = r.lo; i0 < r.hi; i0 += kBatch * kSumParts) {
+        float4 x[kBatch], z[kBatch];
+        float d[kBatch][O], c[kBatch];
 #pragma unroll
-        for (int o = 0; o < O; ++o) {
-            const float d = __ldg(dOut + i * O + o);
-            v = fma4(d, reinterpret_cast<const float4*>(s_wo[o])[l], v);
-            aw[o] = fma4(d, x, aw[o]);
+        for (int u = 0; u < kBatch; ++u) {
+            const int64_t i = i0 + u * kSumParts;
+            const bool on = i < r.hi;
+            x[u] = on ? ldf4(h, i * 16 + l) : f4(0.f);
+            z[u] = on ? ldf4(Z, i * 16 + l) : f4(0.f);
+            c[u] = on && l < O ? __ldg(dOut + i * O + l) : 0.f;
+#pragma unroll
+            for (int o = 0; o < O; ++o) d[u][o] = on ? __ldg(dOut + i * O + o) : 0.f;
         }
-        if (l < O) ao += __ldg(dOut + i * O + l);
-        reinterpret_cast<float4*>(dh)[i * 16 + l] = v;
-        const float4 g = silu_grad4(v, z);
-        st_bf4(dZ, i * 16 + l, g);
-        ab = add4(ab, g);
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+            const int64_t i = i0 + u * kSumParts;
+            float4 v = f4(0.f);
+#pragma unroll
+            for (int o = 0; o < O; ++o) {
+                v = fma4(d[u][o], reinterpret_cast<const float4*>(s_wo[o])[l], v);
+                aw[o] = fma4(d[u][o], x[u], aw[o]);
+            }
+            ao += c[u];
+            const float4 g = silu_grad4(v, z[u]);
+            if (i < r.hi) {
+                reinterpret_cast<float4*>(dh)[i * 16 + l] = v;
+                st_bf4(dZ, i * 16 + l, g);
+            }
+            ab = add4(ab, g);
+        }
     }
 #pragma unroll
     for (int o = 0; o < O; ++o) put_sums(dec + (int64_t)o * kSumSet, aw[o], smem);
@@ -1470,18 +1489,31 @@ __global__ void __launch_bounds__(kSumThreads, 2) k_back_decoder(const float* __
                                                               float* __restrict__ dec) {
     __shared__ __align__(16) float smem[kSumParts][kLayerW];
     const int l = threadIdx.x & 15;
-    float4 s0[O], a[O];
+    float4 s0[O + 1], a[O];
+    get_prefix<O + 1>(dec, s0, smem);
 #pragma unroll
-    for (int o = 0; o < O; ++o) a[o] = s0[o] = get_prefix(dec + (int64_t)o * kSumSet, smem);
-    const float so = pick(get_prefix(dec + (int64_t)O * kSumSet, smem));
+    for (int o = 0; o < O; ++o) a[o] = s0[o];
+    const float so = pick(s0[O]);
     float ao = so;                                           // column l of dOut
     const Rows r = part_rows(N);
-#pragma unroll 2
-    for (int64_t i = r.lo; i < r.hi; ++i) {
-        const float4 x = ldf4(h, i * 16 + l);
+    constexpr int kBatch = 4;                             // rows in flight; past the range they add +0
+    const int h0 = threadIdx.x >> 4;                      // block-uniform trips: the shuffles need both halves
+    for (int64_t i0 = r.lo - h0; i0 < r.hi; i0 += kBatch * kSumParts) {
+        float4 x[kBatch];
+        float c[kBatch];
 #pragma unroll
-        for (int o = 0; o < O; ++o) a[o] = add4(a[o], mul4(__ldg(dOut + i * O + o), x));
-        if (l < O) ao = __fadd_rn(ao, __ldg(dOut + i * O + l));
+        for (int u = 0; u < kBatch; ++u) {
+            const int64_t i = i0 + h0 + u * kSumParts;
+            x[u] = i < r.hi ? ldf4(h, i * 16 + l) : f4(0.f);
+            c[u] = i < r.hi && l < O ? __ldg(dOut + i * O + l) : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+#pragma unroll
+            for (int o = 0; o < O; ++o)
+                a[o] = add4(a[o], mul4(__shfl_sync(0xffffffffu, c[u], (threadIdx.x & 16) | o), x[u]));
+            ao = __fadd_rn(ao, c[u]);
+        }
     }
 #pragma unroll
     for (int o = 0; o < O; ++o) put_delta(dec + (int64_t)o * kSumSet, a[o], s0[o], smem);
@@ -1493,12 +1525,23 @@ __global__ void __launch_bounds__(kSumThreads, 2) k_back_bias(const float* __res
                                                            int N, float* __restrict__ bias) {
     __shared__ __align__(16) float smem[kSumParts][kLayerW];
     const int l = threadIdx.x & 15;
-    const float4 s0 = get_prefix(bias, smem);
-    float4 a = s0;
+    float4 s0[1];
+    get_prefix<1>(bias, s0, smem);
+    float4 a = s0[0];
     const Rows r = part_rows(N);
-#pragma unroll 4
-    for (int64_t i = r.lo; i < r.hi; ++i) a = add4(a, silu_grad4(ldf4(dh, i * 16 + l), ldf4(Z, i * 16 + l)));
-    put_delta(bias, a, s0, smem);
+    constexpr int kBatch = 4;                             // rows in flight; past the range they add +0
+    for (int64_t i0 = r.lo; i0 < r.hi; i0 += kBatch * kSumParts) {
+        float4 d[kBatch], z[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+            const int64_t i = i0 + u * kSumParts;
+            d[u] = i < r.hi ? ldf4(dh, i * 16 + l) : f4(0.f);
+            z[u] = i < r.hi ? ldf4(Z, i * 16 + l) : f4(0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) a = add4(a, silu_grad4(d[u], z[u]));
+    }
+    put_delta(bias, a, s0[0], smem);
 }
 
 // dh = dh_in + dA[:, :64] + sum_{j in nbr} dA[j][64:], in that order; dZ = dh SiLU'(Z) with the first
@@ -1511,7 +1554,9 @@ __global__ void __launch_bounds__(kSumThreads, 2) k_back_gather(
     __nv_bfloat16* __restrict__ dZ, float* __restrict__ bias) {
     __shared__ __align__(16) float smem[kSumParts][kLayerW], s_start[kSumParts][kLayerW];
     const int l = threadIdx.x & 15;
-    float4 a = get_prefix(bias_in, smem), ab = f4(0.f);
+    float4 s0[1], ab = f4(0.f);
+    get_prefix<1>(bias_in, s0, smem);
+    float4 a = s0[0];
     float4* start = reinterpret_cast<float4*>(s_start[threadIdx.x >> 4]) + l;   // this thread's own, out of the registers
     *start = a;
     const Rows r = part_rows(N);
@@ -1521,13 +1566,13 @@ __global__ void __launch_bounds__(kSumThreads, 2) k_back_gather(
         for (int q = 0; q < KM; ++q) next[q] = q < KN && i < r.hi ? __ldg(nbr + i * KN + q) : -1;
     };
     fetch(r.lo);
-    for (int64_t i = r.lo; i < r.hi; ++i) {
+    for (int64_t i = r.lo; i < r.hi; i += kSumParts) {
         float4 nb[KM];
 #pragma unroll
         for (int q = 0; q < KM; ++q) nb[q] = next[q] >= 0 ? ldf4(dA, (int64_t)next[q] * 32 + 16 + l) : f4(0.f);
         const float4 own = ldf4(dA, i * 32 + l), up = ldf4(dh_in, i * 16 + l);
         const float4 zi = ldf4(Z_in, i * 16 + l), z = ldf4(Z, i * 16 + l);
-        fetch(i + 1);
+        fetch(i + kSumParts);
         a = add4(a, silu_grad4(up, zi));
         float4 v = add4(own, up);
 #pragma unroll

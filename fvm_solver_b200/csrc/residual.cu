@@ -1,7 +1,8 @@
 // Fused finite-volume residual and explicit time-stepping kernels.
 //
 // One residual evaluation (FVMEquation.forward, time_fvm/fvm_equation.py:406-435) is three
-// kernels (four with boundaries) instead of the reference's ~60 eager PyTorch ops:
+// kernels instead of the reference's ~60 eager PyTorch ops (boundary values in the cell kernel's launch,
+// k_cell_bc; a kernel of their own for parts, sub-ranges and widened stencils):
 //
 //   k_bc        boundary facets: A_bc U + b_bc + A_corr grads_prev, then the characteristic BC
 //               (facet_boundary.py:124-168, 418-512).  Each block recomputes the group mean of the

@@ -416,7 +416,7 @@ int fvm_corrector_propose(const float *state, const float *base, const float *ou
  *   fvm_back_gather:  dh = dh_in + dA[:, :64] + sum_{j in nbr(i)} dA[j][64:]; dZ = dh SiLU'(Z) with the first
  *                     pass of bias; second pass of bias_in (dh_in, Z_in).  dh must not alias dh_in.
  *   fvm_back_bias:    second pass of bias alone (dh, Z) */
-#define FVM_BACK_SET ((296 * 24 + 2 * 296) * 64)
+#define FVM_BACK_SET (2 * 296 * 64)
 int fvm_back_top(const float *h, const float *Wo, const float *dOut, const float *Z, int32_t N, int32_t O, float *dh,
                  void *dZ, float *dec, float *bias, void *stream);
 int fvm_back_decoder(const float *h, const float *dOut, int32_t N, int32_t O, float *dec, void *stream);
