@@ -117,6 +117,8 @@ _SIGS = [
     ("fvm_decoder_f32", ct.c_int, [_P, _P, _P, ct.c_int32, ct.c_int32, _P, _P]),
     ("fvm_decoder_back_f32", ct.c_int, [_P, _P, _P, ct.c_int32, ct.c_int32, _P, _P, _P, _P]),
     ("fvm_mse", ct.c_int, [_P, _P, ct.c_int64, _P, _P, _P]),
+    ("fvm_adam_many", ct.c_int, [ct.c_int32, _P, _P, _P, _P, _P, ct.c_float, ct.c_float, ct.c_float, ct.c_float,
+                                 ct.c_int32, _P, _P, _P, _P, _P]),
     ("fvm_adam", ct.c_int, [_P, _P, _P, _P, ct.c_int64, ct.c_float, ct.c_float, ct.c_float, ct.c_float,
                             ct.c_int32, _P, _P, ct.c_int32, ct.c_int32, _P]),
     ("fvm_corrector_features", ct.c_int, [_P, ct.c_int32, ct.c_int32, _P, _P, _P, ct.c_int32, _P, ct.c_int32, _P]),

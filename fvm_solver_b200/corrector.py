@@ -271,14 +271,18 @@ class CorrectorNet:
 
     def adam(self, beta1=0.9, beta2=0.999, eps=1e-8):
         self.step_count += 1
-        s = _lib.stream_ptr()
-        for k, prm in self.params.items():
-            pb = self.bf.get(k)
-            pbT = self.bfT.get(k)
-            rows, cols = (prm.shape[0], prm.shape[1]) if prm.ndim == 2 else (1, prm.shape[0])
-            _lib.check(self.lib.fvm_adam(prm.data_ptr(), self.grads[k].data_ptr(), self.m[k].data_ptr(),
-                                         self.v[k].data_ptr(), prm.numel(), self.lr, beta1, beta2, eps,
-                                         self.step_count, _lib.ptr(pb), _lib.ptr(pbT), rows, cols, s), "fvm_adam")
+        names = list(self.params)
+        at = lambda d: [d[k].data_ptr() if k in d else None for k in names]
+        p, g, m, v, pb, pbT = (at(d) for d in (self.params, self.grads, self.m, self.v, self.bf, self.bfT))
+        n = [t.numel() for t in self.params.values()]
+        cols = [t.shape[-1] for t in self.params.values()]
+        for q in range(0, len(names), 32):             # one launch for up to 32 tensors
+            c = len(names[q:q + 32])
+            P = lambda x: (ct.c_void_p * c)(*x[q:q + c])
+            I = lambda x: (ct.c_int32 * c)(*x[q:q + c])
+            _lib.check(self.lib.fvm_adam_many(
+                c, P(p), P(g), P(m), P(v), (ct.c_int64 * c)(*n[q:q + c]), self.lr, beta1, beta2, eps, self.step_count,
+                P(pb), P(pbT), I([a // b for a, b in zip(n, cols)]), I(cols), _lib.stream_ptr()), "fvm_adam_many")
 
     def state_dict(self) -> dict:
         """FP32 master weights and the layer count (the Adam moments are not kept)."""

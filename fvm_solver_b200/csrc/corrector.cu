@@ -441,23 +441,34 @@ __global__ void k_mse(const float* __restrict__ pred, const float* __restrict__ 
 
 // Adam (decoupled bias correction) on fp32 master weights; refreshes the bf16 copy [rows][cols]
 // and, if requested, its transpose [cols][rows] used by the backward GEMMs.  Zeroes the gradient.
-__global__ void k_adam(float* __restrict__ p, float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                       int64_t n, float lr, float b1, float b2, float eps, float c1, float c2,
-                       __nv_bfloat16* __restrict__ pb, __nv_bfloat16* __restrict__ pbT, int rows, int cols) {
+// blockIdx.y is the tensor: the network's dozen tensors of 4 to 8192 entries are bound by their launches
+// (12 x 2.4 us one by one), so all of them go in one.
+constexpr int kAdamMany = 32;
+struct AdamTensor {
+    float *p, *g, *m, *v;
+    __nv_bfloat16 *pb, *pbT;
+    int64_t n;
+    int rows, cols;
+};
+struct AdamArgs {
+    AdamTensor t[kAdamMany];
+};
+__global__ void k_adam(const __grid_constant__ AdamArgs args, float lr, float b1, float b2, float eps, float c1, float c2) {
+    const AdamTensor& a = args.t[blockIdx.y];
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const float gr = g[t];
-    const float mt = b1 * m[t] + (1.f - b1) * gr;
-    const float vt = b2 * v[t] + (1.f - b2) * gr * gr;
-    m[t] = mt;
-    v[t] = vt;
-    const float w = p[t] - lr * (mt / c1) / (sqrtf(vt / c2) + eps);
-    p[t] = w;
-    g[t] = 0.f;
-    if (pb) pb[t] = __float2bfloat16(w);
-    if (pbT) {
-        const int r = (int)(t / cols), c = (int)(t % cols);
-        pbT[(int64_t)c * rows + r] = __float2bfloat16(w);
+    if (t >= a.n) return;
+    const float gr = a.g[t];
+    const float mt = b1 * a.m[t] + (1.f - b1) * gr;
+    const float vt = b2 * a.v[t] + (1.f - b2) * gr * gr;
+    a.m[t] = mt;
+    a.v[t] = vt;
+    const float w = a.p[t] - lr * (mt / c1) / (sqrtf(vt / c2) + eps);
+    a.p[t] = w;
+    a.g[t] = 0.f;
+    if (a.pb) a.pb[t] = __float2bfloat16(w);
+    if (a.pbT) {
+        const int r = (int)(t / a.cols), c = (int)(t % a.cols);
+        a.pbT[(int64_t)c * a.rows + r] = __float2bfloat16(w);
     }
 }
 
@@ -611,15 +622,30 @@ extern "C" int fvm_mse(const float* pred, const float* tgt, int64_t n_elem, doub
     return launch_status();
 }
 
-extern "C" int fvm_adam(float* p, float* g, float* m, float* v, int64_t n, float lr, float beta1, float beta2,
-                        float eps, int32_t step, void* pb, void* pbT, int32_t rows, int32_t cols, void* stream) {
-    if (!p || !g || !m || !v || n <= 0 || step < 1 || (pbT && (int64_t)rows * cols != n)) return FVM_E_ARG;
+extern "C" int fvm_adam_many(int32_t count, float* const* p, float* const* g, float* const* m, float* const* v,
+                             const int64_t* n, float lr, float beta1, float beta2, float eps, int32_t step,
+                             void* const* pb, void* const* pbT, const int32_t* rows, const int32_t* cols, void* stream) {
+    if (count < 1 || count > corr::kAdamMany || !p || !g || !m || !v || !n || !pb || !pbT || !rows || !cols || step < 1)
+        return FVM_E_ARG;
+    corr::AdamArgs a{};
+    int64_t most = 0;
+    for (int q = 0; q < count; ++q) {
+        if (!p[q] || !g[q] || !m[q] || !v[q] || n[q] <= 0 || (pbT[q] && (int64_t)rows[q] * cols[q] != n[q]))
+            return FVM_E_ARG;
+        a.t[q] = corr::AdamTensor{p[q], g[q], m[q], v[q], static_cast<__nv_bfloat16*>(pb[q]),
+                                  static_cast<__nv_bfloat16*>(pbT[q]), n[q], rows[q], cols[q]};
+        most = std::max(most, n[q]);
+    }
     const float c1 = 1.f - powf(beta1, (float)step), c2 = 1.f - powf(beta2, (float)step);
     cudaStream_t s = (cudaStream_t)stream;
-    FVM_LAUNCH(KID_CORRECTOR, s, corr::k_adam<<<corr::nblk(n, 256), 256, 0, s>>>(
-                                     p, g, m, v, n, lr, beta1, beta2, eps, c1, c2, static_cast<__nv_bfloat16*>(pb),
-                                     static_cast<__nv_bfloat16*>(pbT), rows, cols));
+    FVM_LAUNCH(KID_CORRECTOR, s, corr::k_adam<<<dim3(corr::nblk(most, 256), (unsigned)count), 256, 0, s>>>(
+                                     a, lr, beta1, beta2, eps, c1, c2));
     return launch_status();
+}
+
+extern "C" int fvm_adam(float* p, float* g, float* m, float* v, int64_t n, float lr, float beta1, float beta2, float eps,
+                        int32_t step, void* pb, void* pbT, int32_t rows, int32_t cols, void* stream) {
+    return fvm_adam_many(1, &p, &g, &m, &v, &n, lr, beta1, beta2, eps, step, &pb, &pbT, &rows, &cols, stream);
 }
 
 extern "C" int fvm_corrector_features(const float* state, int32_t N, int32_t C, const float* mean,

@@ -447,6 +447,11 @@ int fvm_mse(const float *pred, const float *tgt, int64_t n_elem, double *loss, f
  * Refreshes the bf16 copy pb (if not NULL) and its [cols][rows] transpose pbT (if not NULL). */
 int fvm_adam(float *p, float *g, float *m, float *v, int64_t n, float lr, float beta1, float beta2, float eps,
              int32_t step, void *pb, void *pbT, int32_t rows, int32_t cols, void *stream);
+/* fvm_adam on `count` (at most 32) tensors in one launch: host arrays of the per-tensor arguments (their
+ * entries as in fvm_adam; pb[q], pbT[q] may be NULL). */
+int fvm_adam_many(int32_t count, float *const *p, float *const *g, float *const *m, float *const *v, const int64_t *n,
+                  float lr, float beta1, float beta2, float eps, int32_t step, void *const *pb, void *const *pbT,
+                  const int32_t *rows, const int32_t *cols, void *stream);
 /* X[i] = [(U_i - mean) * inv_std (C values), geo[i] (G values), zeros] as bf16 [N][XW]. */
 int fvm_corrector_features(const float *state, int32_t N, int32_t C, const float *mean, const float *inv_std,
                            const float *geo, int32_t G, void *X, int32_t XW, void *stream);

@@ -154,3 +154,32 @@ def test_inputs_in_the_input_layer_and_proposal(N, C, G, cases):
     _lib.check(lib.fvm_corrector_combine(P(U), P(base), P(out), P(scale), P(shift), P(cc), N, C, P(a), s), "combine")
     _lib.check(lib.fvm_corrector_propose(P(U), P(base), P(out), P(scale), P(sums), P(vol), C - 2, P(cc), N, C, P(b), s), "propose")
     assert torch.equal(a, b)
+
+
+def test_adam_many():
+    """fvm_adam_many on tensors of different sizes against fvm_adam one by one: bitwise."""
+    from fvm_solver_b200 import _lib
+    lib, s = _lib.load(), _lib.stream_ptr()
+    shapes = [(4, 64), (1, 64), (64, 128), (1, 4), (64, 64), (3, 1)]
+    def tensors():
+        out = []
+        for q, (r, c) in enumerate(shapes):
+            p, g, m = (_rand(r, c, seed=3 * q + e) for e in range(3))
+            pb = torch.zeros(r, c, dtype=torch.bfloat16, device="cuda") if q % 2 == 0 else None
+            pbT = torch.zeros(c, r, dtype=torch.bfloat16, device="cuda") if q % 3 == 2 else None
+            out.append([p, g, m, m.square(), pb, pbT])
+        return out
+    P = lambda t: None if t is None else t.data_ptr()
+    want, got = tensors(), tensors()
+    for (r, c), (p, g, m, v, pb, pbT) in zip(shapes, want):
+        _lib.check(lib.fvm_adam(P(p), P(g), P(m), P(v), r * c, 1e-3, 0.9, 0.999, 1e-8, 3, P(pb), P(pbT), r, c, s), "adam")
+    n = len(shapes)
+    A = lambda e: (ct.c_void_p * n)(*[P(t[e]) for t in got])
+    sizes = (ct.c_int64 * n)(*[r * c for r, c in shapes])
+    rows, cols = (ct.c_int32 * n)(*[r for r, _ in shapes]), (ct.c_int32 * n)(*[c for _, c in shapes])
+    _lib.check(lib.fvm_adam_many(n, A(0), A(1), A(2), A(3), sizes, 1e-3, 0.9, 0.999, 1e-8, 3, A(4), A(5), rows, cols, s),
+               "adam_many")
+    for a, b in zip(want, got):
+        for x, y in zip(a, b):
+            assert x is None or torch.equal(x, y)
+    assert lib.fvm_adam_many(0, A(0), A(1), A(2), A(3), sizes, 1e-3, 0.9, 0.999, 1e-8, 3, A(4), A(5), rows, cols, s) != 0
