@@ -513,7 +513,7 @@ def ensemble_result(cases: int, steps: int, warmup: int, timed, cfl: float = ENS
 
 
 ENSEMBLE_CFL_NOTE = ("AB3 with a time step fixed at the start: CFL 0.3 keeps every case inside AB3's "
-                     "stability region for 2000 steps; see DESIGN section 5")
+                     "stability region for 2000 steps")
 
 
 def ensemble_sharded(args):
