@@ -1673,9 +1673,9 @@ __global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __grid_con
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
     uint8_t* sW = smem + kBackStages * kBackStage;
-    __shared__ __align__(8) uint64_t bar_load[kBackStages], bar_free[kBackStages], bar_full[2], bar_empty[2];
+    __shared__ __align__(8) uint64_t bar_load[kBackStages], bar_free[kBackStages], bar_full[2], bar_empty[2], bar_done;
     __shared__ uint32_t s_taddr;
-    __shared__ int s_fail, s_last;
+    __shared__ int s_fail;
     constexpr int AU = LAYER ? 16 : 8;                    // 8-channel units of an A row
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ntiles = (N + TM - 1) / TM;
@@ -1694,9 +1694,9 @@ __global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __grid_con
             mbar_init(&bar_full[b], 1);
             mbar_init(&bar_empty[b], 8);
         }
+        mbar_init(&bar_done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;");
         s_fail = 0;
-        s_last = -1;
     }
     if (LAYER) {
         for (int t = tid; t < TM * 8; t += kBackThreads)
@@ -1757,9 +1757,12 @@ __global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __grid_con
                     tc_mma(tw, make_desc_sw(sa + 2048 * q, kBackHalf), make_desc_sw(sz + 2048 * q, kBackHalf), id_w,
                            k > 0 || q > 0);
                 tc_commit(&bar_free[st]);
-                tc_commit(&bar_full[a]);
-                s_last = k;
+                if (LAYER) tc_commit(&bar_full[a]);
             }
+            // Covers every MMA issued, also when a wait gave up.  A barrier of its own, completed once: of
+            // bar_full several phases can be open where no reader follows them (the input layer), and a
+            // parity then says nothing about the last one.
+            tc_commit(&bar_done);
         }
     } else if (LAYER) {
         const int half = warp >> 2;
@@ -1812,12 +1815,12 @@ __global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __grid_con
         }
     }
     __syncthreads();
-    // wait for the last tile's commit (the MMAs of one thread complete in order)
-    bool done = true;
-    if (s_last >= 0) done = mbar_wait(&bar_full[s_last & 1], (uint32_t)((s_last >> 1) & 1));
+    // no MMA is in flight past this point (a second bounded chance before tensor memory is released)
+    const bool done = mbar_wait(&bar_done, 0u);
     if (!__syncthreads_and(done) || s_fail) {
         if (tid == 0) atomicExch(err, 1);
-    } else if (warp < 4 && s_last >= 0) {
+        if (!done) mbar_wait(&bar_done, 0u);
+    } else if (warp < 4) {
         asm volatile("tcgen05.fence::after_thread_sync;");
         uint32_t v[32];
         const int in = 32 * warp + lane;                  // input channel

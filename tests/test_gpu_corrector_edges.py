@@ -1,0 +1,40 @@
+"""Corrector kernels and entry points at the edges of what they take.  Needs a B200."""
+import ctypes as ct
+
+import pytest
+import torch
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _cuda():
+    if not torch.cuda.is_available():
+        pytest.skip("needs CUDA")
+
+
+def _rand(*shape, seed, scale=1.0):
+    return scale * torch.randn(*shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(seed))
+
+
+@pytest.mark.parametrize("tiles", [1, 2, 3, 4, 5, 6])
+def test_input_layer_gradient_waits_for_its_products(tiles):
+    """The input layer's dW = dZ^T X with 1 to 6 tiles of 128 rows per CTA (no reader follows the tiles'
+    barriers there), many launches in a row.  Products of bf16 values are exact in fp32 and summed in
+    fp32: rel-L2 <= 1e-5 against FP64, as for the other sizes of this kernel."""
+    from fvm_solver_b200 import _lib
+    lib, s = _lib.load(), _lib.stream_ptr()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    N = 128 * (sms * tiles) - 5
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    dZ, X = _rand(N, 64, seed=tiles).bfloat16(), _rand(N, 64, seed=10 + tiles).bfloat16()
+    dW = torch.zeros(24, 64, 64, device="cuda")
+    for q in range(24):
+        _lib.check(lib.fvm_back_layer(dZ.data_ptr(), X.data_ptr(), None, None, 0, N, None, dW[q].data_ptr(),
+                                      err.data_ptr(), s), "fvm_back_layer")
+    want = (dZ.double().t() @ X.double()).cpu().numpy()
+    assert int(err.item()) == 0
+    for q in range(24):
+        assert rel_l2(dW[q].double().cpu().numpy(), want) < 1e-5
