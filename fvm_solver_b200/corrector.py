@@ -403,16 +403,16 @@ class CorrectorModel:
     def predict(self, state: torch.Tensor, out_state: torch.Tensor, r0: torch.Tensor):
         """out_state = proposal for U_{t+k} from state = U_t with residual r0 = dU/dt(U_t).
 
-        The input features are formed inside the input layer (the network's X buffer, which training
-        reads, is left alone), and the offsets that remove the volume-weighted mean of the mass and
+        The input features are formed inside the input layer, which also leaves them in the network's X
+        buffer (what ``forward`` and ``train_step`` read), and the offsets that remove the volume-weighted mean of the mass and
         energy parts of scale * out inside the kernel that adds the proposal up."""
         net, b, N = self.net, self.batch, state.shape[0]
         lib, s, bufs = net.lib, _lib.stream_ptr(), net._alloc(state.shape[0])
-        _lib.check(lib.fvm_corrector_in_layer(
+        _lib.check(lib.fvm_corrector_in_layer_keep(
             state.data_ptr(), r0.data_ptr(), b.t_solver.dt.data_ptr(), self.k, self.cell_case32.data_ptr(), N, self.C,
             self.fmean.data_ptr(), self.finv.data_ptr(), self.geo.data_ptr(), self.geo.shape[1], self.base.data_ptr(),
-            net.bf["W_in"].data_ptr(), net.params["b_in"].data_ptr(), bufs["hf"][0].data_ptr(), net.err.data_ptr(), s),
-            "fvm_corrector_in_layer")
+            bufs["X"].data_ptr(), net.bf["W_in"].data_ptr(), net.params["b_in"].data_ptr(), bufs["hf"][0].data_ptr(),
+            net.err.data_ptr(), s), "fvm_corrector_in_layer_keep")
         out = net._layers(self.nbr, store_pre=False)
         _lib.check(lib.fvm_conservation(ct.byref(b.dev.struct), out.data_ptr(), self.S.data_ptr(),
                                         ct.byref(b.work.struct), s), "fvm_conservation")

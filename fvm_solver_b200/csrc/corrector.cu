@@ -757,6 +757,7 @@ struct LayerArgs {
     const float *state, *r0, *dt, *mean, *inv_std, *geo;   // the features of fvm_corrector_inputs, built
     const int32_t* cell_case;                              // here (C, G columns; base [M][C] is stored)
     float* base;
+    __nv_bfloat16* Xout;         // the feature rows formed here, [M][64], or null
     int C, G;
     float k;
     int M, KN;
@@ -1017,6 +1018,14 @@ __global__ void __launch_bounds__(kLayerThreads, layer_ctas(INPUT)) k_mp_layer(L
                        make_desc(smem_u32(sW) + 2 * q * kLayerWUnit, kLayerWUnit, 128), idesc, q > 0);
             tc_commit(&bar);
         }
+        if (INPUT && g.Xout)   // features formed here, out of the operand tile while the products run
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int r = r0 + 32 * q;
+                if (m0 + r < g.M)
+                    *reinterpret_cast<uint4*>(g.Xout + (int64_t)(m0 + r) * kLayerW + 8 * u) =
+                        *reinterpret_cast<const uint4*>(sA + u * kUnitBytes + r * 16);
+            }
         if (!__syncthreads_and(mbar_wait(&bar, (uint32_t)(k & 1)))) {
             ok = false;
             break;
@@ -1260,14 +1269,15 @@ extern "C" int fvm_in_layer(const void* X, int32_t M, const void* Wt, const floa
     return corr::launch_layer<true>(g, (cudaStream_t)stream);
 }
 
-extern "C" int fvm_corrector_in_layer(const float* state, const float* r0, const float* dt, int32_t k,
-                                      const int32_t* cell_case, int32_t N, int32_t C, const float* mean,
-                                      const float* inv_std, const float* geo, int32_t G, float* base, const void* Wt,
-                                      const float* bias, float* h_out, int32_t* err, void* stream) {
+extern "C" int fvm_corrector_in_layer_keep(const float* state, const float* r0, const float* dt, int32_t k,
+                                           const int32_t* cell_case, int32_t N, int32_t C, const float* mean,
+                                           const float* inv_std, const float* geo, int32_t G, float* base, void* X,
+                                           const void* Wt, const float* bias, float* h_out, int32_t* err,
+                                           void* stream) {
     if (!state || !r0 || !dt || !mean || !inv_std || (G > 0 && !geo) || !base || !Wt || !bias || !h_out || !err ||
         N <= 0 || G < 0 || k < 1 || (C != 4 && C != 5) || 2 * C + G > corr::kLayerW)
         return FVM_E_ARG;
-    if (((uintptr_t)h_out & 31u) || (uintptr_t)Wt % 16) return FVM_E_ARG;
+    if (((uintptr_t)h_out & 31u) || (uintptr_t)Wt % 16 || (uintptr_t)X % 16) return FVM_E_ARG;
     if (C == 4 && (((uintptr_t)state | (uintptr_t)r0 | (uintptr_t)base) & 15u)) return FVM_E_ARG;   // 128-bit rows
     corr::LayerArgs g{};
     g.M = N;
@@ -1279,6 +1289,7 @@ extern "C" int fvm_corrector_in_layer(const float* state, const float* r0, const
     g.geo = geo;
     g.cell_case = cell_case;
     g.base = base;
+    g.Xout = static_cast<__nv_bfloat16*>(X);
     g.C = C;
     g.G = G;
     g.k = (float)k;
@@ -1287,6 +1298,14 @@ extern "C" int fvm_corrector_in_layer(const float* state, const float* r0, const
     g.h_out = h_out;
     g.err = err;
     return corr::launch_layer<true>(g, (cudaStream_t)stream);
+}
+
+extern "C" int fvm_corrector_in_layer(const float* state, const float* r0, const float* dt, int32_t k,
+                                      const int32_t* cell_case, int32_t N, int32_t C, const float* mean,
+                                      const float* inv_std, const float* geo, int32_t G, float* base, const void* Wt,
+                                      const float* bias, float* h_out, int32_t* err, void* stream) {
+    return fvm_corrector_in_layer_keep(state, r0, dt, k, cell_case, N, C, mean, inv_std, geo, G, base, nullptr, Wt, bias,
+                                       h_out, err, stream);
 }
 
 extern "C" int fvm_mp_gather_f32(const float* h, const int32_t* nbr, int32_t N, int32_t KN, void* out, void* stream) {

@@ -396,6 +396,11 @@ int fvm_in_layer(const void *X, int32_t M, const void *Wt, const float *bias, fl
 int fvm_corrector_in_layer(const float *state, const float *r0, const float *dt, int32_t k, const int32_t *cell_case,
                            int32_t N, int32_t C, const float *mean, const float *inv_std, const float *geo, int32_t G,
                            float *base, const void *Wt, const float *bias, float *h_out, int32_t *err, void *stream);
+/* The same, also keeping the feature rows X (bf16 [N][64], 16-byte aligned, or NULL). */
+int fvm_corrector_in_layer_keep(const float *state, const float *r0, const float *dt, int32_t k,
+                                const int32_t *cell_case, int32_t N, int32_t C, const float *mean,
+                                const float *inv_std, const float *geo, int32_t G, float *base, void *X,
+                                const void *Wt, const float *bias, float *h_out, int32_t *err, void *stream);
 /* prop = state + base + scale[c] * out - shift, where the components c >= first lose their case's
  * volume-weighted mean of scale * out: shift = (float)(sums[case][c] / case_vol[case] * scale[c]) with
  * sums = fvm_conservation(out) (FP64), and 0 below.  C = 4 (rows 16-byte aligned) or 5. */

@@ -1,6 +1,7 @@
 """Corrector kernels and entry points at the edges of what they take.  Needs a B200."""
 import ctypes as ct
 
+import numpy as np
 import pytest
 import torch
 
@@ -38,3 +39,42 @@ def test_input_layer_gradient_waits_for_its_products(tiles):
     assert int(err.item()) == 0
     for q in range(24):
         assert rel_l2(dW[q].double().cpu().numpy(), want) < 1e-5
+
+
+@pytest.fixture(scope="module")
+def batch():
+    if not torch.cuda.is_available():
+        pytest.skip("needs CUDA")
+    from fvm_solver_b200 import batched as B, workloads as W
+    cases, params = [], []
+    for i, n in enumerate([1500, 2011]):
+        p = W.ensemble_params(i)
+        p["n_cells"] = n
+        c = W.channel_cylinder(device="cuda", solver_name="Butcher", solver_extra="SSP_RK3", **p)
+        c.cfg.cfl = None
+        cases.append(c)
+        params.append([p["mach"], np.log10(p["reynolds"])])
+    b = B.BatchedFVM([B.build_case_tables(c) for c in cases], cases[0].cfg, device="cuda")
+    b.t_solver.update_cfl_dt(0.5)
+    return b, torch.tensor(params, dtype=torch.float32)
+
+
+def _model(batch):
+    """(model, state, residual) on the batch, normalised."""
+    from fvm_solver_b200.corrector import CorrectorModel
+    b, params = batch
+    m = CorrectorModel(b, params, seed=3)
+    U = b.cells.state.clone()
+    r0 = m.res(U, torch.empty_like(U))
+    m.set_normalisation(torch.cat([U, U * 1e-3], 1).unsqueeze(0), (U * 1e-3 + 1e-3).unsqueeze(0))
+    return m, U, r0
+
+
+def test_proposal_leaves_its_features_to_the_network(batch):
+    """After ``predict`` the network's input rows are those of its state, as after ``inputs`` (bitwise)."""
+    m, U, r0 = _model(batch)
+    m.inputs(U * 1.01, r0)
+    m.predict(U, torch.empty_like(U), r0)
+    out, X = m.net._bufs["out"].clone(), m.net._bufs["X"].clone()
+    assert torch.equal(m.net.forward(m.nbr), out)
+    assert torch.equal(m.inputs(U, r0), X)
