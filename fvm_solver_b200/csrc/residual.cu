@@ -649,8 +649,8 @@ __device__ __forceinline__ void cell_body(const fvm_mesh_t& m, const Phys& p, co
 // boundary facet, evaluates all of the cell's boundary values (stored for the facet kernel) and its
 // limited gradient.  One thread owns a cell, so the previous gradient is read before it is replaced;
 // the flag that says whether there is one is set by the facet kernel.  Every block forms the
-// characteristic scale 10 / mean(c) itself, per case in a batched mesh.
-template <int DIM, bool TILED>
+// characteristic scale 10 / mean(c) itself, per case in a batched mesh (BATCH).
+template <int DIM, bool TILED, bool BATCH>
 __device__ __forceinline__ void boundary_cells(const fvm_mesh_t& m, const Phys& p, const float* __restrict__ prims,
                                                float* __restrict__ bcv, float* __restrict__ grads,
                                                const int32_t* __restrict__ has_grads, float* __restrict__ copy) {
@@ -667,20 +667,37 @@ __device__ __forceinline__ void boundary_cells(const fvm_mesh_t& m, const Phys& 
 #pragma unroll
     for (int k = 0; k < KG; ++k) first = cols[k] >= N ? min(first, cols[k]) : first;
     const bool live = in && first == N + b && (m.case_active == nullptr || case_on(m, m.bc_case, b));
-    const int cse = in && m.n_cases > 0 ? __ldg(m.bc_case + b) : 0;
     float scale = 0.f;
-    if (m.n_char > 0) {   // block-uniform bounds: the cases of the block's facets are one range
-        const int last_b = min((int)((blockIdx.x + 1) * blockDim.x), m.n_bc) - 1;
-        const int c0 = m.n_cases > 0 ? __ldg(m.bc_case + blockIdx.x * blockDim.x) : 0;
-        const int c1 = m.n_cases > 0 ? __ldg(m.bc_case + last_b) : 0;
-        for (int c = c0; c <= c1; ++c) {
-            const int lo = m.n_cases > 0 ? __ldg(m.ch_off + c) : 0, hi = m.n_cases > 0 ? __ldg(m.ch_off + c + 1) : m.n_char;
-            if (hi <= lo || (m.case_active && !m.case_active[c])) continue;
+    if (m.n_char > 0) {
+        auto mean = [&](int lo, int hi) {                // block-wide; scale of facets [lo, hi) in s_scale
             const double sum = char_c_sum<DIM, false>(m, p, prims, lo, hi, red);
             if (threadIdx.x == 0) s_scale = 10.0f / (float)(sum / (double)(hi - lo));
             __syncthreads();
-            if (c == cse) scale = s_scale;
+        };
+        if constexpr (!BATCH) {
+            mean(0, m.n_char);
+            scale = s_scale;
+        } else {
+            // The lowest to the highest case of the block's facets, in whatever order these are; of a wider
+            // range those that are there.  All bounds are the same for the whole block.
+            __shared__ int s_lo, s_hi;
+            const int cse = in ? __ldg(m.bc_case + b) : -1;
+            if (threadIdx.x == 0) s_lo = INT_MAX, s_hi = -1;
             __syncthreads();
+            if (in) {
+                atomicMin(&s_lo, cse);
+                atomicMax(&s_hi, cse);
+            }
+            __syncthreads();
+            const int c0 = s_lo, c1 = s_hi;
+            for (int c = c0; c <= c1; ++c) {
+                if (c1 - c0 > 1 && !__syncthreads_or(cse == c)) continue;
+                const int lo = __ldg(m.ch_off + c), hi = __ldg(m.ch_off + c + 1);
+                if (hi <= lo || (m.case_active && !m.case_active[c])) continue;
+                mean(lo, hi);
+                if (c == cse) scale = s_scale;
+                __syncthreads();
+            }
         }
     }
     if (!live) return;
@@ -832,13 +849,13 @@ __global__ void __maxnreg__(FVM_CELL_MAXNREG) k_cell(fvm_mesh_t m, Phys p, const
 // with their boundary values, the others the inner cells, which wait for nothing.  A boundary kernel
 // of its own put its launch and the serial characteristic sum in front of every stage (4.1 of 12.8 us
 // per stage of an 11 k-cell channel, 13 of 44 us per residual of a 120 k-cell sphere).
-template <int DIM, bool TILED>
+template <int DIM, bool TILED, bool BATCH>
 __global__ void __maxnreg__(FVM_CELL_MAXNREG) k_cell_bc(fvm_mesh_t m, Phys p, const float* __restrict__ prims,
                                                      float* __restrict__ bcv, float* __restrict__ grads,
                                                      const int32_t* __restrict__ has_grads, int waves, int nb,
                                                      float* __restrict__ copy) {
     dependency_wait();
-    if ((int)blockIdx.x < nb) boundary_cells<DIM, TILED>(m, p, prims, bcv, grads, has_grads, copy);
+    if ((int)blockIdx.x < nb) boundary_cells<DIM, TILED, BATCH>(m, p, prims, bcv, grads, has_grads, copy);
     else cell_body<DIM, false, TILED, true>(m, p, prims, bcv, grads, nullptr, waves, blockIdx.x - nb, gridDim.x - nb, copy);
 }
 
@@ -2087,8 +2104,13 @@ static int launch_begin(const fvm_mesh_t* m, const Phys& p, const float* prims, 
             FVM_LAUNCH(KID_CELL, s, launch(kernel, dim3(nb + gc), dim3(g_block_cell), 0, s, *m, p, prims, w->bc_vals, grads,
                                            has_grads, waves_of(g_pf_cell), (int)nb, copy));
         };
-        if (cell_tiled(m)) cells(k_cell_bc<DIM, true>);
-        else cells(k_cell_bc<DIM, false>);
+        auto form = [&](auto batch) {
+            constexpr bool B = decltype(batch)::value;
+            if (cell_tiled(m)) cells(k_cell_bc<DIM, true, B>);
+            else cells(k_cell_bc<DIM, false, B>);
+        };
+        if (m->n_cases > 0) form(std::true_type{});
+        else form(std::false_type{});
         return launch_status();
     }
     if (m->n_bc > 0) {
