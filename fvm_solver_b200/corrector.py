@@ -210,6 +210,9 @@ class CorrectorNet:
         p, s = self.params, _lib.stream_ptr()
         err = self.err.data_ptr()
         Z = [z.data_ptr() for z in b["Z"]] if store_pre else [None] * (L + 1)
+        if L == 0:                                       # no layer whose kernel would form the outputs
+            _lib.check(self.lib.fvm_decoder_f32(b["hf"][0].data_ptr(), p["W_out"].data_ptr(), p["b_out"].data_ptr(), N,
+                                                self.O, b["out"].data_ptr(), s), "fvm_decoder_f32")
         for l in range(L):
             last = l == L - 1
             keep = store_pre or not last

@@ -78,3 +78,22 @@ def test_proposal_leaves_its_features_to_the_network(batch):
     out, X = m.net._bufs["out"].clone(), m.net._bufs["X"].clone()
     assert torch.equal(m.net.forward(m.nbr), out)
     assert torch.equal(m.inputs(U, r0), X)
+
+
+def test_network_without_layers():
+    """layers=0: the decoder reads the input layer's activations.  The bf16 products are exact in fp32 and
+    summed in fp32, SiLU by the fast exponential: rel-L2 <= 1e-5 of FP64."""
+    from fvm_solver_b200.corrector import CorrectorNet
+    N = 300
+    net = CorrectorNet(3, layers=0, seed=1, lr=1e-2)
+    X = net._alloc(N)["X"]
+    X[:N].copy_(_rand(N, 64, seed=2))
+    nbr = torch.full((N, 3), -1, dtype=torch.int32, device="cuda")
+    h = torch.nn.functional.silu(X[:N].double() @ net.bf["W_in"].double().t() + net.params["b_in"].double())
+    want = h @ net.params["W_out"].double().t() + net.params["b_out"].double()
+    for store_pre in (False, True):
+        net._bufs["out"].zero_()
+        out = net.forward(nbr, store_pre=store_pre)
+        assert rel_l2(out.double().cpu().numpy(), want.cpu().numpy()) < 1e-5
+    assert float(net.train_step(nbr, want.float() + 1.0)) == pytest.approx(1.0, rel=1e-4)
+    assert float(net.params["b_out"].abs().min()) > 0
