@@ -1426,12 +1426,14 @@ __device__ __forceinline__ void get_prefix(const float* set, float4 (&out)[S], f
         out[o] = t;
     }
 }
-// Second pass: what this half-warp's accumulator gained (exact) -> the block's increment; block-wide call.
+// What an accumulator gained; an infinity it started from is an earlier block's, which counted it.
+__device__ __forceinline__ float gain(float acc, float start) { return acc == start ? 0.f : acc - start; }
+// Second pass: what this half-warp's accumulator gained -> the block's increment; block-wide call.
 __device__ __forceinline__ void put_delta(float* set, float4 acc, float4 start, float (*smem)[kLayerW]) {
     const int h = threadIdx.x >> 4, l = threadIdx.x & 15;
     __syncthreads();
     reinterpret_cast<float4*>(smem[h])[l] =
-        make_float4(acc.x - start.x, acc.y - start.y, acc.z - start.z, acc.w - start.w);
+        make_float4(gain(acc.x, start.x), gain(acc.y, start.y), gain(acc.z, start.z), gain(acc.w, start.w));
     __syncthreads();
     if (threadIdx.x < kLayerW) {
         double t = 0.0;

@@ -97,3 +97,27 @@ def test_network_without_layers():
         assert rel_l2(out.double().cpu().numpy(), want.cpu().numpy()) < 1e-5
     assert float(net.train_step(nbr, want.float() + 1.0)) == pytest.approx(1.0, rel=1e-4)
     assert float(net.params["b_out"].abs().min()) > 0
+
+
+def test_column_sums_with_infinite_terms():
+    """A sum with an infinite term is infinite, not NaN, and the others stay finite."""
+    from fvm_solver_b200 import _lib
+    lib, s = _lib.load(), _lib.stream_ptr()
+    N, O = 5000, 4
+    P = lambda t: t.data_ptr()
+    h, Wo, dout, Z = _rand(N, 64, seed=1).abs(), _rand(O, 64, seed=2), _rand(N, O, seed=3).abs() + 0.1, _rand(N, 64, seed=4)
+    h[2000, 5] = float("inf")
+    dout[3000, 2] = float("inf")
+    sums = torch.empty((O + 2, _lib.FVM_BACK_SET), device="cuda")
+    dh, dZ = torch.empty(N, 64, device="cuda"), torch.empty(N, 64, device="cuda", dtype=torch.bfloat16)
+    _lib.check(lib.fvm_back_top(P(h), P(Wo), P(dout), P(Z), N, O, P(dh), P(dZ), P(sums[1]), P(sums[0]), s), "top")
+    _lib.check(lib.fvm_back_decoder(P(h), P(dout), N, O, P(sums[1]), s), "decoder")
+    got = torch.zeros(O + 1, 64, device="cuda")
+    n = O + 1
+    _lib.check(lib.fvm_back_finish(n, (ct.c_void_p * n)(*[P(sums[1 + q]) for q in range(n)]),
+                                   (ct.c_void_p * n)(*[P(got[q]) for q in range(n)]), (ct.c_int32 * n)(*([64] * O + [O])), s),
+               "finish")
+    want = torch.stack([(dout[:, o:o + 1].double() * h.double()).sum(0) for o in range(O)])
+    assert not got.isnan().any()
+    assert torch.equal(got[:O].isinf(), want.isinf())
+    assert torch.equal(got[O, :O].isinf(), dout.sum(0).isinf())
