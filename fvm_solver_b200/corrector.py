@@ -169,13 +169,6 @@ class CorrectorNet:
              # column-sum workspace: one set per bias gradient (input layer first), O + 1 for the decoder
              "sums": torch.zeros((L + 1 + self.O + 1, _lib.FVM_BACK_SET), device=d),
              "loss": torch.zeros(1, dtype=torch.float64, device=d)}
-        g = self.grads
-        dst = [(g["b_in"], W)] + [(g[f"b{l}"], W) for l in range(L)] + [(g["W_out"][o], W) for o in range(self.O)] + \
-            [(g["b_out"], self.O)]
-        n = len(dst)
-        b["finish"] = [(min(32, n - q), (ct.c_void_p * 32)(*[b["sums"][i].data_ptr() for i in range(q, min(q + 32, n))]),
-                        (ct.c_void_p * 32)(*[t.data_ptr() for t, _ in dst[q:q + 32]]),
-                        (ct.c_int32 * 32)(*[c for _, c in dst[q:q + 32]])) for q in range(0, n, 32)]
         self._bufs = b
         return b
 
@@ -254,8 +247,14 @@ class CorrectorNet:
         chk(lib.fvm_back_layer(ptr(b["dZ"]), ptr(b["X"]), None, None, 0, N, None, ptr(g["W_in"]), err, s),
             "fvm_back_layer")
         chk(lib.fvm_back_bias(ptr(dh), ptr(b["Z"][0]), N, ptr(bias[0]), s), "fvm_back_bias")
-        for n, sets, dst, cols in b["finish"]:
-            chk(lib.fvm_back_finish(n, sets, dst, cols, s), "fvm_back_finish")
+        dst = [(g["b_in"], W)] + [(g[f"b{l}"], W) for l in range(L)] + [(g["W_out"][o], W) for o in range(self.O)] + \
+            [(g["b_out"], self.O)]
+        n_sets = len(dst)
+        for q in range(0, n_sets, 32):                   # the gradients as they are now, set by set
+            c = min(32, n_sets - q)
+            P, I = ct.c_void_p * c, ct.c_int32 * c
+            chk(lib.fvm_back_finish(c, P(*[ptr(bias[q + i]) for i in range(c)]), P(*[ptr(t) for t, _ in dst[q:q + c]]),
+                                    I(*[w for _, w in dst[q:q + c]]), s), "fvm_back_finish")
         self.bucket.average()
         self.adam()
         return b["loss"]

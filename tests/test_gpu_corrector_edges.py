@@ -121,3 +121,22 @@ def test_column_sums_with_infinite_terms():
     assert not got.isnan().any()
     assert torch.equal(got[:O].isinf(), want.isinf())
     assert torch.equal(got[O, :O].isinf(), dout.sum(0).isinf())
+
+
+def test_gradients_go_where_grads_points():
+    """``train_step`` adds to the tensors that ``grads`` holds at the call, not to earlier ones.  The layers'
+    gradients are added up by atomics in any order: 1e-4 of each."""
+    from fvm_solver_b200.corrector import CorrectorNet
+    N = 300
+    net = CorrectorNet(3, layers=1, seed=1)
+    net._alloc(N)["X"][:N].copy_(_rand(N, 64, seed=2))
+    nbr, target = torch.full((N, 3), -1, dtype=torch.int32, device="cuda"), torch.zeros(N, 3, device="cuda")
+    net.adam = lambda: None
+    old = net.grads
+    net.train_step(nbr, target)
+    want = {k: v.clone() for k, v in old.items()}
+    net.grads = {k: torch.zeros_like(v) for k, v in old.items()}
+    net.train_step(nbr, target)
+    for k, w in want.items():
+        assert torch.equal(old[k], w), k
+        assert torch.allclose(net.grads[k], w, rtol=1e-4, atol=1e-5 * float(w.abs().max())), k
