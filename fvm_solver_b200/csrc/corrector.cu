@@ -551,6 +551,23 @@ __global__ void k_corrector_combine(const float* __restrict__ state, const float
     prop[t] = v;
 }
 
+// Rows of C floats: whole where `whole` says that they start on 16-byte boundaries, else float by float
+// (five floats always).
+template <int C>
+__device__ __forceinline__ void load_row_any(const float* p, bool whole, float (&v)[C]) {
+    if (whole) load_row<C>(p, v);
+    else
+#pragma unroll
+        for (int c = 0; c < C; ++c) v[c] = __ldg(p + c);
+}
+template <int C>
+__device__ __forceinline__ void store_row_any(float* p, bool whole, const float (&v)[C]) {
+    if (whole) store_row<C>(p, v);
+    else
+#pragma unroll
+        for (int c = 0; c < C; ++c) p[c] = v[c];
+}
+
 // The same with the shift formed from the cases' sums of vol * out: the components from `first` on lose
 // the volume-weighted mean of scale * out, (float)(sums / case_vol * scale).  One thread per cell.
 template <int C>
@@ -558,16 +575,16 @@ __global__ void __launch_bounds__(256) k_corrector_propose(const float* __restri
                                                            const float* __restrict__ out, const float* __restrict__ scale,
                                                            const double* __restrict__ sums,
                                                            const double* __restrict__ case_vol, int first,
-                                                           const int32_t* __restrict__ cell_case, int N,
+                                                           const int32_t* __restrict__ cell_case, int N, bool whole,
                                                            float* __restrict__ prop) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= N) return;
     const int cs = cell_case ? __ldg(cell_case + i) : 0;
     const double vol = __ldg(case_vol + cs);
     float u[C], b[C], o[C];
-    load_row<C>(state + (int64_t)i * C, u);
-    load_row<C>(base + (int64_t)i * C, b);
-    load_row<C>(out + (int64_t)i * C, o);
+    load_row_any<C>(state + (int64_t)i * C, whole, u);
+    load_row_any<C>(base + (int64_t)i * C, whole, b);
+    load_row_any<C>(out + (int64_t)i * C, whole, o);
 #pragma unroll
     for (int c = 0; c < C; ++c) {
         const float sc = __ldg(scale + c);
@@ -575,7 +592,7 @@ __global__ void __launch_bounds__(256) k_corrector_propose(const float* __restri
         v -= c >= first ? (float)(__ldg(sums + (int64_t)cs * C + c) / vol * (double)sc) : 0.f;
         u[c] = v;
     }
-    store_row<C>(prop + (int64_t)i * C, u);
+    store_row_any<C>(prop + (int64_t)i * C, whole, u);
 }
 
 static inline unsigned nblk(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs); }
@@ -703,15 +720,15 @@ extern "C" int fvm_corrector_propose(const float* state, const float* base, cons
                                      const int32_t* cell_case, int32_t N, int32_t C, float* prop, void* stream) {
     if (!state || !base || !out || !scale || !sums || !case_vol || !prop || N <= 0 || first < 0) return FVM_E_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    const bool rows16 = (((uintptr_t)state | (uintptr_t)base | (uintptr_t)out | (uintptr_t)prop) & 15u) == 0;
-    if (C == 4 && rows16)
+    const bool whole = (((uintptr_t)state | (uintptr_t)base | (uintptr_t)out | (uintptr_t)prop) & 15u) == 0;
+    if (C == 4)
         FVM_LAUNCH(KID_CORRECTOR, s, corr::k_corrector_propose<4><<<corr::nblk(N, 256), 256, 0, s>>>(
-                                         state, base, out, scale, sums, case_vol, first, cell_case, N, prop));
+                                         state, base, out, scale, sums, case_vol, first, cell_case, N, whole, prop));
     else if (C == 5)
         FVM_LAUNCH(KID_CORRECTOR, s, corr::k_corrector_propose<5><<<corr::nblk(N, 256), 256, 0, s>>>(
-                                         state, base, out, scale, sums, case_vol, first, cell_case, N, prop));
+                                         state, base, out, scale, sums, case_vol, first, cell_case, N, whole, prop));
     else
-        return C == 4 ? FVM_E_ARG : FVM_E_UNSUPPORTED;
+        return FVM_E_UNSUPPORTED;
     return launch_status();
 }
 
@@ -759,6 +776,7 @@ struct LayerArgs {
     float* base;
     __nv_bfloat16* Xout;         // the feature rows formed here, [M][64], or null
     int C, G;
+    bool whole;                  // rows of state, r0 and base start on 16-byte boundaries
     float k;
     int M, KN;
     const __nv_bfloat16* Wt;     // [64][128] (input layer: [64][64])
@@ -846,8 +864,8 @@ __device__ __forceinline__ void stage_features(const LayerArgs& g, uint8_t* sA, 
         float u[C], b[C], x[16];
         float h = 0.f;
         if (valid) {
-            load_row<C>(g.state + row * C, u);
-            load_row<C>(g.r0 + row * C, b);
+            load_row_any<C>(g.state + row * C, g.whole, u);
+            load_row_any<C>(g.r0 + row * C, g.whole, b);
             h = g.k * __ldg(g.dt + (g.cell_case ? __ldg(g.cell_case + row) : 0));
         }
 #pragma unroll
@@ -858,7 +876,7 @@ __device__ __forceinline__ void stage_features(const LayerArgs& g, uint8_t* sA, 
             x[c] = valid ? (u[c] - __ldg(g.mean + c)) * __ldg(g.inv_std + c) : 0.f;
             x[C + c] = valid ? (b[c] - __ldg(g.mean + C + c)) * __ldg(g.inv_std + C + c) : 0.f;
         }
-        if (valid) store_row<C>(g.base + row * C, b);
+        if (valid) store_row_any<C>(g.base + row * C, g.whole, b);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             float v[8];
@@ -1278,7 +1296,6 @@ extern "C" int fvm_corrector_in_layer_keep(const float* state, const float* r0, 
         N <= 0 || G < 0 || k < 1 || (C != 4 && C != 5) || 2 * C + G > corr::kLayerW)
         return FVM_E_ARG;
     if (((uintptr_t)h_out & 31u) || (uintptr_t)Wt % 16 || (uintptr_t)X % 16) return FVM_E_ARG;
-    if (C == 4 && (((uintptr_t)state | (uintptr_t)r0 | (uintptr_t)base) & 15u)) return FVM_E_ARG;   // 128-bit rows
     corr::LayerArgs g{};
     g.M = N;
     g.state = state;
@@ -1292,6 +1309,7 @@ extern "C" int fvm_corrector_in_layer_keep(const float* state, const float* r0, 
     g.Xout = static_cast<__nv_bfloat16*>(X);
     g.C = C;
     g.G = G;
+    g.whole = (((uintptr_t)state | (uintptr_t)r0 | (uintptr_t)base) & 15u) == 0;
     g.k = (float)k;
     g.Wt = static_cast<const __nv_bfloat16*>(Wt);
     g.bias = bias;

@@ -392,7 +392,8 @@ int fvm_in_layer(const void *X, int32_t M, const void *Wt, const float *bias, fl
                  void *stream);
 /* The input layer straight from the corrector's inputs: h_out_i = SiLU(X_i . Wt^T + bias) with the feature
  * rows X of fvm_corrector_inputs for kdt = k * dt[case], formed in the kernel; also stores base = k dt r0
- * [N][C].  C = 4 (state, r0 and base 16-byte aligned) or 5, 2C + G <= 64.  Bitwise equal to fvm_corrector_inputs + fvm_in_layer. */
+ * [N][C].  C = 4 or 5, 2C + G <= 64; C = 4 reads and writes whole rows where state, r0 and base are 16-byte
+ * aligned.  Bitwise equal to fvm_corrector_inputs + fvm_in_layer. */
 int fvm_corrector_in_layer(const float *state, const float *r0, const float *dt, int32_t k, const int32_t *cell_case,
                            int32_t N, int32_t C, const float *mean, const float *inv_std, const float *geo, int32_t G,
                            float *base, const void *Wt, const float *bias, float *h_out, int32_t *err, void *stream);
@@ -403,7 +404,7 @@ int fvm_corrector_in_layer_keep(const float *state, const float *r0, const float
                                 const void *Wt, const float *bias, float *h_out, int32_t *err, void *stream);
 /* prop = state + base + scale[c] * out - shift, where the components c >= first lose their case's
  * volume-weighted mean of scale * out: shift = (float)(sums[case][c] / case_vol[case] * scale[c]) with
- * sums = fvm_conservation(out) (FP64), and 0 below.  C = 4 (rows 16-byte aligned) or 5. */
+ * sums = fvm_conservation(out) (FP64), and 0 below.  C = 4 (whole rows where all are 16-byte aligned) or 5. */
 int fvm_corrector_propose(const float *state, const float *base, const float *out, const float *scale,
                           const double *sums, const double *case_vol, int32_t first, const int32_t *cell_case, int32_t N,
                           int32_t C, float *prop, void *stream);

@@ -140,3 +140,17 @@ def test_gradients_go_where_grads_points():
     for k, w in want.items():
         assert torch.equal(old[k], w), k
         assert torch.allclose(net.grads[k], w, rtol=1e-4, atol=1e-5 * float(w.abs().max())), k
+
+
+def test_proposal_from_and_to_any_address(batch):
+    """State, result and residual that start four bytes past a 16-byte boundary: bitwise as aligned ones."""
+    def off(t):
+        v = torch.empty(t.numel() + 4, device=t.device)[1:1 + t.numel()].view(t.shape)
+        v.copy_(t)
+        return v
+    m, U, r0 = _model(batch)
+    want = m.predict(U, torch.empty_like(U), r0).clone()
+    for q in range(3):
+        a = [U, torch.zeros_like(U), r0]
+        a[q] = off(a[q])
+        assert torch.equal(m.predict(*a), want)
