@@ -104,7 +104,7 @@ _SIGS = [
     ("fvm_in_layer", ct.c_int, [_P, ct.c_int32, _P, _P, _P, _P, _P, _P]),
     ("fvm_corrector_in_layer", ct.c_int, [_P, _P, _P, ct.c_int32, _P, ct.c_int32, ct.c_int32, _P, _P, _P, ct.c_int32,
                                           _P, _P, _P, _P, _P, _P]),
-    ("fvm_corrector_in_layer_keep", ct.c_int, [_P, _P, _P, ct.c_int32, _P, ct.c_int32, ct.c_int32, _P, _P, _P,
+    ("fvm_corrector_in_layer_keep", ct.c_int, [_P, _P, _P, ct.c_float, _P, ct.c_int32, ct.c_int32, _P, _P, _P,
                                                ct.c_int32, _P, _P, _P, _P, _P, _P, _P]),
     ("fvm_corrector_propose", ct.c_int, [_P, _P, _P, _P, _P, _P, ct.c_int32, _P, ct.c_int32, ct.c_int32, _P, _P]),
     ("fvm_back_top", ct.c_int, [_P, _P, _P, _P, ct.c_int32, ct.c_int32, _P, _P, _P, _P, _P]),

@@ -411,7 +411,7 @@ class CorrectorModel:
         net, b, N = self.net, self.batch, state.shape[0]
         lib, s, bufs = net.lib, _lib.stream_ptr(), net._alloc(state.shape[0])
         _lib.check(lib.fvm_corrector_in_layer_keep(
-            state.data_ptr(), r0.data_ptr(), b.t_solver.dt.data_ptr(), self.k, self.cell_case32.data_ptr(), N, self.C,
+            state.data_ptr(), r0.data_ptr(), b.t_solver.dt.data_ptr(), float(self.k), self.cell_case32.data_ptr(), N, self.C,
             self.fmean.data_ptr(), self.finv.data_ptr(), self.geo.data_ptr(), self.geo.shape[1], self.base.data_ptr(),
             bufs["X"].data_ptr(), net.bf["W_in"].data_ptr(), net.params["b_in"].data_ptr(), bufs["hf"][0].data_ptr(),
             net.err.data_ptr(), s), "fvm_corrector_in_layer_keep")

@@ -1287,13 +1287,13 @@ extern "C" int fvm_in_layer(const void* X, int32_t M, const void* Wt, const floa
     return corr::launch_layer<true>(g, (cudaStream_t)stream);
 }
 
-extern "C" int fvm_corrector_in_layer_keep(const float* state, const float* r0, const float* dt, int32_t k,
+extern "C" int fvm_corrector_in_layer_keep(const float* state, const float* r0, const float* dt, float k,
                                            const int32_t* cell_case, int32_t N, int32_t C, const float* mean,
                                            const float* inv_std, const float* geo, int32_t G, float* base, void* X,
                                            const void* Wt, const float* bias, float* h_out, int32_t* err,
                                            void* stream) {
     if (!state || !r0 || !dt || !mean || !inv_std || (G > 0 && !geo) || !base || !Wt || !bias || !h_out || !err ||
-        N <= 0 || G < 0 || k < 1 || (C != 4 && C != 5) || 2 * C + G > corr::kLayerW)
+        N <= 0 || G < 0 || (C != 4 && C != 5) || 2 * C + G > corr::kLayerW)
         return FVM_E_ARG;
     if (((uintptr_t)h_out & 31u) || (uintptr_t)Wt % 16 || (uintptr_t)X % 16) return FVM_E_ARG;
     corr::LayerArgs g{};
@@ -1310,7 +1310,7 @@ extern "C" int fvm_corrector_in_layer_keep(const float* state, const float* r0, 
     g.C = C;
     g.G = G;
     g.whole = (((uintptr_t)state | (uintptr_t)r0 | (uintptr_t)base) & 15u) == 0;
-    g.k = (float)k;
+    g.k = k;
     g.Wt = static_cast<const __nv_bfloat16*>(Wt);
     g.bias = bias;
     g.h_out = h_out;
@@ -1322,7 +1322,8 @@ extern "C" int fvm_corrector_in_layer(const float* state, const float* r0, const
                                       const int32_t* cell_case, int32_t N, int32_t C, const float* mean,
                                       const float* inv_std, const float* geo, int32_t G, float* base, const void* Wt,
                                       const float* bias, float* h_out, int32_t* err, void* stream) {
-    return fvm_corrector_in_layer_keep(state, r0, dt, k, cell_case, N, C, mean, inv_std, geo, G, base, nullptr, Wt, bias,
+    if (k < 1) return FVM_E_ARG;
+    return fvm_corrector_in_layer_keep(state, r0, dt, (float)k, cell_case, N, C, mean, inv_std, geo, G, base, nullptr, Wt, bias,
                                        h_out, err, stream);
 }
 

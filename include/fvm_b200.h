@@ -397,8 +397,8 @@ int fvm_in_layer(const void *X, int32_t M, const void *Wt, const float *bias, fl
 int fvm_corrector_in_layer(const float *state, const float *r0, const float *dt, int32_t k, const int32_t *cell_case,
                            int32_t N, int32_t C, const float *mean, const float *inv_std, const float *geo, int32_t G,
                            float *base, const void *Wt, const float *bias, float *h_out, int32_t *err, void *stream);
-/* The same, also keeping the feature rows X (bf16 [N][64], 16-byte aligned, or NULL). */
-int fvm_corrector_in_layer_keep(const float *state, const float *r0, const float *dt, int32_t k,
+/* The same for any factor k, also keeping the feature rows X (bf16 [N][64], 16-byte aligned, or NULL). */
+int fvm_corrector_in_layer_keep(const float *state, const float *r0, const float *dt, float k,
                                 const int32_t *cell_case, int32_t N, int32_t C, const float *mean,
                                 const float *inv_std, const float *geo, int32_t G, float *base, void *X,
                                 const void *Wt, const float *bias, float *h_out, int32_t *err, void *stream);

@@ -154,3 +154,15 @@ def test_proposal_from_and_to_any_address(batch):
         a = [U, torch.zeros_like(U), r0]
         a[q] = off(a[q])
         assert torch.equal(m.predict(*a), want)
+
+
+@pytest.mark.parametrize("k", [np.int64(8), 8.0, np.float32(2.5)])
+def test_window_length_of_any_number_type(batch, k):
+    """``predict`` takes the window length as ``inputs`` does: base = float(k) dt r0."""
+    m, U, r0 = _model(batch)
+    m.k = k
+    m.inputs(U, r0)
+    base = m.base.clone()
+    m.base.zero_()
+    m.predict(U, torch.empty_like(U), r0)
+    assert torch.equal(m.base, base)
