@@ -150,7 +150,8 @@ __device__ __forceinline__ void ld_vec_cg(const float* p, float (&v)[N]) {
 }
 // Loads of arrays the same launch may have written (COH = true: the fused step kernel, whose
 // phases read what other blocks wrote before a grid barrier) go through L2 (.cg); in the one-phase
-// kernels those arrays are read-only for the launch and use the read-only path.
+// kernels those arrays are read-only for the launch and use the read-only path.  (The cell kernel's
+// boundary blocks replace the gradient rows that they read: plain loads there, bc_value's OWN.)
 template <bool COH, int N>
 __device__ __forceinline__ void ld_mut(const float* p, float (&v)[N]) {
     if constexpr (COH) ld_vec_cg<N>(p, v);
@@ -419,8 +420,9 @@ __device__ __forceinline__ float bc_block_scale(const fvm_mesh_t& m, const Phys&
 }
 
 // Boundary facet b's value (A_bc U + b_bc + A_corr grads_prev, then the characteristic BC) from its
-// cell's primitives U; `prev`: the cell's limited gradient row holds a previous evaluation.
-template <int DIM, bool COH>
+// cell's primitives U; `prev`: the cell's limited gradient row holds a previous evaluation.  OWN: the
+// calling thread replaces that row later in the same launch, so it is read with plain loads.
+template <int DIM, bool COH, bool OWN>
 __device__ __forceinline__ void bc_value(const fvm_mesh_t& m, const Phys& p, const float (&U)[L<DIM>::RS],
                                          const float* grad_row, bool prev, int b, float scale,
                                          float (&out)[L<DIM>::RS]) {
@@ -436,7 +438,8 @@ __device__ __forceinline__ void bc_value(const fvm_mesh_t& m, const Phys& p, con
             float corr = 0.f;
 #pragma unroll
             for (int d = 0; d < DIM; ++d)
-                corr = fmaf(__ldg(m.bc_l + b * DIM + d), ld1_mut<COH>(grad_row + Ly::gi(d, c)), corr);
+                corr = fmaf(__ldg(m.bc_l + b * DIM + d),
+                            OWN ? grad_row[Ly::gi(d, c)] : ld1_mut<COH>(grad_row + Ly::gi(d, c)), corr);
             v += corr;
         }
         out[c] = v;
@@ -495,7 +498,7 @@ __device__ __forceinline__ void bc_item(const fvm_mesh_t& m, const Phys& p, cons
     float U[Ly::RS], out[Ly::RS];
     ld_mut<COH, Ly::RS>(prims + (int64_t)cell * Ly::RS, U);
     const bool prev = (COH ? __ldcg(has_grads) : *has_grads) != 0;
-    bc_value<DIM, COH>(m, p, U, grads + (int64_t)cell * Ly::GS, prev, b, scale, out);
+    bc_value<DIM, COH, false>(m, p, U, grads + (int64_t)cell * Ly::GS, prev, b, scale, out);
     st_vec<Ly::RS>(bcv + (int64_t)b * Ly::RS, out);
 }
 
@@ -709,7 +712,7 @@ __device__ __forceinline__ void boundary_cells(const fvm_mesh_t& m, const Phys& 
         if (cols[k] < N) {
             ld_vec<RS>(prims + (int64_t)cols[k] * RS, X[k]);
         } else {
-            bc_value<DIM, false>(m, p, U, grads + (int64_t)cell * Ly::GS, prev, cols[k] - N, scale, X[k]);
+            bc_value<DIM, false, true>(m, p, U, grads + (int64_t)cell * Ly::GS, prev, cols[k] - N, scale, X[k]);
             st_vec<RS>(bcv + (int64_t)(cols[k] - N) * RS, X[k]);
         }
     }
