@@ -324,7 +324,7 @@ __device__ __forceinline__ float limiter_phi(int p, float delta, float dU, float
 // single and batched meshes, the boundary kernel, the cell kernel's boundary blocks, the fused step.
 // Four elements of a thread are in flight at a time, their cells fetched one step ahead.  (Small on
 // purpose: on small meshes the kernel is bound by latency, and sixteen at a time or prefetches cost
-// it 0.5 us per launch.)
+// it 0.5 us per launch; the loop unrolled by the compiler costs a 120 k-cell sphere 0.6 us.)
 template <int DIM, bool COH, int NP>
 __device__ __forceinline__ void char_parts(const fvm_mesh_t& m, const Phys& p, const float* prims, int first, int hi,
                                            int stride, double (&acc)[4]) {
@@ -335,6 +335,7 @@ __device__ __forceinline__ void char_parts(const fvm_mesh_t& m, const Phys& p, c
         for (int q = 0; q < U; ++q) cell[q] = t + q * stride < hi ? __ldg(m.ch_cell + t + q * stride) : -1;
     };
     fetch(first);
+#pragma unroll 1
     for (int t = first; t < hi; t += U * stride) {
         float T[U];
         bool on[U];
