@@ -2244,8 +2244,12 @@ static int launch_residual(const fvm_mesh_t* m, const Phys& p, const float* prim
 template <int DIM>
 static int residual_impl(const fvm_mesh_t* m, const Phys& p, const float* prims_user, float* grads,
                          int32_t* has_grads, float* dudt, const fvm_work_t* w, cudaStream_t s) {
-    // 2D rows need no padding: aligned primitives are read where they are (a launch and a pass less)
-    if (DIM == 2 && ((uintptr_t)prims_user & 15u) == 0 && owned_cells(m) == m->n_cells && m->cell_lo == 0 && !m->case_active)
+    // 2D rows need no padding: aligned primitives are read where they are (a launch and a pass less).  Not
+    // where the kernel that stores dudt still reads them (owner computes) and the two overlap.
+    const uintptr_t a = (uintptr_t)prims_user, b = (uintptr_t)dudt, bytes = (uintptr_t)m->n_cells * m->n_comp * 4;
+    const bool apart = a + bytes <= b || b + bytes <= a;
+    if (DIM == 2 && (a & 15u) == 0 && owned_cells(m) == m->n_cells && m->cell_lo == 0 && !m->case_active &&
+        (apart || g_div_variant == 0))
         return launch_residual<DIM>(m, p, prims_user, grads, has_grads, dudt, w, s);
     FVM_LAUNCH(KID_STATE_TO_PRIMS, s, launch(k_pad_prims<DIM>, dim3(blocks_for(m->n_cells)), dim3(kBlock), 0, s, 
                                           m->n_cells, prims_user, w->prims));

@@ -231,7 +231,9 @@ int fvm_ell_spmm(const float *vals, const int32_t *cols, int64_t M, int32_t K,
 /* dU/dt [N][C] (conserved variables) of the primitives prims [N][C].  grads [N][FVM_GROW] is
  * read as the previous limited gradient when the device flag *has_grads != 0 (the reference's
  * FacetCalc.cell_grads is not None) and overwritten with this evaluation's limited gradient;
- * the call sets *has_grads = 1.  Meshes with kg > dim + 2 take the generic-width cell kernel. */
+ * the call sets *has_grads = 1.  Meshes with kg > dim + 2 take the generic-width cell kernel.
+ * prims must stay as they are until the call's work on the stream is done (2D rows on 16-byte boundaries
+ * are read where they are, by every kernel but the divergence); dudt may be prims. */
 int fvm_residual(const fvm_mesh_t *mesh, const fvm_physics_t *phys, const float *prims,
                  float *grads, int32_t *has_grads, float *dudt, const fvm_work_t *work,
                  void *stream);
