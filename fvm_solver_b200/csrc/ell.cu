@@ -15,8 +15,8 @@
 
 namespace fvm {
 
-// Every kernel is templated on an upper bound KT of the slot count (2, 4, 5, 8 or 16; five slots are the
-// widest rows of the residual's operators) and unrolls the
+// Every kernel is templated on an upper bound KT of the slot count (2, 4, 5, 6, 8, 12 or 16; five slots are the
+// widest rows of the residual's operators on the reference's stencil) and unrolls the
 // slot loop, so the values, columns and gathers of all slots of a row are in flight together (one
 // dependent round trip per row instead of K); slots are summed in order k = 0, 1, ...
 //
@@ -27,6 +27,14 @@ namespace fvm {
 // stays contiguous over the warp) before it gathers for the current ones.  On the operators of a
 // 438 k-tet box: facet gradient (4.4 M rows of two slots) 41 -> 22 us, cell gradient (1.3 M rows of
 // five) 21 -> 14 us, with five columns 26 -> 19 us, divergence with five columns 14 -> 11 us.
+//
+// Rows of more than five slots, and most products with several columns, take one row per thread and no look
+// ahead (the *_once kernels, all slots loaded before the first gather): a second set of that many slots leaves
+// 8 to 32 warps per SM or spills, and more warps hide the two round trips better.  M rows of K slots with B
+// columns, look ahead against once, in us, operator in the L2 / not there: 240 k x 6 (B 1) 5.1 / 5.6 against
+// 3.5 / 5.1; 240 k x 10 (B 1) 9.4 / 11.8 against 5.2 / 7.2; 1.3 M x 16 (B 1) 43 / 45 against 35 / 36;
+// 240 k x 10 (B 5) 20.9 / 24.0 against 15.9 / 17.2; 1.3 M x 5 (B 2) 28.8 / 31.0 against 22.3 / 24.8;
+// 1.3 M x 16 (B 9) 373 / 376 against 272 / 274.
 constexpr int kEllBlocks = 4;
 
 template <int KT, int RT>
@@ -82,18 +90,83 @@ __global__ void __launch_bounds__(kBlock, kEllBlocks) k_ell_spmv(const float* __
     }
 }
 
+template <int KT>
+__global__ void __launch_bounds__(kBlock) k_ell_spmv_once(const float* __restrict__ vals,
+                                                          const int32_t* __restrict__ cols, int64_t M,
+                                                          int K, const float* __restrict__ x,
+                                                          int64_t incx, const float* __restrict__ bias,
+                                                          float* __restrict__ y, int64_t incy) {
+    const int64_t r = blockIdx.x * (int64_t)kBlock + threadIdx.x;
+    if (r >= M) return;
+    float v[KT], xv[KT];
+    int c[KT];
+#pragma unroll
+    for (int k = 0; k < KT; ++k) {
+        v[k] = k < K ? __ldg(vals + k * M + r) : 0.f;
+        c[k] = k < K ? __ldg(cols + k * M + r) : 0;
+    }
+    const float b = bias ? __ldg(bias + r) : 0.f;
+#pragma unroll
+    for (int k = 0; k < KT; ++k) xv[k] = k < K ? __ldg(x + (int64_t)c[k] * incx) : 0.f;
+    float acc = 0.f;
+#pragma unroll
+    for (int k = 0; k < KT; ++k)
+        if (k < K) acc = fmaf(v[k], xv[k], acc);
+    if (bias) acc += b;
+    y[r * incy] = acc;
+}
+
 // One thread per (row, group of CB columns).
 template <int KT, int CB>
-__global__ void __launch_bounds__(kBlock, KT <= 8 ? kEllBlocks : 1) k_ell_spmm(const float* __restrict__ vals,
+__global__ void __launch_bounds__(kBlock) k_ell_spmm_once(const float* __restrict__ vals,
+                                                          const int32_t* __restrict__ cols, int64_t M,
+                                                          int K, const float* __restrict__ X,
+                                                          int64_t ldx, int B,
+                                                          const float* __restrict__ bias,
+                                                          float* __restrict__ Y, int64_t ldy) {
+    const int64_t r = blockIdx.x * (int64_t)kBlock + threadIdx.x;
+    if (r >= M) return;
+    const int c0 = blockIdx.y * CB;
+    const int nb = min(CB, B - c0);
+    float v[KT];
+    int c[KT];
+#pragma unroll
+    for (int k = 0; k < KT; ++k) {
+        v[k] = k < K ? __ldg(vals + k * M + r) : 0.f;
+        c[k] = k < K ? __ldg(cols + k * M + r) : 0;
+    }
+    float acc[CB];
+#pragma unroll
+    for (int j = 0; j < CB; ++j) acc[j] = 0.f;
+#pragma unroll
+    for (int k = 0; k < KT; ++k) {
+        if (k >= K) break;
+        float xr[CB];
+        const float* xk = X + (int64_t)c[k] * ldx + c0;
+#pragma unroll
+        for (int j = 0; j < CB; ++j) xr[j] = j < nb ? __ldg(xk + j) : 0.f;
+#pragma unroll
+        for (int j = 0; j < CB; ++j)
+            if (j < nb) acc[j] = fmaf(v[k], xr[j], acc[j]);
+    }
+    const float b = bias ? __ldg(bias + r) : 0.f;
+    float* yr = Y + r * ldy + c0;
+#pragma unroll
+    for (int j = 0; j < CB; ++j)
+        if (j < nb) yr[j] = bias ? acc[j] + b : acc[j];
+}
+
+// The same for groups of CB whole columns (B a multiple of CB), with the look ahead.
+template <int KT, int CB>
+__global__ void __launch_bounds__(kBlock, kEllBlocks) k_ell_spmm(const float* __restrict__ vals,
                                                       const int32_t* __restrict__ cols, int64_t M,
                                                       int K, const float* __restrict__ X,
-                                                      int64_t ldx, int B,
+                                                      int64_t ldx,
                                                       const float* __restrict__ bias,
                                                       float* __restrict__ Y, int64_t ldy) {
     const int64_t step = (int64_t)gridDim.x * kBlock;
     int64_t r = blockIdx.x * (int64_t)kBlock + threadIdx.x;
     const int c0 = blockIdx.y * CB;
-    const int nb = min(CB, B - c0);
     EllRows<KT, 1> next;
     next.load(vals, cols, M, K, r);
     for (; r < M; r += step) {
@@ -108,16 +181,14 @@ __global__ void __launch_bounds__(kBlock, KT <= 8 ? kEllBlocks : 1) k_ell_spmm(c
             float xr[CB];
             const float* xk = X + (int64_t)cur.c[0][k] * ldx + c0;
 #pragma unroll
-            for (int j = 0; j < CB; ++j) xr[j] = j < nb ? __ldg(xk + j) : 0.f;
+            for (int j = 0; j < CB; ++j) xr[j] = __ldg(xk + j);
 #pragma unroll
-            for (int j = 0; j < CB; ++j)
-                if (j < nb) acc[j] = fmaf(cur.v[0][k], xr[j], acc[j]);
+            for (int j = 0; j < CB; ++j) acc[j] = fmaf(cur.v[0][k], xr[j], acc[j]);
         }
         const float b = bias ? __ldg(bias + r) : 0.f;
         float* yr = Y + r * ldy + c0;
 #pragma unroll
-        for (int j = 0; j < CB; ++j)
-            if (j < nb) yr[j] = bias ? acc[j] + b : acc[j];
+        for (int j = 0; j < CB; ++j) yr[j] = bias ? acc[j] + b : acc[j];
     }
 }
 
@@ -331,6 +402,8 @@ extern "C" int fvm_ell_spmv(const float* vals, const int32_t* cols, int64_t M, i
     // several rows per thread only where every SM still gets its blocks
 #define FVM_SPMV_R(KT, RT) FVM_LAUNCH(fvm::KID_ELL_SPMV, s, fvm::k_ell_spmv<KT, RT><<<ell_grid(M, RT, wave, fvm::kEllBlocks), \
                                       fvm::kBlock, 0, s>>>(vals, cols, M, K, x, incx, bias, y, incy))
+#define FVM_SPMV_1(KT) FVM_LAUNCH(fvm::KID_ELL_SPMV, s, fvm::k_ell_spmv_once<KT><<<(unsigned)((M + fvm::kBlock - 1) / fvm::kBlock), \
+                                  fvm::kBlock, 0, s>>>(vals, cols, M, K, x, incx, bias, y, incy))
 #define FVM_SPMV(KT, RT)                                                                                \
     do {                                                                                                \
         if (RT > 1 && M >= wave * fvm::kEllBlocks * fvm::kBlock * RT) FVM_SPMV_R(KT, RT);              \
@@ -339,8 +412,11 @@ extern "C" int fvm_ell_spmv(const float* vals, const int32_t* cols, int64_t M, i
     if (K <= 2) FVM_SPMV(2, 4);
     else if (K <= 4) FVM_SPMV(4, 2);
     else if (K <= 5) FVM_SPMV(5, 1);
-    else if (K <= 8) FVM_SPMV(8, 1);
-    else FVM_SPMV(16, 1);
+    else if (K <= 6) FVM_SPMV_1(6);
+    else if (K <= 8) FVM_SPMV_1(8);
+    else if (K <= 12) FVM_SPMV_1(12);
+    else FVM_SPMV_1(16);
+#undef FVM_SPMV_1
 #undef FVM_SPMV_R
 #undef FVM_SPMV
     return launch_status();
@@ -376,12 +452,18 @@ extern "C" int fvm_ell_spmm(const float* vals, const int32_t* cols, int64_t M, i
 #undef FVM_SPMM5
     } else {
         const unsigned gy = (unsigned)((B + 7) / 8);
-#define FVM_SPMM(KT) FVM_LAUNCH(fvm::KID_ELL_SPMM, s, fvm::k_ell_spmm<KT, 8><<<dim3(ell_grid(M, 1, wave, fvm::kEllBlocks), gy), fvm::kBlock, 0, s>>>( \
-                                    vals, cols, M, K, X, ldx, B, bias, Y, ldy))
-        if (K <= 4) FVM_SPMM(4);
-        else if (K <= 8) FVM_SPMM(8);
-        else FVM_SPMM(16);
-#undef FVM_SPMM
+#define FVM_SPMM_1(KT) FVM_LAUNCH(fvm::KID_ELL_SPMM, s, fvm::k_ell_spmm_once<KT, 8><<<dim3((unsigned)gx, gy), fvm::kBlock, 0, s>>>( \
+                                      vals, cols, M, K, X, ldx, B, bias, Y, ldy))
+        if (B % 8 == 0 && K > 4 && K <= 8)   // whole groups: 1.3 M rows of six slots with eight columns 112 against 129 us
+            FVM_LAUNCH(fvm::KID_ELL_SPMM, s, fvm::k_ell_spmm<8, 8><<<dim3(ell_grid(M, 1, wave, fvm::kEllBlocks), gy),
+                                                                    fvm::kBlock, 0, s>>>(vals, cols, M, K, X, ldx, bias, Y, ldy));
+        else if (K <= 4) FVM_SPMM_1(4);
+        else if (K <= 5) FVM_SPMM_1(5);
+        else if (K <= 6) FVM_SPMM_1(6);
+        else if (K <= 8) FVM_SPMM_1(8);
+        else if (K <= 12) FVM_SPMM_1(12);
+        else FVM_SPMM_1(16);
+#undef FVM_SPMM_1
     }
     return launch_status();
 }
