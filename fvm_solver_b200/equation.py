@@ -81,6 +81,12 @@ class FluidConstitution3D(FluidConstitution):
         assert self.dim == 3, "Only for 3D fluids"
 
 
+# Largest share of the device's memory that the row tables may take for the tiled copies (about as large
+# again) to be made beside them: with both, the state and the work arrays of a tetrahedral mesh at this size
+# (some 160 M cells on 180 GB) fill about three quarters.  Larger meshes run from the rows.
+TILED_SHARE = 0.25
+
+
 class DeviceMesh:
     """Kernel tables uploaded to one device (record layout), plus the ``fvm_mesh_t`` struct."""
 
@@ -95,9 +101,12 @@ class DeviceMesh:
         self.n_facets, self.n_bc, self.kg, self.kf = kt.n_facets, kt.n_bc, kt.kg, kt.kf
         self.row, self.grow = row_sizes(kt.dim)
         up = {k: v.contiguous().to(self.device) for k, v in (records or kt.records()).items()}
+        rows = sum(v.numel() * v.element_size() for v in up.values())
         for f in self._struct_fields:
             up[f] = getattr(kt, f).contiguous().to(self.device)
-        up.update(tiled_records(kt.dim, kt.kg, kt.kf, up))
+        if self.device.type != "cuda" or \
+                rows <= TILED_SHARE * torch.cuda.get_device_properties(self.device).total_memory:
+            up.update(tiled_records(kt.dim, kt.kg, kt.kf, up))
         self.t = SimpleNamespace(**up)
         m = _lib.Mesh(dim=kt.dim, n_comp=kt.n_comp, n_cells=kt.n_cells, n_facets=kt.n_facets,
                       n_bc=kt.n_bc, n_char=kt.n_char, kg=kt.kg, kf=kt.kf)
