@@ -1676,16 +1676,21 @@ __global__ void __launch_bounds__(256) k_back_finish(FinishArgs f) {
 //   TMA in the 128-byte swizzle (64 channels of a row = one swizzled line; rows past N read as zero);
 //   warp 9 issues the MMAs
 //     dA  [128 x 128] = dZ . W       (K-major dZ and W^T; two accumulators)
-//     dW^T [128 x 64] += A^T . dZ    (the same copies read MN-major, the tile's rows as K; one
-//                                     accumulator in tensor memory for the CTA's whole run);
+//     dW^T [128 x 64] += A^T . dZ    (the same copies read MN-major, the tile's rows as K; two
+//                                     accumulators for chunks of four tiles in turn);
 //   warps 0-7 read dA (warp w: TMEM lanes 32 (w % 4), columns 64 (w / 4)), divide the neighbour half
 //   by the row's neighbour count and store it, a row's 32 columns on four lanes as one 128-byte line.
-//   At the end the CTA adds its dW^T to dW.
+//   After each chunk they also add its dW^T to their registers, and at the end the CTA's sum to dW.
+// The chunks are there for accuracy: the tensor core's fp32 accumulator does not round to nearest, and its
+// error grows with the rows it has taken.  Relative error of one-signed sums at 278 k and 4.1 M rows: one
+// accumulator for the whole run 5.0e-6 and 1.4e-4, split-K products over 512 ranges 1.1e-6 and 3.5e-5, chunks
+// of 512 rows summed in registers 8.4e-7 and 9.1e-7 (at less than 1 % of a training step).
 // Without dA (the input layer) A is the [N][64] feature rows and only dW is formed.
 // Bound by memory, 0.9 kB per row.  Copies by four warps' cp.async into no-swizzle operands held the L1's
 // path for 3000 cycles per tile, and their warp also issued the MMAs (2200 cycles per tile); with stores
 // of one row per lane that took 75 us per layer at 278 k rows.
 constexpr int kBackThreads = 320, kBackStages = 4;
+constexpr int kChunkTiles = 4;                                                   // tiles per dW^T accumulation
 constexpr int kBackHalf = TM * kLayerW * 2;                                      // 128 rows x 64 channels
 constexpr int kBackStage = 3 * kBackHalf;                                        // dZ and A of one tile
 constexpr int kBackSmem = 1024 + kBackStages * kBackStage + 8 * kUnitBytes;      // + alignment, W^T (128 x 64)
@@ -1713,7 +1718,8 @@ __global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __grid_con
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
     uint8_t* sW = smem + kBackStages * kBackStage;
-    __shared__ __align__(8) uint64_t bar_load[kBackStages], bar_free[kBackStages], bar_full[2], bar_empty[2], bar_done;
+    __shared__ __align__(8) uint64_t bar_load[kBackStages], bar_free[kBackStages], bar_full[2], bar_empty[2];
+    __shared__ __align__(8) uint64_t bar_wfull[2], bar_wfree[2], bar_done;
     __shared__ uint32_t s_taddr;
     __shared__ int s_fail;
     constexpr int AU = LAYER ? 16 : 8;                    // 8-channel units of an A row
@@ -1733,6 +1739,8 @@ __global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __grid_con
         for (int b = 0; b < 2; ++b) {
             mbar_init(&bar_full[b], 1);
             mbar_init(&bar_empty[b], 8);
+            mbar_init(&bar_wfull[b], 1);
+            mbar_init(&bar_wfree[b], 8);
         }
         mbar_init(&bar_done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;");
@@ -1751,9 +1759,29 @@ __global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __grid_con
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
-    const uint32_t taddr = s_taddr, tw = taddr + 256;     // dA: columns 0..255, dW^T: 256..319
+    const uint32_t taddr = s_taddr, tw = taddr + 256;     // dA: columns 0..255, dW^T: 256..383
     const uint32_t id_a = make_idesc(TM);
     const uint32_t id_w = make_idesc(kLayerW) | (1u << 15) | (1u << 16);   // both operands MN-major
+    float sum[32];                                        // warps 0-7: dW^T, input channel 32 (w % 4) + lane,
+#pragma unroll                                            // output channels 32 (w / 4) ..
+    for (int n = 0; n < 32; ++n) sum[n] = 0.f;
+    // Chunk c's dW^T -> the sums (warps 0-7, all lanes).
+    auto take = [&](int c) {
+        const bool ok = mbar_wait(&bar_wfull[c & 1], (uint32_t)((c >> 1) & 1));
+        if (!__all_sync(0xffffffffu, ok)) {
+            if (lane == 0) atomicExch(&s_fail, 1);
+            return false;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        uint32_t v[32];
+        tmem_ld32(tw + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(kLayerW * (c & 1) + 32 * (warp >> 2)), v);
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar_wfree[c & 1]);
+#pragma unroll
+        for (int n = 0; n < 32; ++n) sum[n] += __uint_as_float(v[n]);
+        return true;
+    };
 
     if (warp == 8) {
         if (lane == 0) {
@@ -1779,9 +1807,11 @@ __global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __grid_con
     } else if (warp == 9) {
         if (lane == 0) {
             for (int k = 0; k < nlocal; ++k) {
-                const int a = k & 1, st = k % kBackStages;
+                const int a = k & 1, st = k % kBackStages, c = k / kChunkTiles;
+                const bool first = k % kChunkTiles == 0, last = (k + 1) % kChunkTiles == 0 || k + 1 == nlocal;
                 if (!mbar_wait(&bar_load[st], (uint32_t)((k / kBackStages) & 1)) ||
-                    (LAYER && k >= 2 && !mbar_wait(&bar_empty[a], (uint32_t)(((k >> 1) - 1) & 1)))) {
+                    (LAYER && k >= 2 && !mbar_wait(&bar_empty[a], (uint32_t)(((k >> 1) - 1) & 1))) ||
+                    (first && c >= 2 && !mbar_wait(&bar_wfree[c & 1], (uint32_t)(((c >> 1) - 1) & 1)))) {
                     atomicExch(&s_fail, 1);
                     break;
                 }
@@ -1794,10 +1824,11 @@ __global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __grid_con
                                make_desc(smem_u32(sW) + 2 * q * kUnitBytes, kUnitBytes, 128), id_a, q > 0);
 #pragma unroll
                 for (int q = 0; q < TM / 16; ++q)
-                    tc_mma(tw, make_desc_sw(sa + 2048 * q, kBackHalf), make_desc_sw(sz + 2048 * q, kBackHalf), id_w,
-                           k > 0 || q > 0);
+                    tc_mma(tw + kLayerW * (c & 1), make_desc_sw(sa + 2048 * q, kBackHalf),
+                           make_desc_sw(sz + 2048 * q, kBackHalf), id_w, !first || q > 0);
                 tc_commit(&bar_free[st]);
                 if (LAYER) tc_commit(&bar_full[a]);
+                if (last) tc_commit(&bar_wfull[c & 1]);
             }
             // Covers every MMA issued, also when a wait gave up.  A barrier of its own, completed once: of
             // bar_full several phases can be open where no reader follows them (the input layer), and a
@@ -1852,7 +1883,11 @@ __global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __grid_con
                     }
                 }
             }
+            if (((k + 1) % kChunkTiles == 0 || k + 1 == nlocal) && !take(k / kChunkTiles)) break;
         }
+    } else {
+        for (int c = 0; c * kChunkTiles < nlocal; ++c)
+            if (!take(c)) break;
     }
     __syncthreads();
     // no MMA is in flight past this point (a second bounded chance before tensor memory is released)
@@ -1860,17 +1895,11 @@ __global__ void __launch_bounds__(kBackThreads, 1) k_back_layer(const __grid_con
     if (!__syncthreads_and(done) || s_fail) {
         if (tid == 0) atomicExch(err, 1);
         if (!done) mbar_wait(&bar_done, 0u);
-    } else if (warp < 4) {
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        uint32_t v[32];
-        const int in = 32 * warp + lane;                  // input channel
+    } else if (warp < 8) {
+        const int in = 32 * (warp & 3) + lane;            // input channel
+        if (in < 8 * AU)
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            tmem_ld32(tw + ((uint32_t)(32 * warp) << 16) + 32 * half, v);
-            if (in < 8 * AU)
-#pragma unroll
-                for (int n = 0; n < 32; ++n) atomicAdd(dW + (int64_t)(32 * half + n) * (8 * AU) + in, __uint_as_float(v[n]));
-        }
+            for (int n = 0; n < 32; ++n) atomicAdd(dW + (int64_t)(32 * (warp >> 2) + n) * (8 * AU) + in, sum[n]);
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();

@@ -166,3 +166,27 @@ def test_window_length_of_any_number_type(batch, k):
     m.base.zero_()
     m.predict(U, torch.empty_like(U), r0)
     assert torch.equal(m.base, base)
+
+
+@pytest.mark.parametrize("N", [128 * 148 * 4 - 1, 128 * 148 * 9 + 1, 1_000_003])
+@pytest.mark.parametrize("layer", [True, False])
+def test_weight_gradients_keep_their_accuracy(layer, N):
+    """dW of one-signed terms against FP64, one to many chunks of rows per block.  A chunk is 512 rows: 32
+    accumulations in the tensor core, each off by less than an ulp of the running sum in one direction, so
+    at most 32 * 2^-23 = 3.8e-6 of a chunk and, with the rounded additions of the chunks, 4e-6 of the sum
+    (a single accumulator for the block's rows is off by 2.5e-5 at 1 M rows)."""
+    from fvm_solver_b200 import _lib
+    lib, s = _lib.load(), _lib.stream_ptr()
+    C = 128 if layer else 64
+    err, P = torch.zeros(1, dtype=torch.int32, device="cuda"), lambda t: t.data_ptr()
+    dZ, A = _rand(N, 64, seed=1).abs().bfloat16(), _rand(N, C, seed=2).abs().bfloat16()
+    dW = torch.zeros(64, C, device="cuda")
+    if layer:
+        WT, nbr = torch.zeros(128, 64, device="cuda").bfloat16(), torch.full((N, 3), -1, dtype=torch.int32, device="cuda")
+        dA = torch.empty(N, 128, device="cuda")
+        rc = lib.fvm_back_layer(P(dZ), P(A), P(WT), P(nbr), 3, N, P(dA), P(dW), P(err), s)
+    else:
+        rc = lib.fvm_back_layer(P(dZ), P(A), None, None, 0, N, None, P(dW), P(err), s)
+    want = sum(dZ[i:i + 400_000].double().t() @ A[i:i + 400_000].double() for i in range(0, N, 400_000))
+    assert rc == 0 and int(err.item()) == 0
+    assert float(((dW.double() - want).abs() / want).max()) < 4e-6
