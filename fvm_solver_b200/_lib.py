@@ -113,11 +113,7 @@ _SIGS = [
     ("fvm_back_gather", ct.c_int, [_P, _P, ct.c_int32, ct.c_int32, _P, _P, _P, _P, _P, _P, _P, _P]),
     ("fvm_back_bias", ct.c_int, [_P, _P, ct.c_int32, _P, _P]),
     ("fvm_back_finish", ct.c_int, [ct.c_int32, _P, _P, _P, _P]),
-    ("fvm_mp_scatter_back", ct.c_int, [_P, _P, ct.c_int32, ct.c_int32, ct.c_int32, _P, _P, _P]),
-    ("fvm_silu_back", ct.c_int, [_P, _P, ct.c_int32, ct.c_int32, _P, _P, ct.c_int64, _P, _P]),
-    ("fvm_transpose_bf16", ct.c_int, [_P, ct.c_int32, ct.c_int32, ct.c_int64, _P, ct.c_int64, _P]),
     ("fvm_decoder_f32", ct.c_int, [_P, _P, _P, ct.c_int32, ct.c_int32, _P, _P]),
-    ("fvm_decoder_back_f32", ct.c_int, [_P, _P, _P, ct.c_int32, ct.c_int32, _P, _P, _P, _P]),
     ("fvm_mse", ct.c_int, [_P, _P, ct.c_int64, _P, _P, _P]),
     ("fvm_adam_many", ct.c_int, [ct.c_int32, _P, _P, _P, _P, _P, ct.c_float, ct.c_float, ct.c_float, ct.c_float,
                                  ct.c_int32, _P, _P, _P, _P, _P]),

@@ -376,55 +376,6 @@ extern "C" int fvm_gemm_bf16(const void* A, int64_t lda, const void* B, int64_t 
 namespace fvm {
 namespace corr {
 
-// dh_out[i] = dh_in[i] + dA[i][:W] + sum_{j in nbr(i)} dA[j][W:] / deg(j)   (adjacency symmetric).
-__global__ void k_mp_scatter_back(const float* __restrict__ dA, const int32_t* __restrict__ nbr, int N, int W, int KN,
-                                  const float* __restrict__ dh_in, float* __restrict__ dh_out) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= (int64_t)N * W) return;
-    const int i = (int)(t / W), c = (int)(t % W);
-    float v = dA[(int64_t)i * 2 * W + c] + (dh_in ? dh_in[t] : 0.f);
-    for (int k = 0; k < KN; ++k) {
-        const int j = __ldg(nbr + (int64_t)i * KN + k);
-        if (j < 0) continue;
-        int deg = 0;
-        for (int q = 0; q < KN; ++q) deg += __ldg(nbr + (int64_t)j * KN + q) >= 0;
-        v += dA[(int64_t)j * 2 * W + W + c] / (float)deg;
-    }
-    dh_out[t] = v;
-}
-
-// dZ = dh * silu'(Z); writes dZ as bf16 [N][W] and transposed bf16 [W][ldT] (columns >= N zero),
-// and accumulates the bias gradient sum_i dZ[i].
-__global__ void k_silu_back(const float* __restrict__ dh, const float* __restrict__ Z, int N, int W,
-                            __nv_bfloat16* __restrict__ dZ, __nv_bfloat16* __restrict__ dZT, int64_t ldT,
-                            float* __restrict__ db) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= (int64_t)N * W) return;
-    const int i = (int)(t / W), c = (int)(t % W);
-    const float z = Z[t];
-    const float s = 1.f / (1.f + __expf(-z));
-    const float g = dh[t] * s * (1.f + z * (1.f - s));
-    dZ[t] = __float2bfloat16(g);
-    if (dZT) dZT[(int64_t)c * ldT + i] = __float2bfloat16(g);
-    if (db) atomicAdd(db + c, g);
-}
-
-// dst[c][r] = src[r][c] for a bf16 [R][Cc] matrix (32 x 32 tiles through shared memory).
-__global__ void k_transpose_bf16(const __nv_bfloat16* __restrict__ src, int R, int Cc, int64_t lds,
-                                 __nv_bfloat16* __restrict__ dst, int64_t ldd) {
-    __shared__ __nv_bfloat16 tile[32][33];
-    const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;   // rows on x: R may exceed 65535 * 32
-    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const int r = r0 + k, c = c0 + threadIdx.x;
-        tile[k][threadIdx.x] = (r < R && c < Cc) ? src[(int64_t)r * lds + c] : __float2bfloat16(0.f);
-    }
-    __syncthreads();
-    for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-        const int c = c0 + k, r = r0 + threadIdx.x;
-        if (c < Cc && r < R) dst[(int64_t)c * ldd + r] = tile[threadIdx.x][k];
-    }
-}
-
 __global__ void k_mse(const float* __restrict__ pred, const float* __restrict__ tgt, int64_t n_elem, float inv_n,
                       double* __restrict__ loss, float* __restrict__ dpred) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -599,36 +550,6 @@ static inline unsigned nblk(int64_t n, int bs) { return (unsigned)((n + bs - 1) 
 
 }  // namespace corr
 }  // namespace fvm
-
-extern "C" int fvm_mp_scatter_back(const float* dA, const int32_t* nbr, int32_t N, int32_t W, int32_t KN,
-                                   const float* dh_in, float* dh_out, void* stream) {
-    if (!dA || !nbr || !dh_out || N <= 0 || W <= 0 || KN <= 0) return FVM_E_ARG;
-    cudaStream_t s = (cudaStream_t)stream;
-    FVM_LAUNCH(KID_CORRECTOR, s, corr::k_mp_scatter_back<<<corr::nblk((int64_t)N * W, 256), 256, 0, s>>>(
-                                     dA, nbr, N, W, KN, dh_in, dh_out));
-    return launch_status();
-}
-
-extern "C" int fvm_silu_back(const float* dh, const float* Z, int32_t N, int32_t W, void* dZ, void* dZT, int64_t ldT,
-                             float* db, void* stream) {
-    if (!dh || !Z || !dZ || N <= 0 || W <= 0 || (dZT && ldT < N)) return FVM_E_ARG;
-    cudaStream_t s = (cudaStream_t)stream;
-    FVM_LAUNCH(KID_CORRECTOR, s, corr::k_silu_back<<<corr::nblk((int64_t)N * W, 256), 256, 0, s>>>(
-                                     dh, Z, N, W, static_cast<__nv_bfloat16*>(dZ), static_cast<__nv_bfloat16*>(dZT),
-                                     ldT, db));
-    return launch_status();
-}
-
-extern "C" int fvm_transpose_bf16(const void* src, int32_t R, int32_t Cc, int64_t lds, void* dst, int64_t ldd,
-                                  void* stream) {
-    if (!src || !dst || R <= 0 || Cc <= 0 || ldd < R || lds < Cc || (Cc + 31) / 32 > 65535) return FVM_E_ARG;
-    cudaStream_t s = (cudaStream_t)stream;
-    dim3 grid((unsigned)((R + 31) / 32), (unsigned)((Cc + 31) / 32));
-    FVM_LAUNCH(KID_CORRECTOR, s, corr::k_transpose_bf16<<<grid, dim3(32, 8), 0, s>>>(
-                                     static_cast<const __nv_bfloat16*>(src), R, Cc, lds,
-                                     static_cast<__nv_bfloat16*>(dst), ldd));
-    return launch_status();
-}
 
 extern "C" int fvm_mse(const float* pred, const float* tgt, int64_t n_elem, double* loss, float* dpred,
                        void* stream) {
@@ -1216,25 +1137,6 @@ __global__ void k_decoder_f32(const float* __restrict__ h, const float* __restri
     for (int o = 0; o < O; ++o) out[(int64_t)i * O + o] = acc[o];
 }
 
-// Decoder backward on the fp32 stream: dh[i][c] = sum_o dOut[i][o] Wo[o][c];
-// dWo[o][c] += sum_i dOut[i][o] h[i][c]; dbo[o] += sum_i dOut[i][o].
-__global__ void k_decoder_back_f32(const float* __restrict__ h, const float* __restrict__ Wo,
-                                   const float* __restrict__ dOut, int N, int O, float* __restrict__ dh,
-                                   float* __restrict__ dWo, float* __restrict__ dbo) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= (int64_t)N * kLayerW) return;
-    const int i = (int)(t / kLayerW), c = (int)(t % kLayerW);
-    const float x = h[t];
-    float v = 0.f;
-    for (int o = 0; o < O; ++o) {
-        const float d = dOut[(int64_t)i * O + o];
-        v = fmaf(d, Wo[o * kLayerW + c], v);
-        atomicAdd(dWo + o * kLayerW + c, d * x);
-        if (c == 0) atomicAdd(dbo + o, d);
-    }
-    dh[t] = v;
-}
-
 }  // namespace corr
 }  // namespace fvm
 
@@ -1341,15 +1243,6 @@ extern "C" int fvm_decoder_f32(const float* h, const float* Wo, const float* bo,
     if (!h || !Wo || !bo || !out || N <= 0 || O < 1 || O > 8 || ((uintptr_t)h & 31u)) return FVM_E_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     FVM_LAUNCH(KID_CORRECTOR, s, corr::k_decoder_f32<<<corr::nblk(N, 256), 256, 0, s>>>(h, Wo, bo, N, O, out));
-    return launch_status();
-}
-
-extern "C" int fvm_decoder_back_f32(const float* h, const float* Wo, const float* dOut, int32_t N, int32_t O,
-                                    float* dh, float* dWo, float* dbo, void* stream) {
-    if (!h || !Wo || !dOut || !dh || !dWo || !dbo || N <= 0 || O < 1 || O > 8) return FVM_E_ARG;
-    cudaStream_t s = (cudaStream_t)stream;
-    FVM_LAUNCH(KID_CORRECTOR, s, corr::k_decoder_back_f32<<<corr::nblk((int64_t)N * corr::kLayerW, 256), 256, 0, s>>>(
-                                     h, Wo, dOut, N, O, dh, dWo, dbo));
     return launch_status();
 }
 

@@ -83,26 +83,6 @@ __device__ __forceinline__ void store_row(float* p, const float (&v)[C]) {
     }
 }
 
-// Rows of NC consecutive floats of 32 consecutive items, item per lane, stored as whole 128-byte lines:
-// through the warp's shared-memory buffer (32 NC floats), lanes whose bit in `mask` is 0 left out.  A
-// scalar store per component puts 20 partial sectors into each request for rows of five floats, 100
-// sector writes per warp where 20 do (the L2 takes about 25 bytes of stores per SM and cycle, partial
-// sectors whole).  All lanes of the warp must call it; the buffer is free again on return.
-template <int NC>
-__device__ __forceinline__ void store_rows(float* dst /* row of lane 0 */, const float (&v)[NC], unsigned mask,
-                                           float* buf) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int c = 0; c < NC; ++c) buf[lane * NC + c] = v[c];
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < NC; ++q) {
-        const int e = 32 * q + lane;
-        if ((mask >> (e / NC)) & 1u) dst[e] = buf[e];
-    }
-    __syncwarp();
-}
-
 // Block-wide sum of NV doubles; the result is valid in thread 0.  blockDim.x <= 1024.
 template <int NV>
 __device__ __forceinline__ void block_sum(double (&v)[NV], double* smem /* [32 * NV] */) {

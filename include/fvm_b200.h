@@ -436,19 +436,8 @@ int fvm_back_bias(const float *dh, const float *Z, int32_t N, float *bias, void 
 int fvm_back_finish(int32_t n_sets, const float *const *sets, float *const *dst, const int32_t *n, void *stream);
 /* out[i] = [bf16(h_i), bf16(mean_{j in nbr(i)} h_j)]  (bf16 [N][128]) from the fp32 stream. */
 int fvm_mp_gather_f32(const float *h, const int32_t *nbr, int32_t N, int32_t KN, void *out, void *stream);
-/* dh_out[i] = dh_in[i] + dA[i][:W] + sum_{j in nbr(i)} dA[j][W:] / deg(j)  (fp32; dh_in may be NULL). */
-int fvm_mp_scatter_back(const float *dA, const int32_t *nbr, int32_t N, int32_t W, int32_t KN, const float *dh_in,
-                        float *dh_out, void *stream);
-/* dZ = dh * SiLU'(Z) -> bf16 [N][W] and (if dZT) bf16 [W][ldT]; db[c] += sum_i dZ[i][c] (if db). */
-int fvm_silu_back(const float *dh, const float *Z, int32_t N, int32_t W, void *dZ, void *dZT, int64_t ldT, float *db,
-                  void *stream);
-/* dst[c][r] = src[r][c] for a bf16 [R][Cc] matrix (leading dimensions lds, ldd). */
-int fvm_transpose_bf16(const void *src, int32_t R, int32_t Cc, int64_t lds, void *dst, int64_t ldd, void *stream);
 /* out[i][o] = bo[o] + sum_c h[i][c] Wo[o][c] (fp32 fma over c ascending; h fp32 [N][64], O <= 8). */
 int fvm_decoder_f32(const float *h, const float *Wo, const float *bo, int32_t N, int32_t O, float *out, void *stream);
-/* Decoder backward: dh = dOut Wo; dWo += dOut^T h; dbo += column sums of dOut (h fp32 [N][64]). */
-int fvm_decoder_back_f32(const float *h, const float *Wo, const float *dOut, int32_t N, int32_t O, float *dh,
-                         float *dWo, float *dbo, void *stream);
 /* loss[0] += mean((pred - tgt)^2) over n_elem values (FP64); dpred = 2 (pred - tgt) / n_elem. */
 int fvm_mse(const float *pred, const float *tgt, int64_t n_elem, double *loss, float *dpred, void *stream);
 /* Adam on fp32 master weights p with gradient g (zeroed afterwards), moments m, v; step >= 1.
