@@ -1260,14 +1260,16 @@ extern "C" int fvm_decoder_f32(const float* h, const float* Wo, const float* bo,
 // with one atomic per element (1178 us per layer at 278 k cells), two transposes, two GEMMs with
 // their operands read again and a scatter that counted every neighbour's neighbours.
 //
-// Column sums (the gradients of the biases and of the decoder) keep the value of one running fp32 sum
-// over the cells in order: with terms of one sign that sum's rounding is systematic (1.6e-4 of the
-// decoder's gradient at 278 k cells), so summing pieces from zero would move the results.  Rounding
-// a + t to fp32 depends on a only through its binade, so a block walks a contiguous range of rows with
-// accumulators that start at the sum of everything before it, taken from a first pass over the same
-// terms, and what they added is exact: the first pass runs in the kernel that produces the terms, the
-// second in the next kernel that reads them, the blocks' increments are added up once at the
-// end (k_back_finish).  The result does not depend on scheduling.
+// Column sums (the gradients of the biases and of the decoder) follow one running fp32 accumulator over the
+// cells, rounding error included: with terms of one sign that error is systematic (1.6e-4 of the decoder's
+// gradient at 278 k cells), and trained weights would move with it if pieces were summed from zero, which
+// is closer to the exact sum (5e-7) and would save the second pass.  Rounding a + t depends on a mostly
+// through its binade, so a block walks a contiguous range of rows with one accumulator per half-warp, each
+// started from the sum of the blocks before it (a first pass over the same terms); what an accumulator
+// gained is exact while it stays in its binade.  With 296 blocks of 24 half-warps the result is within
+// 3e-6 of the running sum, not equal to it, and it does not depend on scheduling.  The first pass runs in
+// the kernel that produces the terms, the second in the next kernel that reads them, and the blocks'
+// increments are added up once at the end (k_back_finish).
 // ------------------------------------------------------------------------------------------
 namespace fvm {
 namespace corr {

@@ -65,7 +65,8 @@ extern "C" {
  * Fc characteristic facets, K = dim + 1 facets per cell, KG = kg gradient slots: dim + 2 (the
  * reference's face-neighbour stencil) up to FVM_MAX_KG (a widened stencil); the cell record is then
  * FVM_CELL_REC_KG(dim, kg) floats wide.
- * Integer fields inside float records are stored bit-cast (int32 bits in a float slot). */
+ * Integer fields inside float records are stored bit-cast (int32 bits in a float slot).
+ * Zero-initialise the struct before filling it in: a field left at zero is switched off. */
 typedef struct fvm_mesh {
     int32_t dim, n_comp, n_cells, n_facets, n_bc, n_char, kg, kf;
     /* Cell records.  kg = dim + 2 (the reference's stencil): [N][FVM_CELL_REC] = the KG - 1
@@ -151,7 +152,10 @@ typedef struct fvm_work {
     float *prims;       /* [N][FVM_ROW] padded primitives (used by fvm_residual only)   */
     float *flux;        /* [F][FVM_ROW] facet fluxes                                    */
     double *red;        /* [FVM_RED_DOUBLES + 8 * n_cases], zero-initialised once; a partitioned
-                         * mesh (char_scale_given, fvm_char_partial) needs FVM_RED_DOUBLES + 8 */
+                         * mesh (char_scale_given, fvm_char_partial) needs FVM_RED_DOUBLES + 8.
+                         * Words 60 and 61 are the fused step's barrier and status, word 62 the block
+                         * counter of fvm_cfl_dt and fvm_conservation (zero between calls): a caller
+                         * leaves them alone */
 } fvm_work_t;
 
 /* Explicit Runge-Kutta tableau (optionally with an embedded low-order row). */
@@ -223,7 +227,9 @@ int fvm_ell_spmv(const float *vals, const int32_t *cols, int64_t M, int32_t K,
                  const float *x, int64_t incx, const float *bias, float *y, int64_t incy,
                  void *stream);
 
-/* Y[M][B] = A X (+ bias[:, None]).  X is [N][B] with leading dimension ldx, Y [M][B] with ldy. */
+/* Y[M][B] = A X (+ bias[:, None]).  X is [N][B] with leading dimension ldx, Y [M][B] with ldy.  With five
+ * columns a row of X may be read as the 16-byte words that hold its first and last float: up to 12 bytes
+ * beside the row, never outside those words, and not used. */
 int fvm_ell_spmm(const float *vals, const int32_t *cols, int64_t M, int32_t K,
                  const float *X, int64_t ldx, int32_t B, const float *bias, float *Y, int64_t ldy,
                  void *stream);
@@ -414,8 +420,11 @@ int fvm_corrector_propose(const float *state, const float *base, const float *ou
  * workspace sets of FVM_BACK_SET floats (16-byte aligned, no clearing needed):
  * one for each bias gradient and O + 1 consecutive ones (`dec`) for the decoder.  A set is filled by a
  * first and a second pass over the same terms, and fvm_back_finish adds set q's n[q] column sums to
- * dst[q] (host arrays, at most 32 sets).  A column sum has the value of one fp32 accumulator that
- * takes the cells in order, whatever the launch shape.
+ * dst[q] (host arrays, at most 32 sets).  The first pass leaves the sums of 296 equal ranges of cells; in
+ * the second each range's partial accumulators start from the sum of the ranges before it, and what they
+ * gained is added up in FP64.  A column sum so carries the rounding of a running fp32 accumulator over
+ * all cells (its error grows with their number, to 1.6e-4 of one-signed sums at 278 k cells); it does not
+ * depend on scheduling.
  *   fvm_back_top:     dh = dOut Wo; dZ (bf16) = dh SiLU'(Z); first pass of dec and bias
  *   fvm_back_decoder: second pass of dec (dWo[o] = set o, dbo = the last set's first O columns)
  *   fvm_back_layer:   dW [64][128] += dZ^T A and dA [N][128] = dZ W with columns 64.. divided by the row's
