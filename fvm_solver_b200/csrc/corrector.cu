@@ -1255,7 +1255,7 @@ extern "C" int fvm_decoder_f32(const float* h, const float* Wo, const float* bo,
 //     neighbour count) and dW += dZ^T A, both on tcgen05 from one staged copy of the tile;
 //   * k_back_gather: dh_l = dh_{l+1} + dA[:, :64] + sum over neighbours of dA[:, 64:], then
 //     dZ = dh_l SiLU'(Z_l) for the layer below.
-// Both are bound by memory: 0.9 kB and 1.7 kB per cell and layer (50 and 86 us at 278 k cells, 5.0 and
+// Both are bound by memory: 0.9 kB and 1.7 kB per cell and layer (52 and 86 us at 278 k cells, 4.8 and
 // 5.4 TB/s).  They replace a SiLU kernel
 // with one atomic per element (1178 us per layer at 278 k cells), two transposes, two GEMMs with
 // their operands read again and a scatter that counted every neighbour's neighbours.
