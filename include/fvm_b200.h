@@ -203,7 +203,7 @@ int fvm_profile_start(int32_t capacity);
  * kernel; stages always use 0. */
 int fvm_set_variant(int32_t kernel_id, int32_t variant);
 /* Launch overlap (no reference counterpart; results unchanged; default 1): 1 = the boundary,
- * cell, facet, divergence, conversion and finalisation kernels are launched with programmatic
+ * cell, facet, divergence, conversion, reduction and finalisation kernels are launched with programmatic
  * stream serialisation, so each is launched while the previous kernel of its stream (or CUDA
  * graph) drains and waits on the device (griddepcontrol.wait) for that kernel's completion and
  * writes; 0 = plain stream order. */
